@@ -207,7 +207,11 @@ const char *ih_autotune_report(const ih_context *c);
  * whole kz planes, transform the six sources of a plane one after the other
  * and accumulate their TT projection, so that update_h reads two projected
  * spectra instead of six; mixed form at 256^3 only, IH_ERR_ARG elsewhere;
- * 0: the row and column passes);
+ * 0: the row and column passes), 9 = the passes of the FP64 form that run in
+ * 64-bit block fixed point on the integer pipe (a mask of 1 << pass over the
+ * passes 0, 1, 3, 4 and 6, IH_FFT_FIXED_ALL by default on power-of-two grids,
+ * 0 = none; IH_ERR_ARG for a mask other than 0 in the mixed form and on
+ * radix-3 grids; pinning an engine of one of these passes takes its bit out);
  * engine IH_FFT_STOCKHAM, IH_FFT_TWOSTEP (register two-step,
  * 128-byte tiles), IH_FFT_TWOSTEP_HALF (64-byte tiles), IH_FFT_PIPELINED
  * (register two-step in persistent CTAs that copy the next tile in with
@@ -217,6 +221,7 @@ const char *ih_autotune_report(const ih_context *c);
  * per SM; passes 0 and 1, FP32; FP64 runs IH_FFT_TWOSTEP_HALF). */
 enum { IH_FFT_STOCKHAM = 0, IH_FFT_TWOSTEP = 1, IH_FFT_TWOSTEP_HALF = 2, IH_FFT_PIPELINED = 3,
        IH_FFT_THREESTEP = 4, IH_FFT_TWOSTEP_HALF_OCC = 5 };
+enum { IH_FFT_FIXED_ALL = 0x5b };
 int ih_fft_set_engine(ih_context *c, int pass, int engine);
 int ih_fft_get_engine(const ih_context *c, int pass);
 /* How an RHS without the filter and output flags forms the derivatives of

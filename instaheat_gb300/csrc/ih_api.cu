@@ -213,6 +213,9 @@ static void destroy(Ctx *c) {
   if (c->tw_y) cudaFree(c->tw_y);
   if (c->tw_h) cudaFree(c->tw_h);
   if (c->tw_z) cudaFree(c->tw_z);
+  for (void *p : c->fx_tw)
+    if (p) cudaFree(p);
+  if (c->fx_coef) cudaFree(c->fx_coef);
   if (c->spec[0]) cudaFree(c->spec[0]);
   if (c->rbuf[0]) cudaFree(c->rbuf[0]);
   if (c->gscratch) cudaFree(c->gscratch);
@@ -520,6 +523,16 @@ int ih_fft_set_engine(ih_context *h, int pass, int engine) {
     h->c.graph_epoch += 1;
     return IH_OK;
   }
+  if (pass == 9) {  // fixed-point transforms of the FP64 form
+    if (engine & ~kFxAll) return IH_ERR_ARG;
+    if (engine && !h->c.fx_coef) {
+      h->c.err = "fixed-point transforms apply to the FP64 form on power-of-two grids";
+      return IH_ERR_ARG;
+    }
+    h->c.fx_on = engine;
+    h->c.graph_epoch += 1;
+    return IH_OK;
+  }
   if (pass == 7) {  // kz slab width of the tensor sources' y/x passes
     if (engine < 0 || engine > 64 || engine % 8) return IH_ERR_ARG;
     h->c.gw_slab = engine;
@@ -532,6 +545,8 @@ int ih_fft_set_engine(ih_context *h, int pass, int engine) {
     return IH_ERR_ARG;
   if (pass == 5 && engine > 1) return IH_ERR_ARG;
   if (pass == 6 && (engine > 2 || (engine == 2 && !h->c.mixed))) return IH_ERR_ARG;
+  // a pinned engine replaces the fixed-point form of its pass
+  h->c.fx_on &= ~(1 << pass);
   if (pass < 2) {
     h->c.xy_var[pass] = engine;
   } else if (pass == 2) {
@@ -575,7 +590,8 @@ int ih_graphs_enable(ih_context *h, int on) {
 }
 
 int ih_fft_get_engine(const ih_context *h, int pass) {
-  if (!h || pass < 0 || pass > 8) return -1;
+  if (!h || pass < 0 || pass > 9) return -1;
+  if (pass == 9) return h->c.fx_on;
   if (pass == 8) return h->c.gw_plane;
   if (pass == 7) return h->c.gw_slab;
   if (pass < 2) return h->c.xy_var[pass];
@@ -960,6 +976,7 @@ int ih_ensemble_autotune(ih_ensemble *e) {
       c->tensor_fused = twin->tensor_fused;
       c->zwide = twin->zwide;
       c->gw_slab = twin->gw_slab;
+      c->fx_on = twin->fx_on;
       c->velocity_form = twin->velocity_form;
       c->tune_report = twin->tune_report;
       c->graph_epoch += 1;

@@ -1726,6 +1726,8 @@ int fft_xy(Ctx *c, C2<T> *data, long long stride, int count, int axis, int sign)
     XYLaunch<T> xl{c, data, stride, count, axis, sign, FV_STOCKHAM};
     IH_TRY((xl.template run_st<B, true>(L, dim3((g.mz + B - 1) / B, outer, count), sj, so,
                                         tab<T>(axis == 0 ? c->tw_x : c->tw_y))));
+  } else if (sizeof(T) == 8 && (c->fx_on >> axis & 1)) {
+    IH_TRY(fix_xy(c, data, stride, count, axis, sign, 0));
   } else {
     IH_TRY(dispatch_len(L, XYLaunch<T>{c, data, stride, count, axis, sign, c->xy_var[axis]},
                         allow512<T>()));
@@ -1761,7 +1763,11 @@ int fft_gw_yx(Ctx *c, C2<T> *spec, int w) {
         prof_begin(c, KK_FFT_XY);
         XYLaunch<T> xl{c, d, M, count, axis, -1, c->xy_var[axis]};
         xl.cols = ws;
-        IH_TRY(dispatch_len(L, xl, allow512<T>()));
+        if (sizeof(T) == 8 && (c->fx_on >> axis & 1)) {
+          IH_TRY(fix_xy(c, d, M, count, axis, -1, ws));
+        } else {
+          IH_TRY(dispatch_len(L, xl, allow512<T>()));
+        }
         prof_end(c, KK_FFT_XY, 2.0 * count * (double)g.nx * g.ny * ws * sizeof(C2<T>));
         IH_TRY(check_launch(c, "k_fft_xy"));
       }
@@ -1808,7 +1814,9 @@ int fft_zr2c(Ctx *c, const T *in, long long in_stride, C2<T> *out, long long out
              int count) {
   const Geom &g = c->g;
   prof_begin(c, KK_FFT_ZR2C);
-  if (fused_wide_ok(c)) {
+  if (sizeof(T) == 8 && (c->fx_on >> 6 & 1)) {
+    IH_TRY(fix_z(c, in, in_stride, out, out_stride, count, true));
+  } else if (fused_wide_ok(c)) {
     IH_TRY(zr2c_wide_launch(c, in, in_stride, out, out_stride, count));
   } else if (g.h & (g.h - 1)) {
     const long long rows = (long long)g.nx * g.ny;
@@ -1829,7 +1837,9 @@ int fft_zc2r(Ctx *c, const C2<T> *in, long long in_stride, T *out, long long out
              int count) {
   const Geom &g = c->g;
   prof_begin(c, KK_FFT_ZC2R);
-  if (g.h & (g.h - 1)) {
+  if (sizeof(T) == 8 && (c->fx_on >> 6 & 1)) {
+    IH_TRY(fix_z(c, in, in_stride, out, out_stride, count, false));
+  } else if (g.h & (g.h - 1)) {
     const long long rows = (long long)g.nx * g.ny;
     const size_t sm = zg_smem<T>(g.h);
     cudaFuncSetAttribute(k_fft_zc2r_g<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -2036,8 +2046,12 @@ template <typename T>
 int fft_xy_roundtrip(Ctx *c, const C2<T> *z, C2<T> *d1, C2<T> *d2, int axis) {
   const Geom &g = c->g;
   prof_begin(c, KK_XY_RT);
-  IH_TRY(dispatch_len(axis == 0 ? g.nx : g.ny, RTLaunch<T>{c, z, d1, d2, axis, c->rt_var[axis]},
-                      allow512<T>()));
+  if (sizeof(T) == 8 && (c->fx_on >> (3 + axis) & 1)) {
+    IH_TRY(fix_roundtrip(c, z, d1, d2, axis));
+  } else {
+    IH_TRY(dispatch_len(axis == 0 ? g.nx : g.ny, RTLaunch<T>{c, z, d1, d2, axis, c->rt_var[axis]},
+                        allow512<T>()));
+  }
   prof_end(c, KK_XY_RT, (axis == 1 ? 4.0 : 3.0) * g.M * sizeof(C2<T>));
   return check_launch(c, "k_fft_xy_rt");
 }
@@ -2099,7 +2113,9 @@ int fft_z_rhs_fused(Ctx *c, const C2<T> *d4, const T *yfl, const double *ysc, T 
                     int plane) {
   const Geom &g = c->g;
   prof_begin(c, KK_Z_RHS_FUSED);
-  if (fused_wide_ok(c)) {  // nz = 256: the wide-row engine
+  if (sizeof(T) == 8 && (c->fx_on >> 6 & 1)) {
+    IH_TRY(fix_z_rhs(c, d4, yfl, ysc, lap, p, rho, s6, gw, partials, nblocks_out, zsrc));
+  } else if (fused_wide_ok(c)) {  // nz = 256: the wide-row engine
     IH_TRY(fused_wide_launch(c, d4, yfl, ysc, lap, p, rho, s6, gw, partials, nblocks_out, zsrc,
                              plane));
   } else {
@@ -2145,7 +2161,7 @@ int fft_tables(Ctx *c) {
     IH_TRY(upload_table<double>(c, &c->tw_h, g.h));
     IH_TRY(upload_table<double>(c, &c->tw_z, g.nz));
   }
-  return IH_OK;
+  return fix_tables(c);
 }
 
 // ---------------------------------------------------------------------------
@@ -2185,15 +2201,22 @@ static int autotune_t(Ctx *c) {
   static const char *pass_name[5] = {"x", "y", "deriv4-x", "rt-x", "rt-y"};
   int best_t = 0;
   float tbest_t = 0.f;
-  // x, y, fused x, x and y round trips
+  // x, y, fused x, x and y round trips; FP64: the fixed-point form of each
+  // against the fastest FP64 engine
+  const int fixed = FV_COUNT;
+  const bool fx = sizeof(T) == 8 && c->fx_coef;
   for (int pass = 0; pass < 5 && st == IH_OK; ++pass) {
     int best = -1;
-    float tbest = 0.f;
-    for (int v = 0; v < FV_COUNT && st == IH_OK; ++v) {
+    float tbest = 0.f, tfixed = -1.f;
+    c->fx_on &= ~(1 << pass);
+    for (int v = 0; v <= FV_COUNT && st == IH_OK; ++v) {
       if (pass == 2 && (v == FV_THREESTEP || v == FV_TWOSTEP_HALF_OCC))
         continue;  // the fused x pass has neither form
-      if (pass > 2 && v != FV_TWOSTEP && v != FV_TWOSTEP_HALF) continue;
-      if (pass < 2) {
+      if (pass > 2 && v != FV_TWOSTEP && v != FV_TWOSTEP_HALF && v != fixed) continue;
+      if (v == fixed) {
+        if (!fx || !(kFxAll >> pass & 1)) continue;
+        c->fx_on |= 1 << pass;
+      } else if (pass < 2) {
         c->xy_var[pass] = v;
       } else if (pass == 2) {
         c->d4_var = v;
@@ -2219,14 +2242,18 @@ static int autotune_t(Ctx *c) {
         break;
       }
       ms /= reps;
-      snprintf(line, sizeof line, "%s %s %.1f us; ", pass_name[pass], variant_name(v), 1e3 * ms);
+      snprintf(line, sizeof line, "%s %s %.1f us; ", pass_name[pass],
+               v == fixed ? "fixed-point" : variant_name(v), 1e3 * ms);
       rep += line;
-      if (best < 0 || ms < tbest) {
+      if (v == fixed) {
+        tfixed = ms;
+      } else if (best < 0 || ms < tbest) {
         best = v;
         tbest = ms;
       }
     }
     if (best < 0) break;
+    if (tfixed < 0.f || tbest < tfixed) c->fx_on &= ~(1 << pass);
     if (pass < 2) {
       c->xy_var[pass] = best;
     } else if (pass == 2) {
@@ -2391,10 +2418,10 @@ static int autotune_t(Ctx *c) {
   if (st != IH_OK) return st;
   snprintf(line, sizeof line,
            "chosen: x %s, y %s, deriv4-x %s, rt-x %s, rt-y %s, tensor %s, gw-yx slab %d, "
-           "gw planes %d, z pass %d",
+           "gw planes %d, z pass %d, fixed-point passes %#x",
            variant_name(c->xy_var[0]), variant_name(c->xy_var[1]), variant_name(c->d4_var),
            variant_name(c->rt_var[0]), variant_name(c->rt_var[1]),
-           c->tensor_fused ? "fused" : "separate", c->gw_slab, c->gw_plane, c->zwide);
+           c->tensor_fused ? "fused" : "separate", c->gw_slab, c->gw_plane, c->zwide, c->fx_on);
   c->tune_report = rep + line;
   return IH_OK;
 }

@@ -1,0 +1,290 @@
+// ih_fix.cuh -- 64-bit block fixed point for the transforms of the plain FP64
+// form.
+//
+// An FP64 addition issues at 1.8 per clock per SM on this GPU (measured:
+// independent DADD chains, 152 SMs at 1.92 GHz; DFMA 2.1), a 64-bit integer
+// addition at 60, and the product of two 64-bit fractions (the upper 64 bits,
+// one IMAD.WIDE and two IMAD.HI) at 7.5 against 1.8 DMUL.  A transform is
+// mostly additions, so the passes here hold a pencil as 64-bit integers that
+// share one exponent: the largest magnitude of the pencil is brought to 2^p,
+// the butterflies are integer additions (exact), and every multiplication by
+// a twiddle rounds to a unit of 2^-p (or 2^(2-p) after the middle twiddle) of
+// the largest value, where p is as large as the worst-case growth of the
+// transform leaves room for.  With p >= 53 the error of a pass is at or below
+// that of the same pass in FP64, whose additions each round to 2^-53 of
+// partial sums that grow with the transform.
+//
+// Growth: |Re|, |Im| <= 2^p at the input of an L-point transform bound every
+// output by L sqrt(2) 2^p; the multiplication by a table twiddle keeps the
+// upper 64 bits of a product with a Q62 fraction, a factor 1/4, so the bound
+// is L sqrt(2) 2^(p - 2) < 2^63 for p = 64 - log2 L.
+#pragma once
+#include "ih_internal.cuh"
+#include "ih_fftcore.cuh"
+
+namespace ih {
+
+struct __align__(16) fx2 {
+  long long x, y;
+};
+
+// a table twiddle c + i s as the three products of a complex multiplication
+// need it: c, s - c, s + c in Q62, each split as high * 2^32 + low with a
+// signed low word (a = {c high, c low, s-c high, s-c low}, b = {s+c})
+struct FxTab {
+  const int4 *a;
+  const int2 *b;
+};
+struct FxW {
+  int4 a;
+  int2 b;
+};
+__device__ __forceinline__ FxW fx_tw(const FxTab &t, int i) {
+  FxW w;
+  w.a = __ldg(t.a + i);
+  w.b = __ldg(t.b + i);
+  return w;
+}
+
+__device__ __forceinline__ fx2 fx_mk(long long x, long long y) {
+  fx2 r;
+  r.x = x;
+  r.y = y;
+  return r;
+}
+__device__ __forceinline__ fx2 operator+(fx2 a, fx2 b) { return fx_mk(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ fx2 operator-(fx2 a, fx2 b) { return fx_mk(a.x - b.x, a.y - b.y); }
+
+// high * 2^32 + low with a signed low word
+__device__ __forceinline__ int fx_hi(long long a) {
+  return (int)(a >> 32) + (int)((unsigned)a >> 31);
+}
+// a w / 2^64 from the split halves of both: the low * low product is left out
+// (below half a unit, of either sign), the two cross products round down, on
+// average by one unit together, which the + 1 returns
+__device__ __forceinline__ long long fx_mul(int ah, int al, int wh, int wl) {
+  const int c = __mulhi(ah, wl) + __mulhi(al, wh) + 1;
+  return (long long)ah * wh + c;
+}
+__device__ __forceinline__ long long fx_mul(long long a, int wh, int wl) {
+  return fx_mul(fx_hi(a), (int)a, wh, wl);
+}
+// by a 64-bit constant or variable fraction
+__device__ __forceinline__ long long fx_mul(long long a, long long w) {
+  return fx_mul(fx_hi(a), (int)a, fx_hi(w), (int)w);
+}
+// v (c + i s) / 4 (S = -1) or v (c - i s) / 4 (S = +1), the table holding the
+// forward twiddle
+template <int S>
+__device__ __forceinline__ fx2 fx_cmul(fx2 v, const FxW &w) {
+  const long long k = fx_mul(v.x + v.y, w.a.x, w.a.y);
+  const int xh = fx_hi(v.x), xl = (int)v.x, yh = fx_hi(v.y), yl = (int)v.y;
+  if (S < 0)
+    return fx_mk(k - fx_mul(yh, yl, w.b.x, w.b.y), k + fx_mul(xh, xl, w.a.z, w.a.w));
+  return fx_mk(k + fx_mul(yh, yl, w.a.z, w.a.w), k - fx_mul(xh, xl, w.b.x, w.b.y));
+}
+// v / 4, the trivial twiddle
+__device__ __forceinline__ fx2 fx_quarter(fx2 v) { return fx_mk((v.x + 2) >> 2, (v.y + 2) >> 2); }
+
+// rotation by D x 90 degrees
+template <int D>
+__device__ __forceinline__ fx2 fx_rot90(fx2 v) {
+  if ((D & 3) == 0) return v;
+  if ((D & 3) == 1) return fx_mk(-v.y, v.x);
+  if ((D & 3) == 2) return fx_mk(-v.x, -v.y);
+  return fx_mk(v.y, -v.x);
+}
+// v exp(2 pi i M / 32) at v's own scale: quarter turns and a rotation by at
+// most 45 degrees, which is three shears (tan, sin, tan of Q64 fractions
+// below 1/2) or, at 45 degrees, a sum and a difference by sqrt(1/2) = 1 -
+// 0.29289...
+constexpr long long kFxOneMinusSqrtHalf = 0x4afb0ccc06219b7cLL;  // 1 - sqrt(1/2)
+constexpr long long kFxTanPi16 = 0x32ebebc0aa62b00fLL;           // tan(pi/16)
+constexpr long long kFxSinPi8 = 0x61f78a9abaa58b47LL;            // sin(pi/8)
+constexpr long long kFxTanPi32 = 0x1936bb8c5b2da262LL;           // tan(pi/32)
+constexpr long long kFxSinPi16 = 0x31f17078d34c156dLL;           // sin(pi/16)
+constexpr long long kFxTan3Pi32 = 0x4da820d5718f6f14LL;          // tan(3 pi/32)
+constexpr long long kFxOneMinusSin3Pi16 = 0x71c626328cb9bc9bLL;  // 1 - sin(3 pi/16)
+
+template <int M>
+__device__ __forceinline__ fx2 fx_rot32(fx2 v) {
+  constexpr int m = ((M % 32) + 32) % 32;
+  constexpr int q = (m + 4) / 8;  // quarter turns; the rest r in (-45, 45]
+  constexpr int r = m - 8 * q;    // -4 .. 3 units of 11.25 degrees
+  v = fx_rot90<q>(v);
+  if (r == 0) return v;
+  if (r == -4) {  // 45 degrees clockwise: (x + y, y - x) sqrt(1/2)
+    const long long a = v.x + v.y, b = v.y - v.x;
+    return fx_mk(a - fx_mul(a, kFxOneMinusSqrtHalf), b - fx_mul(b, kFxOneMinusSqrtHalf));
+  }
+  constexpr int ra = r < 0 ? -r : r;
+  constexpr long long T = ra == 1 ? kFxTanPi32 : ra == 2 ? kFxTanPi16 : kFxTan3Pi32;
+  if (r > 0) {
+    v.x -= fx_mul(v.y, T);
+    if (ra == 3)
+      v.y += v.x - fx_mul(v.x, kFxOneMinusSin3Pi16);
+    else
+      v.y += fx_mul(v.x, ra == 1 ? kFxSinPi16 : kFxSinPi8);
+    v.x -= fx_mul(v.y, T);
+  } else {
+    v.x += fx_mul(v.y, T);
+    if (ra == 3)
+      v.y -= v.x - fx_mul(v.x, kFxOneMinusSin3Pi16);
+    else
+      v.y -= fx_mul(v.x, ra == 1 ? kFxSinPi16 : kFxSinPi8);
+    v.x += fx_mul(v.y, T);
+  }
+  return v;
+}
+
+template <int R, int... K>
+__device__ __forceinline__ void fx_brev(fx2 (&v)[R], std::integer_sequence<int, K...>) {
+  const fx2 t[R] = {v[Brev<K, clog2(R)>::value]...};
+  ((v[K] = t[K]), ...);
+}
+
+// one radix-2 decimation-in-frequency stage of span LEN, butterfly J..
+template <int R, int LEN, int S, int J>
+__device__ __forceinline__ void fx_stage(fx2 (&v)[R]) {
+  if constexpr (J < LEN / 2) {
+#pragma unroll
+    for (int st = 0; st < R; st += LEN) {
+      const fx2 a = v[st + J], b = v[st + J + LEN / 2];
+      v[st + J] = a + b;
+      v[st + J + LEN / 2] = fx_rot32<S * J * (32 / LEN)>(a - b);
+    }
+    fx_stage<R, LEN, S, J + 1>(v);
+  }
+}
+template <int R, int LEN, int S>
+__device__ __forceinline__ void fx_stages(fx2 (&v)[R]) {
+  if constexpr (LEN > 1) {
+    fx_stage<R, LEN, S, 0>(v);
+    fx_stages<R, LEN / 2, S>(v);
+  }
+}
+// in-register DFT of R <= 32 points, v[k] <- sum_n v[n] exp(S 2 pi i nk/R)
+template <int R, int S>
+__device__ __forceinline__ void fx_dft(fx2 (&v)[R]) {
+  fx_stages<R, R, S>(v);
+  fx_brev<R>(v, std::make_integer_sequence<int, R>{});
+}
+
+// ---------------------------------------------------------------------------
+// FP64 <-> fixed point of one pencil.  m: the largest |high word| of its
+// components (fx_max_in).
+__device__ __forceinline__ unsigned fx_absbits(double a) {
+  return (unsigned)__double2hiint(a) & 0x7fffffffu;
+}
+struct FxScale {
+  int in;       // exponent added to the inputs: integer = round(x 2^in)
+  int out;      // exponent of the result so far: value = integer 2^out
+  bool slow;    // the pencil needs the factors below
+  double pre, post;
+};
+// The common case (largest value 2^-323 to 2^37) takes exponents for which
+// adding `in` to the exponent field of any component (zeros and subnormals
+// included) stays a finite number, and for which the exponents of products of
+// two pencils stay in range; other pencils are brought there by an exact power
+// of two, and a pencil with an Inf or NaN comes out as NaN.
+__device__ __forceinline__ FxScale fx_scale(unsigned m, int p) {
+  FxScale s;
+  int E = (int)(m >> 20);
+  s.slow = E < 700 || E > 1060;
+  s.pre = s.post = 1.0;
+  if (s.slow) {
+    int d;  // exponent taken off: values of the order of one, or as near as a factor comes
+    if (E == 2047) {
+      d = 0;
+      E = 1023;
+    } else {
+      d = E < 1 ? -1000 : (E > 2023 ? 1000 : E - 1023);
+      E = (E < 1 ? 1 : E) - d;
+    }
+    s.pre = __hiloint2double((1023 - d) << 20, 0);
+    s.post = __hiloint2double((1023 + d) << 20, 0);
+    if ((m >> 20) == 2047) {
+      s.pre = 0.0;
+      s.post = __longlong_as_double(0x7ff8000000000000LL);
+    }
+    if (m == 0) s.post = 0.0;  // all zero: products of zeros carry a rounding unit
+  }
+  s.in = p + 1022 - E;
+  s.out = -s.in;
+  return s;
+}
+__device__ __forceinline__ long long fx_in(double a, const FxScale &s) {
+  return __double2ll_rn(
+      __hiloint2double(__double2hiint(a) + s.in * (1 << 20), __double2loint(a)));
+}
+__device__ __forceinline__ double fx_out(long long v, int e) {
+  const double d = __ll2double_rn(v);
+  const int h = __double2hiint(d);
+  return __hiloint2double(h == 0 ? 0 : h + e * (1 << 20), __double2loint(d));
+}
+template <int R>
+__device__ __forceinline__ unsigned fx_max_in(const double2 (&x)[R]) {
+  unsigned m = 0, low = 0;
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    m = max(m, max(fx_absbits(x[i].x), fx_absbits(x[i].y)));
+    low |= (unsigned)(__double2loint(x[i].x) | __double2loint(x[i].y));
+  }
+  return low ? m | 1u : m;  // 0 only where every value is 0
+}
+template <int R>
+__device__ __forceinline__ void fx_load(double2 (&x)[R], const FxScale &s, fx2 (&v)[R]) {
+  if (s.slow) {
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      x[i].x = s.pre == 0.0 ? 0.0 : x[i].x * s.pre;
+      x[i].y = s.pre == 0.0 ? 0.0 : x[i].y * s.pre;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < R; ++i) v[i] = fx_mk(fx_in(x[i].x, s), fx_in(x[i].y, s));
+}
+// value of v at exponent e, through the slow factor where the pencil has one
+__device__ __forceinline__ double2 fx_store(fx2 v, int e, const FxScale &s) {
+  double2 r = make_double2(fx_out(v.x, e), fx_out(v.y, e));
+  if (s.slow) {
+    r.x *= s.post;
+    r.y *= s.post;
+  }
+  return r;
+}
+// |high word| of integers, and the shift that brings a largest such word just
+// below 2^bits (a left shift loses nothing; a right shift rounds)
+__device__ __forceinline__ unsigned fx_abshi(long long a) {
+  const int h = (int)(a >> 32);
+  return (unsigned)(h ^ (h >> 31));
+}
+template <int R>
+__device__ __forceinline__ unsigned fx_max_int(const fx2 (&v)[R]) {
+  unsigned m = 0;
+#pragma unroll
+  for (int i = 0; i < R; ++i) m = max(m, max(fx_abshi(v[i].x), fx_abshi(v[i].y)));
+  return m;
+}
+__device__ __forceinline__ int fx_room(unsigned maxhi, int bits) {
+  return bits - (64 - __clz(maxhi));  // |v| < 2^(64 - clz(maxhi))
+}
+struct FxShift {
+  int l, r;
+  long long half;
+};
+__device__ __forceinline__ FxShift fx_shift_of(int s) {
+  FxShift f;
+  f.l = max(s, 0);
+  f.r = max(-s, 0);
+  f.half = (1LL << f.r) >> 1;
+  return f;
+}
+__device__ __forceinline__ long long fx_shift(long long v, const FxShift &f) {
+  return ((v << f.l) + f.half) >> f.r;
+}
+__device__ __forceinline__ fx2 fx_shift(fx2 v, const FxShift &f) {
+  return fx_mk(fx_shift(v.x, f), fx_shift(v.y, f));
+}
+
+}  // namespace ih

@@ -237,8 +237,18 @@ struct Ctx {
   int stage_fusion = 0;  // DOPRI853 stage inputs formed by the RHS of the previous stage
   int velocity_form = 1; // mixed form: stage combinations from the velocity halves only
   int skip_pos = 0;      // set during the stage evaluations of a velocity-form try
+  // FP64 form, power-of-two axes: transforms in 64-bit block fixed point
+  // (ih_fix.cu).  fx_on: the passes that run so (bits as the passes of
+  // ih_fft_set_engine: 0 x, 1 y, 3 / 4 the round trips, 6 the z passes);
+  // fx_tw: twiddles of x, y, h, nz; fx_coef: derivative coefficients;
+  // fx_e: their exponents (x first, x second, y first, y and z second, z first)
+  int fx_on = 0;
+  void *fx_tw[4] = {};
+  void *fx_coef = nullptr;
+  int fx_e[5] = {};
   std::string tune_report;
 };
+constexpr int kFxAll = 0x5b;
 
 
 // ---------------------------------------------------------------------------
@@ -337,6 +347,15 @@ int gw_tt_plane(Ctx *c, void *spec);
 int update_h_tt(Ctx *c, const void *spec, const void *y, void *out, double *outsc);
 
 int fft_tables(Ctx *c);
+
+// the fixed-point passes of the FP64 form (ih_fix.cu)
+int fix_tables(Ctx *c);
+int fix_xy(Ctx *c, void *data, long long stride, int count, int axis, int sign, int cols);
+int fix_roundtrip(Ctx *c, const void *z, void *d1, void *d2, int axis);
+int fix_z(Ctx *c, const void *in, long long istride, void *out, long long ostride, int count,
+          bool forward);
+int fix_z_rhs(Ctx *c, const void *d4, const void *yfl, const double *ysc, void *lap, void *p,
+              void *rho, void *s6, int gw, double *partials, int *nblk_out, int zsrc);
 // time every engine variant of the x/y passes and the fused x pass on the
 // context's scratch spectra and keep the fastest
 int fft_autotune(Ctx *c);

@@ -21,6 +21,7 @@ PREC_F64 = 0
 PREC_MIXED = 1
 FFT_STOCKHAM, FFT_TWOSTEP, FFT_TWOSTEP_HALF, FFT_PIPELINED, FFT_THREESTEP = 0, 1, 2, 3, 4
 FFT_TWOSTEP_HALF_OCC = 5
+FFT_FIXED_ALL = 0x5b  # pass 9: every pass that has a fixed-point form
 
 STATUS = {0: "ok", 1: "invalid argument", 2: "CUDA error", 3: "allocation failed",
           4: "call out of order", 5: "step size underflow", 6: "non-finite value"}
@@ -377,8 +378,11 @@ class Context:
             except ValueError:
                 known = None
             if known and len(known.get("engines", ())) == len(self.engines()):
+                fixed = self.L_.ih_fft_get_engine(self.h, 9)
                 for p, e in enumerate(known["engines"]):
                     self.set_engine(p, e)
+                if fixed:  # the pinned engines lie under the fixed-point form
+                    self.set_engine(9, known.get("fixed", fixed))
                 self._wisdom_report = "from wisdom: " + known["report"]
                 return self._wisdom_report
         self._ck(self.L_.ih_autotune(self.h), "ih_autotune")
@@ -389,7 +393,8 @@ class Context:
                 data = json.loads(path.read_text()) if path.exists() else {}
             except ValueError:
                 data = {}
-            data[key] = {"engines": list(self.engines()), "report": report}
+            data[key] = {"engines": list(self.engines()), "report": report,
+                         "fixed": int(self.L_.ih_fft_get_engine(self.h, 9))}
             path.parent.mkdir(parents=True, exist_ok=True)
             path.write_text(json.dumps(data))
         return report
