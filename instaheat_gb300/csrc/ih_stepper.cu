@@ -252,34 +252,40 @@ __device__ __forceinline__ void vstore(T *p, const T *v) {
   }
 }
 
-// y_stage = y + dt * sum_j a_sj k_j (dopri853.c:340-436, rk4.c:131-150)
-template <typename T>
-__global__ void k_lincomb(const T *__restrict__ base, const double *basesc, T *__restrict__ out,
-                          double *outsc, LinArgs args, long long nf) {
+// y_stage = y + dt * sum_j a_sj k_j (dopri853.c:340-436, rk4.c:131-150).  NT:
+// the number of terms.  A term behind a run-time test (12 of them, whatever
+// the stage) still takes its issue slot when the test is a predicate, and in
+// FP64 the slots are what there is: 143 DFMA slots per element over the 11
+// stages of a step against 61 with the count known.  FP64 256^3, the 11
+// combinations of a step: 15.9 ms against 35.7, 4.9 TB/s (bound by the FP64
+// pipe, 13 ms of DFMA, and HBM, 11.6 ms, together).
+template <typename T, int NT>
+__global__ void __launch_bounds__(256) k_lincomb(const T *__restrict__ base, const double *basesc,
+                                                 T *__restrict__ out, double *outsc, LinArgs args,
+                                                 long long nf) {
   constexpr int W = Vec4<T>::W;
   const long long nv = nf / W;
-  T cf[kMaxTerms];
+  T cf[NT + 1];
 #pragma unroll
-  for (int j = 0; j < kMaxTerms; ++j) cf[j] = (T)args.coef[j];
+  for (int j = 0; j < NT; ++j) cf[j] = (T)args.coef[j];
   const double scd = args.scale_dev ? *args.scale_dev : args.scale;
   const T sc = (T)scd;
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nv;
        v += (long long)gridDim.x * blockDim.x) {
-    T acc[W], x[W];
+    T x[NT + 1][W], acc[W];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) vload<T>((const T *)args.in[j] + v * W, x[j]);
+    vload<T>(base + v * W, x[NT]);
 #pragma unroll
     for (int w = 0; w < W; ++w) acc[w] = 0;
 #pragma unroll
-    for (int j = 0; j < kMaxTerms; ++j) {
-      if (j < args.n) {
-        vload<T>((const T *)args.in[j] + v * W, x);
+    for (int j = 0; j < NT; ++j) {
 #pragma unroll
-        for (int w = 0; w < W; ++w) acc[w] += cf[j] * x[w];
-      }
+      for (int w = 0; w < W; ++w) acc[w] += cf[j] * x[j][w];
     }
-    vload<T>(base + v * W, x);
 #pragma unroll
-    for (int w = 0; w < W; ++w) x[w] = x[w] + sc * acc[w];
-    vstore<T>(out + v * W, x);
+    for (int w = 0; w < W; ++w) acc[w] = x[NT][w] + sc * acc[w];
+    vstore<T>(out + v * W, acc);
   }
   if (blockIdx.x == 0 && threadIdx.x < 5) {
     const int s = threadIdx.x;
@@ -295,6 +301,7 @@ struct FinalArgs {
   const void *k[8];
   const double *ksc[8];
   double b[8], e5[8], e3[8];  // e5 = b - bhh on stages 1, 9, 12
+  double bhh[3];              // of stages 1, 9, 12 (k[0], k[4], k[7])
   const double *dt;           // step size (device memory)
   double rtol, atol;
   double noise;               // eta * eps32 (mixed form), 0 for FP64
@@ -365,22 +372,31 @@ __global__ void __launch_bounds__(256) k_dopri_final(const T *__restrict__ y, co
   for (int i = 0; i < (DIAG ? 12 : 1); ++i) dacc[i] = 0.0;
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nv;
        v += (long long)gridDim.x * blockDim.x) {
-    T ab[W], a5[W], a3[W], t5[W], t3[W], x[W];
+    T ab[W], a5[W], a3[W], t5[W], t3[W];
+    T x[8][W];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) vload<T>((const T *)a.k[j] + v * W, x[j]);
 #pragma unroll
     for (int w = 0; w < W; ++w) ab[w] = a5[w] = a3[w] = t5[w] = t3[w] = 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      vload<T>((const T *)a.k[j] + v * W, x);
 #pragma unroll
       for (int w = 0; w < W; ++w) {
-        ab[w] += cb[j] * x[w];
-        a5[w] += c5[j] * x[w];
-        a3[w] += c3[j] * x[w];
+        ab[w] += cb[j] * x[j][w];
+        a3[w] += c3[j] * x[j][w];
         if constexpr (sizeof(T) == 4) {
-          t5[w] += fabsf(c5[j] * x[w]);
-          t3[w] += fabsf(c3[j] * x[w]);
+          a5[w] += c5[j] * x[j][w];
+          t5[w] += fabsf(c5[j] * x[j][w]);
+          t3[w] += fabsf(c3[j] * x[j][w]);
         }
       }
+    }
+    if constexpr (sizeof(T) == 8) {
+      // the 3rd-order difference as the reference forms it (dopri853.c:451),
+      // three terms off the 8th-order sum instead of eight of its own
+#pragma unroll
+      for (int w = 0; w < W; ++w)
+        a5[w] = ab[w] - a.bhh[0] * x[0][w] - a.bhh[1] * x[4][w] - a.bhh[2] * x[7][w];
     }
     T yv[W], yn[W];
     vload<T>(y + v * W, yv);
@@ -412,15 +428,17 @@ __global__ void __launch_bounds__(256) k_dopri_final(const T *__restrict__ y, co
       acc5d = (double)acc5;
       acc3d = (double)acc3;
     } else {
-      const double ys = seg < 4 ? hs[3][seg] : 0.0, yns = seg < 4 ? hs[4][seg] : 0.0;
-      const double q5s = seg < 4 ? hs[1][seg] : 0.0, q3s = seg < 4 ? hs[2][seg] : 0.0;
+      // the homogeneous parts of the plain form are 0; one reciprocal for both
+      // ratios; |y| compared as bits, off the FP64 pipe, which bounds this
+      // kernel (256^3: 8.2 ms against 12.3 with the sums and divisions apart)
       acc5d = 0.0;
       acc3d = 0.0;
 #pragma unroll
       for (int w = 0; w < W; ++w) {
-        const double q5 = (double)a5[w] + q5s, q3 = (double)a3[w] + q3s;
-        const double sk = a.atol + a.rtol * fmax(fabs((double)yv[w] + ys), fabs((double)yn[w] + yns));
-        const double r5 = q5 / sk, r3 = q3 / sk;
+        const long long m = max(__double_as_longlong(fabs((double)yv[w])),
+                                __double_as_longlong(fabs((double)yn[w])));
+        const double isk = 1.0 / (a.atol + a.rtol * __longlong_as_double(m));
+        const double r5 = (double)a5[w] * isk, r3 = (double)a3[w] * isk;
         acc5d += r5 * r5;
         acc3d += r3 * r3;
       }
@@ -835,17 +853,22 @@ __global__ void __launch_bounds__(256, 2) k_dopri_final_vel(const float *__restr
   }
 }
 
-static int lincomb(Ctx *c, const Vec &base, Vec &out, const LinArgs &args) {
-  const long long nf = c->g.Nf;
-  prof_begin(c, KK_LINCOMB);
-  if (c->mixed) {
-    k_lincomb<float><<<stream_grid(nf / 4), 256, 0, c->stream>>>(
-        (const float *)base.fl, base.sc, (float *)out.fl, out.sc, args, nf);
-  } else {
-    k_lincomb<double><<<stream_grid(nf / 2), 256, 0, c->stream>>>(
-        (const double *)base.fl, base.sc, (double *)out.fl, out.sc, args, nf);
+template <typename T, int NT>
+static void lincomb_launch(Ctx *c, const Vec &base, Vec &out, const LinArgs &args) {
+  if constexpr (NT > 0) {  // no terms: a copy (dense output at the step's start)
+    if (args.n < NT) return lincomb_launch<T, NT - 1>(c, base, out, args);
   }
-  prof_end(c, KK_LINCOMB, (double)(args.n + 2) * nf * c->tsize);
+  const long long nf = c->g.Nf;
+  k_lincomb<T, NT><<<stream_grid(nf / Vec4<T>::W), 256, 0, c->stream>>>(
+      (const T *)base.fl, base.sc, (T *)out.fl, out.sc, args, nf);
+}
+static int lincomb(Ctx *c, const Vec &base, Vec &out, const LinArgs &args) {
+  prof_begin(c, KK_LINCOMB);
+  if (c->mixed)
+    lincomb_launch<float, kMaxTerms>(c, base, out, args);
+  else
+    lincomb_launch<double, kMaxTerms>(c, base, out, args);
+  prof_end(c, KK_LINCOMB, (double)(args.n + 2) * c->g.Nf * c->tsize);
   return check_launch(c, "k_lincomb");
 }
 
@@ -1177,6 +1200,7 @@ static int try_body(Ctx *c) {
     f.e5[j] = DB[sidx] - bhh;
     f.e3[j] = DE3[sidx];
   }
+  for (int i = 0; i < 3; ++i) f.bhh[i] = DBHH[i];
   f.dt = c->dt_dev;
   f.rtol = c->cfg.rtol;
   f.atol = c->cfg.atol;
