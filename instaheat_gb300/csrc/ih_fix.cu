@@ -16,9 +16,10 @@ namespace ih {
 // thread (b, n1) holds x[n1 + R1 n2] of column b, an R2-point DFT, the table
 // twiddle, one exchange through shared memory, an R1-point DFT.  Tiles of 8
 // columns are 128-byte lines.  At 256^3 (55 launches of a DOPRI853 step, 3 to
-// 4 arrays each): 338 us a launch against 1298 us on the FP64 pipe, 2.4 TB/s;
-// 128^3: 57 against 163 us.  Bound by the conversions (FP64 pipe, 1.9 clocks
-// per complex value and SM) and the integer pipe (about 1.7) side by side.
+// 4 arrays each): 272 us a launch against 1298 us on the FP64 pipe, 3.0 TB/s;
+// 128^3: 47 against 163 us.  Both conversions are on the integer pipe: on the
+// FP64 pipe (1.9 clocks per complex value and SM) they bound the pass, 340 and
+// 57 us (inputs alone on the integer pipe 295 / 51, outputs alone 271 / 49).
 template <int L> struct FxFac;
 template <> struct FxFac<8> { static constexpr int R1 = 4, R2 = 2; };
 template <> struct FxFac<16> { static constexpr int R1 = 4, R2 = 4; };
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), L <= 256 ? 512 / fx_thread
   const FxScale sc = fx_scale(m, fx_p<L>());
   if (q < R1) {
     fx2 v[R2];
-    fx_load(x, sc, v);
+    fx_load<true>(x, sc, v);
     fx_dft<R2, S>(v);
 #pragma unroll
     for (int k2 = 0; k2 < R2; ++k2)
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), L <= 256 ? 512 / fx_thread
     if (col) {
 #pragma unroll
       for (int k1 = 0; k1 < R1; ++k1)
-        base[(long long)(q + R2 * k1) * sj] = fx_store(u[k1], sc.out + 2, sc);
+        base[(long long)(q + R2 * k1) * sj] = fx_store<true>(u[k1], sc.out + 2, sc);
     }
   }
 }
@@ -107,12 +108,14 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), L <= 256 ? 512 / fx_thread
 // in Q62 (first derivative 0 on the Nyquist index).  ACC (the y round trip):
 // the coefficient of d2 takes -kz^2 too (cz, at the scale of c2), so that d2
 // is the y and z part of the laplacian, and the x part in out1 is added.
-// At 256^3: 378 us a round trip against 1359 us on the FP64 pipe.
+// At 256^3: 347 us a round trip against 1359 us on the FP64 pipe, 128^3 58 us
+// against 178.  Inputs convert on the FP64 pipe, outputs (two per input) on the
+// integer pipe: 375 us with both on the former, 388 on the latter.
 // Between the transforms the spectrum is brought to 2 bits above the inverse
 // transform's p (the coefficients take 2), so no precision is lost whatever
 // its size.
 template <int L, int B, bool ACC>
-__global__ void __launch_bounds__(fx_threads<L, B>()) k_fx_rt(
+__global__ void __launch_bounds__(fx_threads<L, B>(), L <= 256 ? 384 / fx_threads<L, B>() : 1) k_fx_rt(
     const double2 *__restrict__ in, double2 *__restrict__ out0, double2 *out1, long long sj,
     long long so, int mz, FxTab tw, const long long *__restrict__ c1,
     const long long *__restrict__ c2, const long long *__restrict__ cz, int e1, int e2) {
@@ -145,7 +148,7 @@ __global__ void __launch_bounds__(fx_threads<L, B>()) k_fx_rt(
   const FxScale sc = fx_scale(m, fx_p<L>());
   if (q < R1) {
     fx2 v[R2];
-    fx_load(x, sc, v);
+    fx_load<false>(x, sc, v);
     fx_dft<R2, -1>(v);
 #pragma unroll
     for (int k2 = 0; k2 < R2; ++k2)
@@ -167,32 +170,40 @@ __global__ void __launch_bounds__(fx_threads<L, B>()) k_fx_rt(
   __syncthreads();  // ex0 is rewritten below (also where fx_col_max has no barrier)
   const int room = fx_room(mu, fx_p<L>() + 2);
   const FxShift sh = fx_shift_of(room);
+  // the spectrum waits in the thread's own slots of ex1 between the two
+  // inverse transforms (in registers it would halve the resident CTAs)
+  auto slot = [&](int k1) { return (k1 * R2 + q) * B + b; };
+  fx2 w[R1];
   if (q < R2) {
 #pragma unroll
-    for (int k1 = 0; k1 < R1; ++k1) u[k1] = fx_shift(u[k1], sh);
+    for (int k1 = 0; k1 < R1; ++k1) {
+      const fx2 v = fx_shift(u[k1], sh);
+      ex1[slot(k1)] = v;
+      const long long c = __ldg(c1 + q + R2 * k1);
+      const int ch = fx_hi(c), cl = (int)c;
+      w[k1] = fx_mk(-fx_mul(v.y, ch, cl), fx_mul(v.x, ch, cl));  // i k X
+    }
+    fx_dft<R1, +1>(w);
+#pragma unroll
+    for (int n1 = 0; n1 < R1; ++n1)
+      ex0[fx_row<L, B>(q * R1 + n1) * B + b] =
+          n1 == 0 ? fx_quarter(w[n1]) : fx_cmul<+1>(w[n1], fx_tw(tw, n1 * q));
     const long long z2 = ACC ? __ldg(cz + min(z0 + b, mz - 1)) : 0;
 #pragma unroll
-    for (int o = 0; o < 2; ++o) {
-      fx2 w[R1];
-#pragma unroll
-      for (int k1 = 0; k1 < R1; ++k1) {
-        if (o == 0) {
-          const long long c = __ldg(c1 + q + R2 * k1);
-          const int ch = fx_hi(c), cl = (int)c;
-          w[k1] = fx_mk(-fx_mul(u[k1].y, ch, cl), fx_mul(u[k1].x, ch, cl));  // i k X
-        } else {
-          const long long c = __ldg(c2 + q + R2 * k1) + z2;
-          const int ch = fx_hi(c), cl = (int)c;
-          w[k1] = fx_mk(fx_mul(u[k1].x, ch, cl), fx_mul(u[k1].y, ch, cl));
-        }
-      }
-      fx_dft<R1, +1>(w);
-      fx2 *e = o ? ex1 : ex0;
-#pragma unroll
-      for (int n1 = 0; n1 < R1; ++n1)
-        e[fx_row<L, B>(q * R1 + n1) * B + b] =
-            n1 == 0 ? fx_quarter(w[n1]) : fx_cmul<+1>(w[n1], fx_tw(tw, n1 * q));
+    for (int k1 = 0; k1 < R1; ++k1) {
+      const fx2 v = ex1[slot(k1)];
+      const long long c = __ldg(c2 + q + R2 * k1) + z2;
+      const int ch = fx_hi(c), cl = (int)c;
+      w[k1] = fx_mk(fx_mul(v.x, ch, cl), fx_mul(v.y, ch, cl));  // -k^2 X
     }
+    fx_dft<R1, +1>(w);
+  }
+  __syncthreads();  // every slot of ex1 is read
+  if (q < R2) {
+#pragma unroll
+    for (int n1 = 0; n1 < R1; ++n1)
+      ex1[fx_row<L, B>(q * R1 + n1) * B + b] =
+          n1 == 0 ? fx_quarter(w[n1]) : fx_cmul<+1>(w[n1], fx_tw(tw, n1 * q));
   }
   __syncthreads();
   if (q < R1) {
@@ -210,7 +221,7 @@ __global__ void __launch_bounds__(fx_threads<L, B>()) k_fx_rt(
 #pragma unroll
         for (int n2 = 0; n2 < R2; ++n2) {
           double2 *d = dst + (long long)(q + R1 * n2) * sj;
-          double2 r = fx_store(v[n2], e + (o ? e2 : e1), sc);
+          double2 r = fx_store<true>(v[n2], e + (o ? e2 : e1), sc);
           if (ACC && o == 1) {
             const double2 a = *d;
             r.x += a.x;
@@ -230,9 +241,9 @@ __global__ void __launch_bounds__(fx_threads<L, B>()) k_fx_rt(
 // z[E t + e + A q] (e < E = A / B, q < B; register E q + e) on the real side,
 // one transpose through the warp's shared scratch in between.  Scratch
 // columns are swizzled and rows padded so that the eight 16-byte accesses of
-// a phase hit different banks.  At 256^3: r2c 196 us an array against 606 us,
-// c2r of four arrays 625 against 2564 us (FP64 pipe, wide rows and a warp per
-// row).
+// a phase hit different banks.  At 256^3: r2c 144 us an array against 606 us,
+// c2r of four arrays 449 against 2564 us (FP64 pipe, wide rows and a warp per
+// row); both conversions on the integer pipe (on the FP64 pipe 195 and 625 us).
 template <int H> struct FxZ;
 template <> struct FxZ<4> { static constexpr int A = 2, B = 2; };
 template <> struct FxZ<8> { static constexpr int A = 4, B = 2; };
@@ -410,7 +421,7 @@ __global__ void __launch_bounds__(32 * kFxWarps) k_fx_zr2c(
   }
   const FxScale sc = fx_scale(fx_row_max<H>(fx_max_in(x)), G::pr);
   fx2 v[A];
-  fx_load(x, sc, v);
+  fx_load<true>(x, sc, v);
   fx_z_forward<H>(v, t, &xs[warp][grp * G::X], twh);
   fx2 xH;
   fx_z_r2c_post<H>(v, t, gbase, twz, xH);
@@ -418,11 +429,11 @@ __global__ void __launch_bounds__(32 * kFxWarps) k_fx_zr2c(
     double2 *dst = out + blockIdx.y * ostride + row * (H + 1);
 #pragma unroll
     for (int m = 0; m < A; ++m) {
-      double2 r = fx_store(v[m], sc.out + 4, sc);
+      double2 r = fx_store<true>(v[m], sc.out + 4, sc);
       if (m == 0 && t == 0) r.x += 2 * H * x0;
       dst[t + B * m] = r;
     }
-    if (t == 0) dst[H] = fx_store(xH, sc.out + 4, sc);
+    if (t == 0) dst[H] = fx_store<true>(xH, sc.out + 4, sc);
   }
 }
 
@@ -435,15 +446,15 @@ __device__ __forceinline__ void fx_z_fetch(const double2 *row, int t, bool valid
     x[m] = valid ? row[t + FxZG<H>::B * m] : make_double2(0.0, 0.0);
   xH = (valid && t == 0) ? row[H] : make_double2(0.0, 0.0);
 }
-template <int H>
+template <int H, bool BITS>
 __device__ __forceinline__ FxScale fx_z_load(double2 (&x)[FxZG<H>::A], double2 xH,
                                              fx2 (&v)[FxZG<H>::A], fx2 &vH) {
   double2 h[1] = {xH};
   fx2 u[1];
   const FxScale sc =
       fx_scale(fx_row_max<H>(max(fx_max_in(x), fx_max_in(h))), FxZG<H>::pc);
-  fx_load(x, sc, v);
-  fx_load(h, sc, u);
+  fx_load<BITS>(x, sc, v);
+  fx_load<BITS>(h, sc, u);
   vH = u[0];
   return sc;
 }
@@ -468,7 +479,7 @@ __global__ void __launch_bounds__(32 * kFxWarps) k_fx_zc2r(
   if (fx_absbits(x0) >= 0x7ff00000u) x0 = 0.0;
   if (t == 0) x[0].x -= x0;
   fx2 v[A], vH;
-  const FxScale sc = fx_z_load<H>(x, xH, v, vH);
+  const FxScale sc = fx_z_load<H, true>(x, xH, v, vH);
   fx_z_c2r_prep<H>(v, vH, t, gbase, twz);
   fx_z_inverse<H>(v, t, &xs[warp][grp * G::X], twh);
   if (valid) {
@@ -477,7 +488,7 @@ __global__ void __launch_bounds__(32 * kFxWarps) k_fx_zc2r(
     for (int q = 0; q < B; ++q) {
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        double2 r = fx_store(v[E * q + e], sc.out + 4, sc);
+        double2 r = fx_store<true>(v[E * q + e], sc.out + 4, sc);
         r.x += x0;
         r.y += x0;
         dst[E * t + e + A * q] = r;
@@ -492,9 +503,12 @@ __global__ void __launch_bounds__(32 * kFxWarps) k_fx_zc2r(
 // their FP64 sums, the six products d_i phi d_j phi and their r2c.  d/dx,
 // d/dy, d/dz stay integers with a shared exponent per row, brought to 2^62;
 // products of two rows are the upper 64 bits and go into the forward transform
-// without a conversion.  rho and p are FP64.  At 256^3: 2.50 ms against 5.90 ms
-// on the FP64 pipe (wide rows); at 128^3 0.262 against 0.915 ms (a warp per
-// row).
+// without a conversion.  rho and p are FP64.  At 256^3: 2.44 ms against 5.90 ms
+// on the FP64 pipe (wide rows); at 128^3 0.181 against 0.915 ms (a warp per
+// row).  It takes about 2500 instructions per complex point and issues on 0.3
+// to 0.4 of the cycles: latency, with the few warps that the three derivative
+// rows leave room for (H = 64: 8 resident warps 221 us, 12 201, 16 181; H = 128
+// is held to 8 by its 96 KB per CTA).  Outputs convert on the integer pipe.
 template <int H> struct FxZSmem {
   fx2 xs[kFxWarps][FxZG<H>::G * FxZG<H>::X];
   fx2 grad[kFxWarps][2][FxZG<H>::A][32];  // d/dx, d/dy: thread-private
@@ -502,7 +516,7 @@ template <int H> struct FxZSmem {
 };
 
 template <int H, bool ZSRC>
-__global__ void __launch_bounds__(32 * kFxWarps, 2) k_fx_z_rhs(
+__global__ void __launch_bounds__(32 * kFxWarps, H == 64 ? 4 : H < 64 ? 3 : 2) k_fx_z_rhs(
     const double2 *d4, long long dstride, const double *__restrict__ yfl, const double *ysc,
     double *lap, double *pout, double *rhoout, double2 *s6, long long sstride4, double2 *s6b,
     int gw, double *partials, Geom g, FxTab twh, FxTab twz, const long long *__restrict__ ckz,
@@ -530,7 +544,7 @@ __global__ void __launch_bounds__(32 * kFxWarps, 2) k_fx_z_rhs(
     fx_z_fetch<H>(d4 + (ZSRC && a == 2 ? 4 : a) * dstride + row * (H + 1), t, valid, x, xH);
     if (ZSRC && a == 2) {  // i kz Z / nz: the constant drops out
       if (t == 0) x[0] = make_double2(0.0, 0.0);
-      sc = fx_z_load<H>(x, xH, v, vH);
+      sc = fx_z_load<H, false>(x, xH, v, vH);
 #pragma unroll
       for (int m = 0; m < A; ++m) {
         const long long c = __ldg(ckz + t + B * m);
@@ -540,7 +554,7 @@ __global__ void __launch_bounds__(32 * kFxWarps, 2) k_fx_z_rhs(
       vH = fx_mk(0, 0);  // zero on the Nyquist index
       e = sc.out + 2 + ekz - lognz;
     } else {
-      sc = fx_z_load<H>(x, xH, v, vH);
+      sc = fx_z_load<H, false>(x, xH, v, vH);
       e = sc.out;
     }
     fx_z_c2r_prep<H>(v, vH, t, gbase, twz);
@@ -552,7 +566,7 @@ __global__ void __launch_bounds__(32 * kFxWarps, 2) k_fx_z_rhs(
 #pragma unroll
         for (int q = 0; q < B; ++q) {
 #pragma unroll
-          for (int j = 0; j < E; ++j) dst[E * t + j + A * q] = fx_store(v[E * q + j], e, sc);
+          for (int j = 0; j < E; ++j) dst[E * t + j + A * q] = fx_store<true>(v[E * q + j], e, sc);
         }
       }
     } else {
@@ -592,11 +606,11 @@ __global__ void __launch_bounds__(32 * kFxWarps, 2) k_fx_z_rhs(
     double2 *ro = reinterpret_cast<double2 *>(rhoout) + row * H;
     auto grad2 = [&](long long gx, long long gy, long long gz) {
       if (slow) {  // extreme rows: in FP64
-        const double fx = fx_out(gx, ex[0]) * post[0], fy = fx_out(gy, ex[1]) * post[1],
-                     fz = fx_out(gz, ex[2]) * post[2];
+        const double fx = fx_out<true>(gx, ex[0]) * post[0], fy = fx_out<true>(gy, ex[1]) * post[1],
+                     fz = fx_out<true>(gz, ex[2]) * post[2];
         return fx * fx + fy * fy + fz * fz;
       }
-      return fx_out((fx_mul(gx, gx) >> r0) + (fx_mul(gy, gy) >> r1) + (fx_mul(gz, gz) >> r2), eg);
+      return fx_out<true>((fx_mul(gx, gx) >> r0) + (fx_mul(gy, gy) >> r1) + (fx_mul(gz, gz) >> r2), eg);
     };
 #pragma unroll
     for (int q = 0; q < B; ++q) {
@@ -675,8 +689,8 @@ __global__ void __launch_bounds__(32 * kFxWarps, 2) k_fx_z_rhs(
       so.slow = slow;
       so.post = pa * pb;
 #pragma unroll
-      for (int m = 0; m < A; ++m) dst[t + B * m] = fx_store(v[m], e, so);
-      if (t == 0) dst[H] = fx_store(xH, e, so);
+      for (int m = 0; m < A; ++m) dst[t + B * m] = fx_store<true>(v[m], e, so);
+      if (t == 0) dst[H] = fx_store<true>(xH, e, so);
     }
   }
 }

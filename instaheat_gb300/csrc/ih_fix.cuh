@@ -213,14 +213,45 @@ __device__ __forceinline__ FxScale fx_scale(unsigned m, int p) {
   s.out = -s.in;
   return s;
 }
-__device__ __forceinline__ long long fx_in(double a, const FxScale &s) {
+// Conversions on the FP64 pipe (2.1 per clock and SM) ...
+__device__ __forceinline__ long long fx_in_pipe(double a, const FxScale &s) {
   return __double2ll_rn(
       __hiloint2double(__double2hiint(a) + s.in * (1 << 20), __double2loint(a)));
 }
-__device__ __forceinline__ double fx_out(long long v, int e) {
+__device__ __forceinline__ double fx_out_pipe(long long v, int e) {
   const double d = __ll2double_rn(v);
   const int h = __double2hiint(d);
   return __hiloint2double(h == 0 ? 0 : h + e * (1 << 20), __double2loint(d));
+}
+// ... and on the integer pipe (about 3.5 per clock and SM): the mantissa, its
+// leading one put in, shifted to the pencil's exponent, and back by a count of
+// leading zeros; both round to nearest
+__device__ __forceinline__ long long fx_in_bits(double a, const FxScale &s) {
+  const unsigned hi = (unsigned)__double2hiint(a), lo = (unsigned)__double2loint(a);
+  // a = m 2^(e - 1075) with m < 2^53; m 2^10 is below 2^63 and goes right by
+  // r > 0 bits, one of them in the rounding
+  const int e = (int)((hi >> 20) & 0x7ff);
+  unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 10;
+  // (shr clamps: a count of 64 or more, as for zeros, gives 0)
+  asm("shr.u64 %0, %0, %1;" : "+l"(m) : "r"(1084 - s.in - e));
+  const long long t = (long long)((m + 1) >> 1);
+  return (int)hi < 0 ? -t : t;
+}
+__device__ __forceinline__ double fx_out_bits(long long v, int e) {
+  const unsigned long long u = (unsigned long long)(v < 0 ? -v : v);
+  const int lz = __clzll((long long)u);
+  const unsigned long long n = u << (lz & 63);
+  const unsigned long long m = (n >> 11) + ((n >> 10) & 1);  // 2^52 .. 2^53
+  const int h = (int)(m >> 32) + (1085 - lz + e) * (1 << 20);
+  return __hiloint2double(u == 0 ? 0 : (h | ((int)(v >> 32) & (int)0x80000000)), (int)(unsigned)m);
+}
+template <bool BITS>
+__device__ __forceinline__ long long fx_in(double a, const FxScale &s) {
+  return BITS ? fx_in_bits(a, s) : fx_in_pipe(a, s);
+}
+template <bool BITS>
+__device__ __forceinline__ double fx_out(long long v, int e) {
+  return BITS ? fx_out_bits(v, e) : fx_out_pipe(v, e);
 }
 template <int R>
 __device__ __forceinline__ unsigned fx_max_in(const double2 (&x)[R]) {
@@ -232,7 +263,7 @@ __device__ __forceinline__ unsigned fx_max_in(const double2 (&x)[R]) {
   }
   return low ? m | 1u : m;  // 0 only where every value is 0
 }
-template <int R>
+template <bool BITS, int R>
 __device__ __forceinline__ void fx_load(double2 (&x)[R], const FxScale &s, fx2 (&v)[R]) {
   if (s.slow) {
 #pragma unroll
@@ -242,11 +273,12 @@ __device__ __forceinline__ void fx_load(double2 (&x)[R], const FxScale &s, fx2 (
     }
   }
 #pragma unroll
-  for (int i = 0; i < R; ++i) v[i] = fx_mk(fx_in(x[i].x, s), fx_in(x[i].y, s));
+  for (int i = 0; i < R; ++i) v[i] = fx_mk(fx_in<BITS>(x[i].x, s), fx_in<BITS>(x[i].y, s));
 }
 // value of v at exponent e, through the slow factor where the pencil has one
+template <bool BITS>
 __device__ __forceinline__ double2 fx_store(fx2 v, int e, const FxScale &s) {
-  double2 r = make_double2(fx_out(v.x, e), fx_out(v.y, e));
+  double2 r = make_double2(fx_out<BITS>(v.x, e), fx_out<BITS>(v.y, e));
   if (s.slow) {
     r.x *= s.post;
     r.y *= s.post;
