@@ -203,6 +203,7 @@ static int create(const ih_params *p, Ctx *c) {
   IH_TRY(alloc_vec(c, c->ytmp));
   IH_TRY(alloc_vec(c, c->k[1]));
   IH_TRY(mask_init(c, c->mask));
+  if (!c->mixed) IH_TRY(tensor_table(c));
   IH_CUDA(c, cudaStreamSynchronize(c->stream));
   return IH_OK;
 }
@@ -216,6 +217,7 @@ static void destroy(Ctx *c) {
   for (void *p : c->fx_tw)
     if (p) cudaFree(p);
   if (c->fx_coef) cudaFree(c->fx_coef);
+  if (c->tensor_coef) cudaFree(c->tensor_coef);
   if (c->spec[0]) cudaFree(c->spec[0]);
   if (c->rbuf[0]) cudaFree(c->rbuf[0]);
   if (c->gscratch) cudaFree(c->gscratch);

@@ -246,6 +246,7 @@ struct Ctx {
   void *fx_tw[4] = {};
   void *fx_coef = nullptr;
   int fx_e[5] = {};
+  void *tensor_coef = nullptr;  // FP64 form: projection coefficients (k_tensor_table)
   std::string tune_report;
 };
 constexpr int kFxAll = 0x5b;
@@ -384,6 +385,7 @@ int fft_any(Ctx *c, const double *in_dev, double *out_c_dev);
 int get_field(Ctx *c, int which, double *dev_out);
 int read_output(Ctx *c, ih_output *out);
 int mask_init(Ctx *c, void *mask);
+int tensor_table(Ctx *c);
 int convert_add(Ctx *c, const void *a, double add, long long n, double *out);
 
 // learned proposer (ih_mlp.cu, ih_stepper.cu)

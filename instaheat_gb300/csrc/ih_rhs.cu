@@ -307,16 +307,16 @@ __global__ void k_next_sc(const NextLin nl, const double *ksc, double *outsc) {
   outsc[s] = nl.basesc[s] + dt * acc;
 }
 
-// update_h with the TT projection (toolbox.c:311-346, 363-397).  s holds the
-// six S_ij spectra, spectra 4 and 5 at s + 5M.
-// NEXT: also the next stage's input at the tensor entries of y (nl).
-template <typename T, bool NEXT>
-__global__ void __launch_bounds__(256, (sizeof(T) == 4 ? (NEXT ? 3 : 4) : 2)) k_update_h(
-    const C2<T> *__restrict__ s, T *y, T *__restrict__ out, const RhsScalars *rs, Geom g,
+// update_h with the TT projection (toolbox.c:311-346, 363-397), FP32: also the
+// next stage's input at the tensor entries of y (nl).  s holds the six S_ij
+// spectra, spectra 4 and 5 at s + 5M.
+__global__ void __launch_bounds__(256, 3) k_update_h_next(
+    const float2 *__restrict__ s, float *y, float *__restrict__ out, const RhsScalars *rs, Geom g,
     const NextLin nl, double *outsc) {
+  typedef float T;
   const long long M = g.M;
   const TensorConsts<T> tc(rs);
-  const T dt = NEXT ? (T)*nl.dt : (T)0;
+  const T dt = (T)*nl.dt;
   T mx = 0;
   const unsigned mz_magic = g.mz_magic;
   const int mz_shift = g.mz_shift, logny = g.logny;
@@ -344,9 +344,98 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 ? (NEXT ? 3 : 4) : 2)) k_
       ksq = q.ksq;
       tensor_sources<T>(m, q, v, n0, n1);
     }
-    mx = fmax(mx, tensor_eom<T, NEXT>(g, id, n0, n1, ksq, tc, y, out, nl, dt));
+    mx = fmax(mx, tensor_eom<T, true>(g, id, n0, n1, ksq, tc, y, out, nl, dt));
   }
   dh_max_store<T>(mx, outsc);
+}
+
+// The FP64 form's update_h from a table.  The projection is n0 = sum_a alpha_a
+// S_a, n1 = sum_a beta_a S_a with real coefficients that depend on the mode
+// alone (tensor_coef), up to signs that flip with kx and ky; forming them
+// (|k|^2, a division, the products of k) is two thirds of the FP64
+// instructions of a mode, and the FP64 pipe is what bounds this kernel.  The
+// table holds alpha, beta and |k|^2 of the octant kx, ky, kz >= 0; a thread
+// reads one entry and handles the up to four modes (+-kx, +-ky, kz) that share
+// it: 26 bytes of table per mode beside 224 of data.  256^3: 0.594 ms against
+// 1.592 ms with the coefficients formed per mode (3.2 TB/s; 37 FP64
+// instructions per mode are 0.59 ms); 64^3: 21 us against 42.
+constexpr int kTensorCoefs = 13;
+__global__ void k_tensor_table(double *coef, long long Mo, Geom g) {
+  const int nyh = g.ny / 2 + 1;
+  for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < Mo;
+       o += (long long)gridDim.x * blockDim.x) {
+    const int k = (int)(o % g.mz), j = (int)(o / g.mz % nyh), i = (int)(o / g.mz / nyh);
+    const double kx = kxf_of(g, i), ky = kyf_of(g, j), kz = kzf_of(g, k),
+                 ksq = ksq64(g, i, j, k);
+    const double inv = o ? 1.0 / ksq : 0.0;
+    const int branch = k ? 0 : (j ? 1 : 2);
+    for (int a = 0; a < 6; ++a) {
+      double al = 0.0, be = 0.0;  // the zero mode has no sources
+      if (o) tensor_coef<double>(a, branch, kx, ky, kz, kx * inv, ky * inv, kz * inv, al, be);
+      coef[a * Mo + o] = al;
+      coef[(6 + a) * Mo + o] = be;
+    }
+    coef[12 * Mo + o] = ksq;
+  }
+}
+// v, negated where f
+__device__ __forceinline__ double flip(double v, int f) {
+  return __hiloint2double(__double2hiint(v) ^ (f << 31), __double2loint(v));
+}
+// per: modes of an octant entry per thread (4, or fewer with the rest on
+// gridDim.y where the grid would otherwise leave SMs idle)
+template <bool NEXT>
+__global__ void __launch_bounds__(128) k_update_h_tab(
+    const double2 *__restrict__ s, double *y, double *__restrict__ out, const RhsScalars *rs,
+    Geom g, const double *__restrict__ coef, int Mo, const NextLin nl, int per) {
+  const int o = blockIdx.x * blockDim.x + threadIdx.x;
+  if (o >= Mo) return;
+  const int nyh = g.ny / 2 + 1;
+  const int r = o / g.mz, k = o - r * g.mz, i = r / nyh, j = r - i * nyh;
+  const long long M = g.M;
+  const TensorConsts<double> tc(rs);
+  const double dt = NEXT ? *nl.dt : 0.0;
+  double al[6], be[6];
+#pragma unroll
+  for (int a = 0; a < 6; ++a) {
+    al[a] = coef[(long long)a * Mo + o];
+    be[a] = coef[(long long)(6 + a) * Mo + o];
+  }
+  const double ksq = coef[(long long)12 * Mo + o];
+  for (int q = blockIdx.y * per; q < (int)(blockIdx.y + 1) * per; ++q) {
+    const int sx = q & 1, sy = q >> 1;
+    if ((sx && (i == 0 || 2 * i == g.nx)) || (sy && (j == 0 || 2 * j == g.ny))) continue;
+    const long long id =
+        ((long long)(sx ? g.nx - i : i) * g.ny + (sy ? g.ny - j : j)) * g.mz + k;
+    double2 v[6];
+#pragma unroll
+    for (int a = 0; a < 6; ++a) v[a] = s[(a < 4 ? a : a + 1) * M + id];
+    // a coefficient of S_ab in n_cd changes sign with kx (ky) when x (y)
+    // occurs an odd number of times in a, b, c, d; n0 is xx (yy for kz = ky =
+    // 0) and n1 xy (xz for kz = 0, yz for kz = ky = 0)
+    const int sxy = sx ^ sy;
+    const int f1[6] = {sxy, 0, k ? sy : 0, sxy, k ? sx : (j ? sxy : 0), sxy};
+    const int f0[6] = {0, sxy, sx, 0, sy, 0};
+    double2 n0 = make_double2(0.0, 0.0), n1 = n0;
+#pragma unroll
+    for (int a = 0; a < 6; ++a) {
+      const double ca = flip(al[a], f0[a]), cb = flip(be[a], f1[a]);
+      n0.x += ca * v[a].x;
+      n0.y += ca * v[a].y;
+      n1.x += cb * v[a].x;
+      n1.y += cb * v[a].y;
+    }
+    if (id == 0) n0 = n1 = make_double2(0.0, 0.0);
+    tensor_eom<double, NEXT>(g, id, n0, n1, ksq, tc, y, out, nl, dt);
+  }
+}
+int tensor_table(Ctx *c) {
+  const Geom &g = c->g;
+  const long long Mo = (long long)(g.nx / 2 + 1) * (g.ny / 2 + 1) * g.mz;
+  IH_CUDA(c, cudaMalloc(&c->tensor_coef, sizeof(double) * kTensorCoefs * Mo));
+  c->dev_bytes += sizeof(double) * kTensorCoefs * Mo;
+  k_tensor_table<<<grid_for(Mo, 256, 1), 256, 0, c->stream>>>((double *)c->tensor_coef, Mo, g);
+  return check_launch(c, "k_tensor_table");
 }
 
 // update_h without the next stage input, one mode ahead: the ten loads of
@@ -436,16 +525,25 @@ static int tensor_last_pass_t(Ctx *c, C2<T> *s, T *y, T *out, double *outsc,
     IH_TRY((fft_xy<T>(c, s, M, 4, 0, -1)));
     IH_TRY((fft_xy<T>(c, s + 5 * M, M, 2, 0, -1)));
   }
-  const unsigned gm = grid_for(M, 256, 4);
   prof_begin(c, KK_UPDATE_H);
-  if (next) {
-    k_update_h<T, true><<<gm, 256, 0, c->stream>>>(s, y, out, c->rs, g, *next, outsc);
-  } else if constexpr (sizeof(T) == 4) {
-    k_update_h_pf<T><<<gm, 256, 0, c->stream>>>(s, y, out, c->rs, g, c->skip_pos, outsc);
-  } else {  // FP64: ALU-bound; the prefetching form would spill
-    NextLin none{};
-    none.skip_pos = c->skip_pos;
-    k_update_h<T, false><<<gm, 256, 0, c->stream>>>(s, y, out, c->rs, g, none, outsc);
+  if constexpr (sizeof(T) == 4) {
+    const unsigned gm = grid_for(M, 256, 4);
+    if (next)
+      k_update_h_next<<<gm, 256, 0, c->stream>>>(s, y, out, c->rs, g, *next, outsc);
+    else
+      k_update_h_pf<T><<<gm, 256, 0, c->stream>>>(s, y, out, c->rs, g, c->skip_pos, outsc);
+  } else {
+    const int Mo = (g.nx / 2 + 1) * (g.ny / 2 + 1) * g.mz;
+    NextLin nl{};
+    if (next) nl = *next;
+    else nl.skip_pos = c->skip_pos;
+    // four CTAs of 128 threads on every SM, or the modes of an entry on
+    // separate threads
+    const int nb = (Mo + 127) / 128, wave = 4 * c->num_sms;
+    const int per = nb >= wave ? 4 : (2 * nb >= wave ? 2 : 1);
+    auto kf = next ? k_update_h_tab<true> : k_update_h_tab<false>;
+    kf<<<dim3(nb, 4 / per), 128, 0, c->stream>>>(s, y, out, c->rs, g,
+                                                 (const double *)c->tensor_coef, Mo, nl, per);
   }
   prof_end(c, KK_UPDATE_H,
            6.0 * M * sizeof(C2<T>) +
