@@ -182,7 +182,7 @@ int ih_variance_host(ih_context *c, double mean, const double *f_host, size_t n,
  * pass, of the x and y derivative round trips, of the last tensor x pass and
  * the kz slab widths of the tensor sources' y/x passes and, where it
  * applies, the plane-major tail of the tensor sources (pass 8 below) of the
- * RHS on the context's scratch spectra and keeps the fastest per pass.  Until it is called the passes use the shared-memory Stockham
+ * RHS on the context's scratch spectra and keeps the fastest per pass.  Until it is called the passes use the register two-step
  * engine.  Results are identical across variants up to rounding.  The report
  * lists the timings and the choice (valid until the next ih_autotune). */
 int ih_autotune(ih_context *c);
@@ -209,9 +209,11 @@ const char *ih_autotune_report(const ih_context *c);
  * spectra instead of six; mixed form at 256^3 only, IH_ERR_ARG elsewhere;
  * 0: the row and column passes), 9 = the passes of the FP64 form that run in
  * 64-bit block fixed point on the integer pipe (a mask of 1 << pass over the
- * passes 0, 1, 3, 4 and 6, IH_FFT_FIXED_ALL by default on power-of-two grids,
- * 0 = none; IH_ERR_ARG for a mask other than 0 in the mixed form and on
- * radix-3 grids; pinning an engine of one of these passes takes its bit out);
+ * passes 0, 1, 3, 4 and 6; by default all that the grid has: x and y axes of
+ * 2^a, 3 2^a and 9 2^a points, z rows of 2^a and 3 2^a, the round trips where
+ * all three are; IH_FFT_FIXED_ALL = every pass, 0 = none; IH_ERR_ARG for a pass
+ * that has no such form on the grid and for any in the mixed form; pinning an
+ * engine of one of these passes takes its bit out);
  * engine IH_FFT_STOCKHAM, IH_FFT_TWOSTEP (register two-step,
  * 128-byte tiles), IH_FFT_TWOSTEP_HALF (64-byte tiles), IH_FFT_PIPELINED
  * (register two-step in persistent CTAs that copy the next tile in with

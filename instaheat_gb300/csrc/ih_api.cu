@@ -164,10 +164,13 @@ static int create(const ih_params *p, Ctx *c) {
   make_geom(p, &c->g);
   c->mixed = p->precision == IH_PREC_MIXED;
   c->tsize = c->mixed ? 4 : 8;
+  if (c->mixed) c->xy_var[0] = c->xy_var[1] = FV_THREESTEP;
   c->noise_eta = c->mixed ? kDefaultNoiseEta : 0.0;
   IH_CUDA(c, cudaSetDevice(p->device));
   IH_CUDA(c, cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, p->device));
   IH_CUDA(c, cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
+  IH_CUDA(c, cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
+  for (auto &e : c->fork) IH_CUDA(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   const Geom &g = c->g;
   const size_t cs = 2 * c->tsize;  // complex element
   IH_TRY(fft_tables(c));
@@ -210,6 +213,7 @@ static int create(const ih_params *p, Ctx *c) {
 
 static void destroy(Ctx *c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
+  if (c->side) cudaStreamSynchronize(c->side);
   if (c->tw_x) cudaFree(c->tw_x);
   if (c->tw_y) cudaFree(c->tw_y);
   if (c->tw_h) cudaFree(c->tw_h);
@@ -244,6 +248,9 @@ static void destroy(Ctx *c) {
     for (auto e : t.ev) cudaEventDestroy(e);
   for (auto e : c->tev)
     if (e) cudaEventDestroy(e);
+  for (auto e : c->fork)
+    if (e) cudaEventDestroy(e);
+  if (c->side) cudaStreamDestroy(c->side);
   if (c->stream) cudaStreamDestroy(c->stream);
 }
 
@@ -526,9 +533,8 @@ int ih_fft_set_engine(ih_context *h, int pass, int engine) {
     return IH_OK;
   }
   if (pass == 9) {  // fixed-point transforms of the FP64 form
-    if (engine & ~kFxAll) return IH_ERR_ARG;
-    if (engine && !h->c.fx_coef) {
-      h->c.err = "fixed-point transforms apply to the FP64 form on power-of-two grids";
+    if (engine & ~h->c.fx_can) {
+      h->c.err = "a pass that has no fixed-point form on this grid";
       return IH_ERR_ARG;
     }
     h->c.fx_on = engine;

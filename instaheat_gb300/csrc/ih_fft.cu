@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(pass_threads<L, B>()) k_fft_xy_2s(C2<T> *data,
     reg_dft<T, R2>(v, tw, L / R2, sign);
 #pragma unroll
     for (int k2 = 0; k2 < R2; ++k2)
-      x1[xrow<L>(n1 * R2 + k2) * P + b] = (k2 == 0) ? v[k2] : cmul(v[k2], twid(tw, (n1 * k2) & (L - 1), sign));
+      x1[xrow<L>(n1 * R2 + k2) * P + b] = (k2 == 0) ? v[k2] : cmul(v[k2], twid(tw, n1 * k2, sign));
   }
   __syncthreads();
   if (tid < R2 * B) {
@@ -950,7 +950,7 @@ __global__ void __launch_bounds__(pass_threads<L, B>(), (d4_min_blocks<T, L, B>(
       reg_dft<T, R2>(v, tw, L / R2, +1);
 #pragma unroll
       for (int k2 = 0; k2 < R2; ++k2)
-        x1[xrow<L>(n1 * R2 + k2) * P + b1] = (k2 == 0) ? v[k2] : cmul(v[k2], twid(tw, (n1 * k2) & (L - 1), +1));
+        x1[xrow<L>(n1 * R2 + k2) * P + b1] = (k2 == 0) ? v[k2] : cmul(v[k2], twid(tw, n1 * k2, +1));
     }
     __syncthreads();
     if (tid < R2 * B) {
@@ -1195,7 +1195,7 @@ __global__ void __launch_bounds__(pass_threads<L, B>(), (rt_min_blocks<T, L, B>(
     reg_dft<T, R2>(v, tw, L / R2, -1);
 #pragma unroll
     for (int k2 = 0; k2 < R2; ++k2)
-      e0[xrow<L>(q * R2 + k2) * P + b] = (k2 == 0) ? v[k2] : cmul(v[k2], twid(tw, (q * k2) & (L - 1), -1));
+      e0[xrow<L>(q * R2 + k2) * P + b] = (k2 == 0) ? v[k2] : cmul(v[k2], twid(tw, q * k2, -1));
   }
   __syncthreads();
   C2<T> u[R1];
@@ -1226,7 +1226,7 @@ __global__ void __launch_bounds__(pass_threads<L, B>(), (rt_min_blocks<T, L, B>(
       C2<T> *e = o ? e1 : e0;
 #pragma unroll
       for (int n1 = 0; n1 < R1; ++n1)
-        e[xrow<L>(q * R1 + n1) * P + b] = (n1 == 0) ? w[n1] : cmul(w[n1], twid(tw, (n1 * q) & (L - 1), +1));
+        e[xrow<L>(q * R1 + n1) * P + b] = (n1 == 0) ? w[n1] : cmul(w[n1], twid(tw, n1 * q, +1));
     }
   }
   C2<T> acc[R2];  // ACC: the x part in out1 + (-kz^2) in / nz
@@ -1308,7 +1308,7 @@ template <typename T> constexpr size_t xt_smem(int L, int B) {
 
 template <typename T, int L, int B, bool NEXT>
 __global__ void __launch_bounds__(L / 4 * B, (xt_min_blocks<T, L, B>())) k_fft_x_tensor(
-    const C2<T> *s03, const C2<T> *s45, long long astride, T *y, T *__restrict__ out,
+    const C2<T> *s6, long long astride, T *y, T *__restrict__ out,
     const RhsScalars *rs, Geom g, const C2<T> *twg, const NextLin nl, double *outsc) {
   constexpr int Q = L / 4, LB = clog2(B);
   constexpr bool R2F = (clog2(L) & 1) != 0;
@@ -1325,7 +1325,7 @@ __global__ void __launch_bounds__(L / 4 * B, (xt_min_blocks<T, L, B>())) k_fft_x
   const long long sj = (long long)g.ny * mz;
   const long long off = (long long)yj * mz + z0;
   auto src_of = [&](int a) {
-    return (a < 4 ? s03 + a * astride : s45 + (a - 4) * astride) + off;
+    return s6 + a * astride + off;
   };
   C2<T> nxt[4];  // the next spectrum's inputs, loaded while this one is transformed
 #pragma unroll
@@ -1431,12 +1431,11 @@ __global__ void __launch_bounds__(L / 4 * B, (xt_min_blocks<T, L, B>())) k_fft_x
 template <typename T, bool MIXED, int H, bool ZSRC>
 __global__ void __launch_bounds__(32 * zwarps<T>(), (sizeof(T) == 4 && H <= 128 ? 3 : 1)) k_fft_z_rhs_fused(const C2<T> *d4, long long dstride, const T *yfl,
                                   const double *ysc, T *lap, T *pout, T *rhoout, C2<T> *s6,
-                                  long long sstride4, C2<T> *s6b, int gw, double *partials,
+                                  long long sstride, int gw, double *partials,
                                   Geom g, const C2<T> *__restrict__ twh, const C2<T> *__restrict__ twz) {
   using Gm = ZGeo<H>;
   constexpr int WPB = zwarps<T>(), R = Gm::R, W = Gm::W;
   __shared__ C2<T> stage[WPB * Gm::G * Gm::PS];
-  __shared__ double red[2][WPB];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t = lane & (W - 1), gi = lane >> Gm::LW;
   const long long rows = (long long)g.nx * g.ny;
@@ -1502,28 +1501,7 @@ __global__ void __launch_bounds__(32 * zwarps<T>(), (sizeof(T) == 4 && H <= 128 
       sp += p.x + p.y;
     }
   }
-  // block reduction of the two sums (FP64)
-  double dr = (double)srho, dp = (double)sp;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    dr += __shfl_down_sync(0xffffffffu, dr, o);
-    dp += __shfl_down_sync(0xffffffffu, dp, o);
-  }
-  if (lane == 0) {
-    red[0][warp] = dr;
-    red[1][warp] = dp;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double sa = 0.0, sb = 0.0;
-#pragma unroll
-    for (int k = 0; k < WPB; ++k) {
-      sa += red[0][k];
-      sb += red[1][k];
-    }
-    partials[2 * blockIdx.x] = sa;
-    partials[2 * blockIdx.x + 1] = sb;
-  }
+  rhs_partial<32 * WPB>((double)srho, (double)sp, partials);
   if (!gw) return;
   // the six GW source products d_i phi d_j phi, forward transforms
   C2<T> wzl[R];
@@ -1542,7 +1520,7 @@ __global__ void __launch_bounds__(32 * zwarps<T>(), (sizeof(T) == 4 && H <= 128 
     zfft_dif<-1, T, H>(u, w, twh);
     C2<T> xH;
     zr2c_post_lanes<T, H>(u, t, lane & ~(W - 1), wzl, xH);
-    C2<T> *dst = (pr < 4 ? s6 + pr * sstride4 : s6b + (pr - 4) * sstride4) + row * (H + 1);
+    C2<T> *dst = s6 + pr * sstride + row * (H + 1);
     zstore_row<T, H>(u, xH, t, srow, dst, valid);
   }
 }
@@ -1625,8 +1603,7 @@ struct XYLaunch {
   template <int B, bool GEN = false>
   int run_st(int L, dim3 grid, long long sj, long long so, const C2<T> *tw) {
     const size_t sm = sizeof(C2<T>) * ((size_t)L + (size_t)L * (B + 1));
-    cudaFuncSetAttribute(k_fft_xy_st<T, B, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sm);
+    want_smem(k_fft_xy_st<T, B, GEN>, sm);
     k_fft_xy_st<T, B, GEN><<<grid, threads_st(L, B), sm, c->stream>>>(data, stride, L, sj, so,
                                                                        mzv(), sign, tw);
     return IH_OK;
@@ -1634,7 +1611,7 @@ struct XYLaunch {
   template <int L, int B>
   int run_2s(dim3 grid, long long sj, long long so, const C2<T> *tw) {
     const size_t sm = sizeof(C2<T>) * ((size_t)L + (size_t)L * B);
-    cudaFuncSetAttribute(k_fft_xy_2s<T, L, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    want_smem(k_fft_xy_2s<T, L, B>, sm);
     k_fft_xy_2s<T, L, B><<<grid, pass_threads<L, B>(), sm, c->stream>>>(data, stride, sj, so,
                                                                          mzv(), sign, tw);
     return IH_OK;
@@ -1642,8 +1619,7 @@ struct XYLaunch {
   template <int L, int B>
   int run_2s_occ(dim3 grid, long long sj, long long so, const C2<T> *tw) {
     const size_t sm = sizeof(C2<T>) * ((size_t)L + (size_t)L * B);
-    cudaFuncSetAttribute(k_fft_xy_2s_occ<T, L, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sm);
+    want_smem(k_fft_xy_2s_occ<T, L, B>, sm);
     k_fft_xy_2s_occ<T, L, B><<<grid, pass_threads<L, B>(), sm, c->stream>>>(data, stride, sj, so,
                                                                              mzv(), sign, tw);
     return IH_OK;
@@ -1655,8 +1631,7 @@ struct XYLaunch {
     const int nt = pass_threads<L, B>();
     static int occ = 0;  // resident CTAs per SM (a property of the kernel)
     if (!occ) {
-      cudaFuncSetAttribute(k_fft_xy_pipe<T, L, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sm);
+      want_smem(k_fft_xy_pipe<T, L, B>, sm);
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fft_xy_pipe<T, L, B>, nt, sm) !=
               cudaSuccess ||
           occ < 1)
@@ -1672,7 +1647,7 @@ struct XYLaunch {
   template <int L, int B>
   int run_3s(dim3 grid, long long sj, long long so, const C2<T> *tw) {
     const size_t sm = sizeof(C2<T>) * ((size_t)L + (size_t)L * B);
-    cudaFuncSetAttribute(k_fft_xy_3s<T, L, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    want_smem(k_fft_xy_3s<T, L, B>, sm);
     k_fft_xy_3s<T, L, B><<<grid, threads3<L, B>(), sm, c->stream>>>(data, stride, sj, so, mzv(),
                                                                      sign, tw);
     return IH_OK;
@@ -1718,7 +1693,9 @@ int fft_xy(Ctx *c, C2<T> *data, long long stride, int count, int axis, int sign)
   const Geom &g = c->g;
   const int L = axis == 0 ? g.nx : g.ny;
   prof_begin(c, KK_FFT_XY);
-  if (L & (L - 1)) {  // 2^a 3^b: the Stockham engine with a radix-3 stage
+  if (sizeof(T) == 8 && (c->fx_on >> axis & 1)) {
+    IH_TRY(fix_xy(c, data, stride, count, axis, sign, 0));
+  } else if (L & (L - 1)) {  // 2^a 3^b: the Stockham engine with a radix-3 stage
     constexpr int B = tileB<T>();
     const long long sj = axis == 0 ? (long long)g.ny * g.mz : g.mz;
     const long long so = axis == 0 ? g.mz : (long long)g.ny * g.mz;
@@ -1726,8 +1703,6 @@ int fft_xy(Ctx *c, C2<T> *data, long long stride, int count, int axis, int sign)
     XYLaunch<T> xl{c, data, stride, count, axis, sign, FV_STOCKHAM};
     IH_TRY((xl.template run_st<B, true>(L, dim3((g.mz + B - 1) / B, outer, count), sj, so,
                                         tab<T>(axis == 0 ? c->tw_x : c->tw_y))));
-  } else if (sizeof(T) == 8 && (c->fx_on >> axis & 1)) {
-    IH_TRY(fix_xy(c, data, stride, count, axis, sign, 0));
   } else {
     IH_TRY(dispatch_len(L, XYLaunch<T>{c, data, stride, count, axis, sign, c->xy_var[axis]},
                         allow512<T>()));
@@ -1736,8 +1711,8 @@ int fft_xy(Ctx *c, C2<T> *data, long long stride, int count, int axis, int sign)
   return check_launch(c, "k_fft_xy");
 }
 
-// The forward y then x passes of the six S_ij spectra (arrays 0..3 and 5, 6
-// of spec), kz slab by kz slab when w > 0: a slab of the six arrays (6 nx ny w
+// The forward y then x passes of the six S_ij spectra (arrays 0..5 of spec),
+// kz slab by kz slab when w > 0: a slab of the six arrays (6 nx ny w
 // complex values, 50 MB at 256^2 x 16 in FP32) stays in L2 between its y and
 // its x pass, so the x pass reads it from L2 and the y pass's writes are
 // overwritten there before they reach HBM.  w = 0: whole arrays (y passes,
@@ -1747,30 +1722,25 @@ int fft_gw_yx(Ctx *c, C2<T> *spec, int w) {
   const Geom &g = c->g;
   const long long M = g.M;
   if (w <= 0 || !g.pow2 || w >= g.mz) {
-    IH_TRY((fft_xy<T>(c, spec, M, 4, 1, -1)));
-    IH_TRY((fft_xy<T>(c, spec + 5 * M, M, 2, 1, -1)));
-    IH_TRY((fft_xy<T>(c, spec, M, 4, 0, -1)));
-    return fft_xy<T>(c, spec + 5 * M, M, 2, 0, -1);
+    IH_TRY((fft_xy<T>(c, spec, M, 6, 1, -1)));
+    return fft_xy<T>(c, spec, M, 6, 0, -1);
   }
   const int ns = g.mz / w;
   for (int q = 0; q < ns; ++q) {
     const int z0 = q * w, ws = (q + 1 < ns) ? w : g.mz - z0;
     for (int axis = 1; axis >= 0; --axis) {
-      for (int grp = 0; grp < 2; ++grp) {
-        const int count = grp ? 2 : 4;
-        C2<T> *d = spec + (grp ? 5 * M : 0) + z0;
-        const int L = axis == 0 ? g.nx : g.ny;
-        prof_begin(c, KK_FFT_XY);
-        XYLaunch<T> xl{c, d, M, count, axis, -1, c->xy_var[axis]};
-        xl.cols = ws;
-        if (sizeof(T) == 8 && (c->fx_on >> axis & 1)) {
-          IH_TRY(fix_xy(c, d, M, count, axis, -1, ws));
-        } else {
-          IH_TRY(dispatch_len(L, xl, allow512<T>()));
-        }
-        prof_end(c, KK_FFT_XY, 2.0 * count * (double)g.nx * g.ny * ws * sizeof(C2<T>));
-        IH_TRY(check_launch(c, "k_fft_xy"));
+      C2<T> *d = spec + z0;
+      const int L = axis == 0 ? g.nx : g.ny;
+      prof_begin(c, KK_FFT_XY);
+      XYLaunch<T> xl{c, d, M, 6, axis, -1, c->xy_var[axis]};
+      xl.cols = ws;
+      if (sizeof(T) == 8 && (c->fx_on >> axis & 1)) {
+        IH_TRY(fix_xy(c, d, M, 6, axis, -1, ws));
+      } else {
+        IH_TRY(dispatch_len(L, xl, allow512<T>()));
       }
+      prof_end(c, KK_FFT_XY, 2.0 * 6 * (double)g.nx * g.ny * ws * sizeof(C2<T>));
+      IH_TRY(check_launch(c, "k_fft_xy"));
     }
   }
   return IH_OK;
@@ -1816,12 +1786,14 @@ int fft_zr2c(Ctx *c, const T *in, long long in_stride, C2<T> *out, long long out
   prof_begin(c, KK_FFT_ZR2C);
   if (sizeof(T) == 8 && (c->fx_on >> 6 & 1)) {
     IH_TRY(fix_z(c, in, in_stride, out, out_stride, count, true));
+  } else if (zrow_ok(c)) {
+    IH_TRY(zrow_pass(c, in, in_stride, out, out_stride, count, true));
   } else if (fused_wide_ok(c)) {
     IH_TRY(zr2c_wide_launch(c, in, in_stride, out, out_stride, count));
   } else if (g.h & (g.h - 1)) {
     const long long rows = (long long)g.nx * g.ny;
     const size_t sm = zg_smem<T>(g.h);
-    cudaFuncSetAttribute(k_fft_zr2c_g<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    want_smem(k_fft_zr2c_g<T>, sm);
     k_fft_zr2c_g<T><<<dim3((unsigned)((rows + kZB - 1) / kZB), count), threads_st(g.h, kZB), sm,
                       c->stream>>>(in, in_stride, out, out_stride, rows, g.h, tab<T>(c->tw_h),
                                    tab<T>(c->tw_z));
@@ -1839,10 +1811,12 @@ int fft_zc2r(Ctx *c, const C2<T> *in, long long in_stride, T *out, long long out
   prof_begin(c, KK_FFT_ZC2R);
   if (sizeof(T) == 8 && (c->fx_on >> 6 & 1)) {
     IH_TRY(fix_z(c, in, in_stride, out, out_stride, count, false));
+  } else if (zrow_ok(c)) {
+    IH_TRY(zrow_pass(c, in, in_stride, out, out_stride, count, false));
   } else if (g.h & (g.h - 1)) {
     const long long rows = (long long)g.nx * g.ny;
     const size_t sm = zg_smem<T>(g.h);
-    cudaFuncSetAttribute(k_fft_zc2r_g<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    want_smem(k_fft_zc2r_g<T>, sm);
     k_fft_zc2r_g<T><<<dim3((unsigned)((rows + kZB - 1) / kZB), count), threads_st(g.h, kZB), sm,
                       c->stream>>>(in, in_stride, out, out_stride, rows, g.h, tab<T>(c->tw_h),
                                    tab<T>(c->tw_z));
@@ -1882,8 +1856,7 @@ struct D4Launch {
     const Geom &g = c->g;
     dim3 grid((g.mz + B - 1) / B, g.ny, 1);
     const size_t sm = sizeof(C2<T>) * ((size_t)L + (size_t)L * B);
-    cudaFuncSetAttribute(k_fft_x_deriv4_2s<T, L, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sm);
+    want_smem(k_fft_x_deriv4_2s<T, L, B>, sm);
     k_fft_x_deriv4_2s<T, L, B><<<grid, pass_threads<L, B>(), sm, c->stream>>>(
         phihat, out, out_stride, g, tab<T>(c->tw_x));
     return IH_OK;
@@ -1895,8 +1868,7 @@ struct D4Launch {
     const int nt = pass_threads<L, B>();
     static int occ = 0;
     if (!occ) {
-      cudaFuncSetAttribute(k_fft_x_deriv4_pipe<T, L, B>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      want_smem(k_fft_x_deriv4_pipe<T, L, B>, sm);
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fft_x_deriv4_pipe<T, L, B>, nt,
                                                         sm) != cudaSuccess ||
           occ < 1)
@@ -1917,8 +1889,7 @@ struct D4Launch {
     const Geom &g = c->g;
     dim3 grid((g.mz + B - 1) / B, g.ny, 1);
     const size_t sm = sizeof(C2<T>) * ((size_t)L + 2 * (size_t)L * (B + 1));
-    cudaFuncSetAttribute(k_fft_x_deriv4_st<T, B, GEN>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    want_smem(k_fft_x_deriv4_st<T, B, GEN>, sm);
     k_fft_x_deriv4_st<T, B, GEN><<<grid, threads_st(L, B), sm, c->stream>>>(
         phihat, out, out_stride, g, tab<T>(c->tw_x));
     return IH_OK;
@@ -1961,13 +1932,11 @@ struct RTLaunch {
     const size_t sm = sizeof(C2<T>) * ((size_t)L + 2 * (size_t)L * B);
     const double invnz = 1.0 / (double)c->g.nz;
     if (axis == 1) {
-      cudaFuncSetAttribute(k_fft_xy_rt<T, L, B, true>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      want_smem(k_fft_xy_rt<T, L, B, true>, sm);
       k_fft_xy_rt<T, L, B, true><<<grid, pass_threads<L, B>(), sm, c->stream>>>(
           z, d1, d2, sj, so, c->g.mz, ku, k2u, scale, c->g.kz2, invnz, tw);
     } else {
-      cudaFuncSetAttribute(k_fft_xy_rt<T, L, B, false>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      want_smem(k_fft_xy_rt<T, L, B, false>, sm);
       k_fft_xy_rt<T, L, B, false><<<grid, pass_threads<L, B>(), sm, c->stream>>>(
           z, d1, d2, sj, so, c->g.mz, ku, k2u, scale, c->g.kz2, invnz, tw);
     }
@@ -1998,7 +1967,7 @@ struct RTLaunch {
 template <typename T>
 struct XTLaunch {
   Ctx *c;
-  const C2<T> *s03, *s45;
+  const C2<T> *s6;
   T *y;
   T *out;
   double *outsc;
@@ -2008,12 +1977,11 @@ struct XTLaunch {
     constexpr int B = tensor_tile<T>();
     const Geom &g = c->g;
     const size_t sm = xt_smem<T>(L, B);
-    cudaFuncSetAttribute(k_fft_x_tensor<T, L, B, NEXT>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    want_smem(k_fft_x_tensor<T, L, B, NEXT>, sm);
     NextLin nl = next ? *next : NextLin{};
     if (!next) nl.skip_pos = c->skip_pos;
     k_fft_x_tensor<T, L, B, NEXT><<<dim3((g.mz + B - 1) / B, g.ny, 1), L / 4 * B, sm,
-                                     c->stream>>>(s03, s45, g.M, y, out, c->rs, g,
+                                     c->stream>>>(s6, g.M, y, out, c->rs, g,
                                                   tab<T>(c->tw_x), nl, outsc);
   }
   template <int L>
@@ -2031,11 +1999,11 @@ struct XTLaunch {
 };
 
 template <typename T>
-int fft_x_tensor(Ctx *c, const C2<T> *s03, const C2<T> *s45, T *y, T *out, double *outsc,
+int fft_x_tensor(Ctx *c, const C2<T> *s6, T *y, T *out, double *outsc,
                  const NextLin *next) {
   const Geom &g = c->g;
   prof_begin(c, KK_X_TENSOR);
-  IH_TRY(dispatch_len(g.nx, XTLaunch<T>{c, s03, s45, y, out, outsc, next}, allow512<T>()));
+  IH_TRY(dispatch_len(g.nx, XTLaunch<T>{c, s6, y, out, outsc, next}, allow512<T>()));
   prof_end(c, KK_X_TENSOR,
            6.0 * g.M * sizeof(C2<T>) +
                ((c->skip_pos ? 6.0 : 8.0) + (next ? 4.0 * (next->n + 2) : 0.0)) * g.Next * sizeof(T));
@@ -2066,17 +2034,16 @@ struct FusedLaunch {
   C2<T> *s6;
   int gw;
   double *partials;
-  int *nblk_out;
   int zsrc;
   template <int H, bool ZSRC>
-  void launch(unsigned nblk, int nt, long long M, C2<T> *s6b) {
+  void launch(unsigned nblk, int nt, long long M) {
     if constexpr (sizeof(T) == 4) {
       k_fft_z_rhs_fused<T, true, H, ZSRC><<<nblk, nt, 0, c->stream>>>(
-          d4, M, yfl, ysc, lap, p, rho, s6, M, s6b, gw, partials, c->g, tab<T>(c->tw_h),
+          d4, M, yfl, ysc, lap, p, rho, s6, M, gw, partials, c->g, tab<T>(c->tw_h),
           tab<T>(c->tw_z));
     } else {
       k_fft_z_rhs_fused<T, false, H, ZSRC><<<nblk, nt, 0, c->stream>>>(
-          d4, M, yfl, ysc, lap, p, rho, s6, M, s6b, gw, partials, c->g, tab<T>(c->tw_h),
+          d4, M, yfl, ysc, lap, p, rho, s6, M, gw, partials, c->g, tab<T>(c->tw_h),
           tab<T>(c->tw_z));
     }
   }
@@ -2095,13 +2062,12 @@ struct FusedLaunch {
       }
       const int nt = 32 * zwarps<T>();
       const long long M = g.M;
-      C2<T> *s6b = s6 + 5 * M;  // products 4 and 5 go to spec[5], spec[6]
+      c->z_blocks = (int)nblk;
       if (zsrc) {
-        launch<H, true>(nblk, nt, M, s6b);
+        launch<H, true>(nblk, nt, M);
       } else {
-        launch<H, false>(nblk, nt, M, s6b);
+        launch<H, false>(nblk, nt, M);
       }
-      *nblk_out = (int)nblk;
       return IH_OK;
     }
   }
@@ -2109,22 +2075,23 @@ struct FusedLaunch {
 
 template <typename T>
 int fft_z_rhs_fused(Ctx *c, const C2<T> *d4, const T *yfl, const double *ysc, T *lap, T *p,
-                    T *rho, C2<T> *s6, int gw, double *partials, int *nblocks_out, int zsrc,
+                    T *rho, C2<T> *s6, int gw, double *partials, int zsrc,
                     int plane) {
   const Geom &g = c->g;
   prof_begin(c, KK_Z_RHS_FUSED);
   if (sizeof(T) == 8 && (c->fx_on >> 6 & 1)) {
-    IH_TRY(fix_z_rhs(c, d4, yfl, ysc, lap, p, rho, s6, gw, partials, nblocks_out, zsrc));
+    IH_TRY(fix_z_rhs(c, d4, yfl, ysc, lap, p, rho, s6, gw, partials, zsrc));
+  } else if (zrow_ok(c)) {
+    IH_TRY(zrow_rhs(c, d4, yfl, ysc, lap, p, rho, s6, gw, partials, zsrc));
   } else if (fused_wide_ok(c)) {  // nz = 256: the wide-row engine
-    IH_TRY(fused_wide_launch(c, d4, yfl, ysc, lap, p, rho, s6, gw, partials, nblocks_out, zsrc,
-                             plane));
+    IH_TRY(fused_wide_launch(c, d4, yfl, ysc, lap, p, rho, s6, gw, partials, zsrc, plane));
   } else {
     if (plane) {
       c->err = "plane-major tensor sources need the wide-row z pass";
       return IH_ERR_STATE;
     }
     IH_TRY(dispatch_len(
-        g.h, FusedLaunch<T>{c, d4, yfl, ysc, lap, p, rho, s6, gw, partials, nblocks_out, zsrc},
+        g.h, FusedLaunch<T>{c, d4, yfl, ysc, lap, p, rho, s6, gw, partials, zsrc},
         false));
   }
   prof_end(c, KK_Z_RHS_FUSED,
@@ -2165,7 +2132,7 @@ int fft_tables(Ctx *c) {
 }
 
 // ---------------------------------------------------------------------------
-// autotuner: every engine variant of the x/y passes (per axis, on four
+// autotuner: every engine variant of the x/y passes (per axis, on six
 // arrays, the largest batch the RHS issues) and of the fused x pass, timed
 // with CUDA events on the context stream over zeroed scratch spectra; the
 // fastest is kept.  Transform timing does not depend on the data.
@@ -2184,7 +2151,7 @@ static int autotune_t(Ctx *c) {
     c->tensor_fused = 0;
     c->tune_report =
         "grid with a radix-3 factor: Stockham x/y passes, shared-memory z passes, the "
-        "full-spectrum RHS route";
+        "full-spectrum RHS route; FP64: fixed-point passes for the axes that have them";
     return IH_OK;
   }
   C2<T> *sp = reinterpret_cast<C2<T> *>(c->spec[0]);
@@ -2227,7 +2194,7 @@ static int autotune_t(Ctx *c) {
       for (int r = 0; r <= reps && st == IH_OK; ++r) {  // r = 0: warm-up
         if (r == 1) cudaEventRecord(e0, c->stream);
         if (pass < 2)
-          st = fft_xy<T>(c, sp, M, 4, pass, -1);
+          st = fft_xy<T>(c, sp, M, 6, pass, -1);
         else if (pass == 2)
           st = fft_x_deriv4_inv<T>(c, sp + 4 * M, sp, M);
         else
@@ -2355,8 +2322,7 @@ static int autotune_t(Ctx *c) {
           if (st == IH_OK)
             st = tensor_last_pass(c, sp, c->y.fl, c->ytmp.fl, c->ytmp.sc, nullptr, true);
         } else {
-          st = fft_xy<T>(c, sp, M, 4, 1, -1);
-          if (st == IH_OK) st = fft_xy<T>(c, sp + 5 * M, M, 2, 1, -1);
+          st = fft_xy<T>(c, sp, M, 6, 1, -1);
           if (st == IH_OK) st = tensor_last_pass(c, sp, c->y.fl, c->ytmp.fl, c->ytmp.sc, nullptr);
         }
       }
@@ -2389,11 +2355,10 @@ static int autotune_t(Ctx *c) {
     T *lap = (T *)c->rbuf[0], *pz = (T *)c->rbuf[1];
     for (int v = 1; v <= 2 && st == IH_OK; ++v) {
       c->zwide = v;
-      int nblk = 0;
       for (int r = 0; r <= reps && st == IH_OK; ++r) {
         if (r == 1) cudaEventRecord(e0, c->stream);
         st = fft_z_rhs_fused<T>(c, sp, (const T *)c->y.fl, c->y.sc, lap, pz, nullptr, sp,
-                                c->p.enable_gw, c->partials, &nblk, 1, 0);
+                                c->p.enable_gw, c->partials, 1, 0);
       }
       if (st != IH_OK) break;
       cudaEventRecord(e1, c->stream);
@@ -2439,10 +2404,9 @@ int fft_autotune(Ctx *c) {
   template int fft_gw_yx<T>(Ctx *, C2<T> *, int);                                              \
   template int fft_x_deriv4_inv<T>(Ctx *, const C2<T> *, C2<T> *, long long);                   \
   template int fft_z_rhs_fused<T>(Ctx *, const C2<T> *, const T *, const double *, T *, T *,    \
-                                  T *, C2<T> *, int, double *, int *, int, int);                \
+                                  T *, C2<T> *, int, double *, int, int);     \
   template int fft_xy_roundtrip<T>(Ctx *, const C2<T> *, C2<T> *, C2<T> *, int);              \
-  template int fft_x_tensor<T>(Ctx *, const C2<T> *, const C2<T> *, T *, T *, double *,       \
-                               const NextLin *);
+  template int fft_x_tensor<T>(Ctx *, const C2<T> *, T *, T *, double *, const NextLin *);
 IH_INST(float)
 IH_INST(double)
 #undef IH_INST

@@ -1,6 +1,6 @@
 // ih_fix.cu -- the transforms of the plain FP64 form in 64-bit block fixed
 // point (ih_fix.cuh): passes along x and y, the derivative round trips, the
-// real z passes and the fused z pass of the RHS, for power-of-two axes.  Data
+// real z passes and the fused z pass of the RHS.  Data
 // in memory stay FP64 in the layouts of the other engines (ih_fft.cu); each
 // pass converts a pencil on its way in and out of registers.
 #include <math.h>
@@ -8,6 +8,7 @@
 #include "ih_internal.cuh"
 #include "ih_fftcore.cuh"
 #include "ih_fix.cuh"
+#include "ih_zrow.cuh"
 
 namespace ih {
 
@@ -28,8 +29,19 @@ template <> struct FxFac<64> { static constexpr int R1 = 8, R2 = 8; };
 template <> struct FxFac<128> { static constexpr int R1 = 16, R2 = 8; };
 template <> struct FxFac<256> { static constexpr int R1 = 16, R2 = 16; };
 template <> struct FxFac<512> { static constexpr int R1 = 16, R2 = 32; };
-template <int L> __host__ __device__ constexpr int fx_p() {
-  return 64 - clog2(L) < 59 ? 64 - clog2(L) : 59;
+template <> struct FxFac<12> { static constexpr int R1 = 4, R2 = 3; };
+template <> struct FxFac<18> { static constexpr int R1 = 6, R2 = 3; };
+template <> struct FxFac<24> { static constexpr int R1 = 6, R2 = 4; };
+template <> struct FxFac<36> { static constexpr int R1 = 6, R2 = 6; };
+template <> struct FxFac<48> { static constexpr int R1 = 8, R2 = 6; };
+template <> struct FxFac<72> { static constexpr int R1 = 12, R2 = 6; };
+template <> struct FxFac<96> { static constexpr int R1 = 12, R2 = 8; };
+template <> struct FxFac<144> { static constexpr int R1 = 12, R2 = 12; };
+template <> struct FxFac<192> { static constexpr int R1 = 16, R2 = 12; };
+template <> struct FxFac<288> { static constexpr int R1 = 12, R2 = 24; };
+template <> struct FxFac<384> { static constexpr int R1 = 16, R2 = 24; };
+template <int L> __host__ __device__ constexpr int fx_p() {  // log2 rounded up
+  return 64 - clog2(2 * L - 1) < 59 ? 64 - clog2(2 * L - 1) : 59;
 }
 template <int L> __host__ __device__ constexpr int fx_maxr() {
   return FxFac<L>::R1 > FxFac<L>::R2 ? FxFac<L>::R1 : FxFac<L>::R2;
@@ -63,7 +75,7 @@ __device__ __forceinline__ unsigned fx_col_max(unsigned m, unsigned *red, int ti
 }
 
 template <int L, int B, int S>
-__global__ void __launch_bounds__(fx_threads<L, B>(), L <= 256 ? 512 / fx_threads<L, B>() : 1)
+__global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 512 / fx_threads<L, B>() : 1)
     k_fx_xy(double2 *data, long long astride, long long sj, long long so, int mz, FxTab tw) {
   constexpr int R1 = FxFac<L>::R1, R2 = FxFac<L>::R2, NT = fx_threads<L, B>();
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -115,7 +127,7 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), L <= 256 ? 512 / fx_thread
 // transform's p (the coefficients take 2), so no precision is lost whatever
 // its size.
 template <int L, int B, bool ACC>
-__global__ void __launch_bounds__(fx_threads<L, B>(), L <= 256 ? 384 / fx_threads<L, B>() : 1) k_fx_rt(
+__global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 384 / fx_threads<L, B>() : 1) k_fx_rt(
     const double2 *__restrict__ in, double2 *__restrict__ out0, double2 *out1, long long sj,
     long long so, int mz, FxTab tw, const long long *__restrict__ c1,
     const long long *__restrict__ c2, const long long *__restrict__ cz, int e1, int e2) {
@@ -235,158 +247,39 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), L <= 256 ? 384 / fx_thread
 }
 
 // ---------------------------------------------------------------------------
-// z passes.  A row of H = nz/2 complex values (z_j = x_2j + i x_2j+1) on B
-// lanes with A values each, H = A B, as the wide-row engine of ih_zwide.cu
-// has it for H = 128: lane t holds Z[t + B m] (m < A) on the spectral side and
-// z[E t + e + A q] (e < E = A / B, q < B; register E q + e) on the real side,
-// one transpose through the warp's shared scratch in between.  Scratch
-// columns are swizzled and rows padded so that the eight 16-byte accesses of
-// a phase hit different banks.  At 256^3: r2c 144 us an array against 606 us,
-// c2r of four arrays 449 against 2564 us (FP64 pipe, wide rows and a warp per
-// row); both conversions on the integer pipe (on the FP64 pipe 195 and 625 us).
-template <int H> struct FxZ;
-template <> struct FxZ<4> { static constexpr int A = 2, B = 2; };
-template <> struct FxZ<8> { static constexpr int A = 4, B = 2; };
-template <> struct FxZ<16> { static constexpr int A = 4, B = 4; };
-template <> struct FxZ<32> { static constexpr int A = 8, B = 4; };
-template <> struct FxZ<64> { static constexpr int A = 8, B = 8; };
-template <> struct FxZ<128> { static constexpr int A = 16, B = 8; };
-template <> struct FxZ<256> { static constexpr int A = 16, B = 16; };
-template <int H> struct FxZG {
-  static constexpr int A = FxZ<H>::A, B = FxZ<H>::B, E = A / B, G = 32 / B;
-  static constexpr int X = A * B + (B < 8 ? B : 0);  // scratch of a row
+// z passes, on the engine of ih_zrow.cuh.  At 256^3: r2c 144 us an array
+// against 606 us, c2r of four arrays 449 against 2564 us (FP64 pipe, wide rows
+// and a warp per row); both conversions on the integer pipe (on the FP64 pipe
+// 195 and 625 us).
+struct NumFx {
+  using C = fx2;
+  using Tab = FxTab;
+  __device__ static __forceinline__ C mk(long long x, long long y) { return fx_mk(x, y); }
+  __device__ static __forceinline__ C add(C a, C b) { return a + b; }
+  __device__ static __forceinline__ C sub(C a, C b) { return a - b; }
+  __device__ static __forceinline__ C quarter(C v) { return fx_quarter(v); }
+  __device__ static __forceinline__ C half(C v) { return fx_mk((v.x + 1) >> 1, (v.y + 1) >> 1); }
+  __device__ static __forceinline__ C half_quarter(C v) {
+    return fx_mk((v.x + 4) >> 3, (v.y + 4) >> 3);
+  }
+  template <int S>
+  __device__ static __forceinline__ C cmul(C v, Tab t, int i) {
+    return fx_cmul<S>(v, fx_tw(t, i));
+  }
+  template <int R, int S>
+  __device__ static __forceinline__ void dft(C (&v)[R]) { fx_dft<R, S>(v); }
+  __device__ static __forceinline__ C shfl(C v, int src) {
+    return fx_mk(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+  }
+};
+template <int H> struct FxZG : ZRow<NumFx, H> {
   // c2r: the split's 1/4 and the transform's growth H sqrt 2; r2c: the split
   // adds two values and the last bit of growth
-  static constexpr int pc = 64 - clog2(H) < 58 ? 64 - clog2(H) : 58;
-  static constexpr int pr = 63 - clog2(H) < 58 ? 63 - clog2(H) : 58;
+  static constexpr int lg = clog2(2 * H - 1);  // log2 H, rounded up
+  static constexpr int pc = 64 - lg < 58 ? 64 - lg : 58;
+  static constexpr int pr = 63 - lg < 58 ? 63 - lg : 58;
 };
 constexpr int kFxWarps = 4;
-
-template <int H>
-__device__ __forceinline__ unsigned fx_row_max(unsigned m) {
-#pragma unroll
-  for (int o = 1; o < FxZG<H>::B; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  return m;
-}
-__device__ __forceinline__ fx2 fx_shfl(fx2 v, int src) {
-  return fx_mk(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
-}
-
-// spectral side -> real side, unnormalised inverse, scale 1/4
-template <int H>
-__device__ __forceinline__ void fx_z_inverse(fx2 (&v)[FxZG<H>::A], int t, fx2 *xch, FxTab twh) {
-  using G = FxZG<H>;
-  constexpr int A = G::A, B = G::B, E = G::E;
-  fx_dft<A, +1>(v);
-#pragma unroll
-  for (int p = 0; p < A; ++p) {
-    const fx2 w = p == 0 ? fx_quarter(v[p]) : fx_cmul<+1>(v[p], fx_tw(twh, p * t));
-    xch[p * B + (t ^ ((p / E) & (B - 1)))] = w;
-  }
-  __syncwarp();
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    fx2 u[B];
-#pragma unroll
-    for (int s = 0; s < B; ++s) u[s] = xch[(E * t + e) * B + (s ^ t)];
-    fx_dft<B, +1>(u);
-#pragma unroll
-    for (int q = 0; q < B; ++q) v[E * q + e] = u[q];
-  }
-  __syncwarp();
-}
-// real side -> spectral side, forward, scale 1/4
-template <int H>
-__device__ __forceinline__ void fx_z_forward(fx2 (&v)[FxZG<H>::A], int t, fx2 *xch, FxTab twh) {
-  using G = FxZG<H>;
-  constexpr int A = G::A, B = G::B, E = G::E;
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    fx2 u[B];
-#pragma unroll
-    for (int q = 0; q < B; ++q) u[q] = v[E * q + e];
-    fx_dft<B, -1>(u);
-#pragma unroll
-    for (int s = 0; s < B; ++s)
-      xch[(E * t + e) * B + (s ^ t)] =
-          s == 0 ? fx_quarter(u[s]) : fx_cmul<-1>(u[s], fx_tw(twh, (E * t + e) * s));
-  }
-  __syncwarp();
-#pragma unroll
-  for (int p = 0; p < A; ++p) v[p] = xch[p * B + (t ^ ((p / E) & (B - 1)))];
-  __syncwarp();
-  fx_dft<A, -1>(v);
-}
-
-// c2r split, in place: x[m] = X_k (k = t + B m), xH = X_H on t == 0 ->
-// (E + i O) / 4 with E = X_k + conj X_(H-k), O = (X_k - conj X_(H-k)) exp(2 pi i
-// k / nz).  X_(H-k) is register A - 1 - m of lane B - t, or the lane's own for
-// t == 0.
-template <int H>
-__device__ __forceinline__ void fx_z_c2r_prep(fx2 (&x)[FxZG<H>::A], fx2 xH, int t, int gbase,
-                                              FxTab twz) {
-  using G = FxZG<H>;
-  constexpr int A = G::A, B = G::B;
-  const int src = gbase + ((B - t) & (B - 1));
-  auto split = [&](fx2 a, fx2 pc, int k) {
-    pc.y = -pc.y;
-    const fx2 e = a + pc, o = fx_cmul<+1>(a - pc, fx_tw(twz, k));
-    return fx_mk(((e.x + 2) >> 2) - o.y, ((e.y + 2) >> 2) + o.x);
-  };
-  // registers m and A - 1 - m exchange with each other's (m and A - m on
-  // lane 0), so both are formed before either is overwritten; register A - 1
-  // of the next pair feeds lane 0 one step later
-  fx2 prev = xH;  // lane 0: X_(H - B m) for m = 0 is X_H
-#pragma unroll
-  for (int m = 0; m < (A + 1) / 2; ++m) {
-    const int n = A - 1 - m;
-    fx2 pm = fx_shfl(x[n], src), pn = fx_shfl(x[m], src);
-    fx2 keep = x[n];
-    if (t == 0) {
-      pm = prev;                           // X at A - m (X_H for m = 0)
-      pn = m + 1 <= n ? x[m + 1] : pn;     // X at A - n = m + 1
-      if (m + 1 == n) pn = x[m + 1];
-    }
-    const fx2 a = split(x[m], pm, t + B * m);
-    if (n != m) x[n] = split(x[n], pn, t + B * n);
-    x[m] = a;
-    prev = keep;
-  }
-}
-
-// r2c split: v[m] = Z_k (k = t + B m) -> X_k / 4, xH = X_H / 4 on t == 0:
-// X_k = E_k + exp(-2 pi i k / nz) O_k, E_k = (Z_k + conj Z_(H-k)) / 2, O_k =
-// (Z_k - conj Z_(H-k)) / (2 i)
-template <int H>
-__device__ __forceinline__ void fx_z_r2c_post(fx2 (&v)[FxZG<H>::A], int t, int gbase, FxTab twz,
-                                              fx2 &xH) {
-  using G = FxZG<H>;
-  constexpr int A = G::A, B = G::B;
-  const int src = gbase | ((B - t) & (B - 1));
-  auto split = [&](fx2 z, fx2 pz, int k, fx2 *last) {
-    const fx2 e2 = fx_mk(z.x + pz.x, z.y - pz.y);          // 2 E
-    const fx2 o2 = fx_mk(z.y + pz.y, pz.x - z.x);          // 2 O
-    const fx2 o = fx_mk((o2.x + 1) >> 1, (o2.y + 1) >> 1);
-    const fx2 e = fx_mk((e2.x + 4) >> 3, (e2.y + 4) >> 3);
-    if (last) *last = fx_mk(e.x - ((o.x + 2) >> 2), e.y - ((o.y + 2) >> 2));  // exp(-i pi) = -1
-    return e + fx_cmul<-1>(o, fx_tw(twz, k));
-  };
-  fx2 prev = v[0];  // lane 0: Z_(H - 0) = Z_0
-#pragma unroll
-  for (int m = 0; m < (A + 1) / 2; ++m) {
-    const int n = A - 1 - m;
-    fx2 pm = fx_shfl(v[n], src), pn = fx_shfl(v[m], src);
-    const fx2 keep = v[n];
-    if (t == 0) {
-      pm = prev;
-      pn = v[m + 1 <= n ? m + 1 : m];
-    }
-    const fx2 a = split(v[m], pm, t + B * m, m == 0 ? &xH : nullptr);
-    if (n != m) v[n] = split(v[n], pn, t + B * n, nullptr);
-    v[m] = a;
-    prev = keep;
-  }
-}
 
 // Real rows -> half spectra.  The row's first value is taken off before the
 // conversion and nz times it added to X_0: a field that is a large constant
@@ -419,12 +312,12 @@ __global__ void __launch_bounds__(32 * kFxWarps) k_fx_zr2c(
     x[i].x -= x0;
     x[i].y -= x0;
   }
-  const FxScale sc = fx_scale(fx_row_max<H>(fx_max_in(x)), G::pr);
+  const FxScale sc = fx_scale(zrow_max<FxZG<H>::B>(fx_max_in(x)), G::pr);
   fx2 v[A];
   fx_load<true>(x, sc, v);
-  fx_z_forward<H>(v, t, &xs[warp][grp * G::X], twh);
+  zrow_forward<NumFx, H>(v, t, &xs[warp][grp * G::X], twh);
   fx2 xH;
-  fx_z_r2c_post<H>(v, t, gbase, twz, xH);
+  zrow_r2c_post<NumFx, H>(v, t, gbase, twz, xH);
   if (valid) {
     double2 *dst = out + blockIdx.y * ostride + row * (H + 1);
 #pragma unroll
@@ -452,7 +345,7 @@ __device__ __forceinline__ FxScale fx_z_load(double2 (&x)[FxZG<H>::A], double2 x
   double2 h[1] = {xH};
   fx2 u[1];
   const FxScale sc =
-      fx_scale(fx_row_max<H>(max(fx_max_in(x), fx_max_in(h))), FxZG<H>::pc);
+      fx_scale(zrow_max<FxZG<H>::B>(max(fx_max_in(x), fx_max_in(h))), FxZG<H>::pc);
   fx_load<BITS>(x, sc, v);
   fx_load<BITS>(h, sc, u);
   vH = u[0];
@@ -480,8 +373,8 @@ __global__ void __launch_bounds__(32 * kFxWarps) k_fx_zc2r(
   if (t == 0) x[0].x -= x0;
   fx2 v[A], vH;
   const FxScale sc = fx_z_load<H, true>(x, xH, v, vH);
-  fx_z_c2r_prep<H>(v, vH, t, gbase, twz);
-  fx_z_inverse<H>(v, t, &xs[warp][grp * G::X], twh);
+  zrow_c2r_prep<NumFx, H>(v, vH, t, gbase, twz);
+  zrow_inverse<NumFx, H>(v, t, &xs[warp][grp * G::X], twh);
   if (valid) {
     double2 *dst = reinterpret_cast<double2 *>(out + blockIdx.y * ostride) + row * H;
 #pragma unroll
@@ -512,14 +405,13 @@ __global__ void __launch_bounds__(32 * kFxWarps) k_fx_zc2r(
 template <int H> struct FxZSmem {
   fx2 xs[kFxWarps][FxZG<H>::G * FxZG<H>::X];
   fx2 grad[kFxWarps][2][FxZG<H>::A][32];  // d/dx, d/dy: thread-private
-  double red[2][kFxWarps];
 };
 
 template <int H, bool ZSRC>
 __global__ void __launch_bounds__(32 * kFxWarps, H == 64 ? 4 : H < 64 ? 3 : 2) k_fx_z_rhs(
     const double2 *d4, long long dstride, const double *__restrict__ yfl, const double *ysc,
-    double *lap, double *pout, double *rhoout, double2 *s6, long long sstride4, double2 *s6b,
-    int gw, double *partials, Geom g, FxTab twh, FxTab twz, const long long *__restrict__ ckz,
+    double *lap, double *pout, double *rhoout, double2 *s6, long long sstride, int gw,
+    double *partials, Geom g, FxTab twh, FxTab twz, const long long *__restrict__ ckz,
     int ekz, int lognz) {
   using G = FxZG<H>;
   constexpr int A = G::A, B = G::B, E = G::E;
@@ -557,8 +449,8 @@ __global__ void __launch_bounds__(32 * kFxWarps, H == 64 ? 4 : H < 64 ? 3 : 2) k
       sc = fx_z_load<H, false>(x, xH, v, vH);
       e = sc.out;
     }
-    fx_z_c2r_prep<H>(v, vH, t, gbase, twz);
-    fx_z_inverse<H>(v, t, xch, twh);
+    zrow_c2r_prep<NumFx, H>(v, vH, t, gbase, twz);
+    zrow_inverse<NumFx, H>(v, t, xch, twh);
     e += 4;
     if (a == 3) {
       if (valid) {
@@ -570,7 +462,7 @@ __global__ void __launch_bounds__(32 * kFxWarps, H == 64 ? 4 : H < 64 ? 3 : 2) k
         }
       }
     } else {
-      const int room = fx_room(fx_row_max<H>(fx_max_int(v)), 62);
+      const int room = fx_room(zrow_max<FxZG<H>::B>(fx_max_int(v)), 62);
       const FxShift sh = fx_shift_of(room);
 #pragma unroll
       for (int m = 0; m < A; ++m) v[m] = fx_shift(v[m], sh);
@@ -637,26 +529,7 @@ __global__ void __launch_bounds__(32 * kFxWarps, H == 64 ? 4 : H < 64 ? 3 : 2) k
       }
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    dr += __shfl_down_sync(0xffffffffu, dr, o);
-    dp += __shfl_down_sync(0xffffffffu, dp, o);
-  }
-  if (lane == 0) {
-    sm.red[0][warp] = dr;
-    sm.red[1][warp] = dp;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double sa = 0.0, sb = 0.0;
-#pragma unroll
-    for (int w = 0; w < kFxWarps; ++w) {
-      sa += sm.red[0][w];
-      sb += sm.red[1][w];
-    }
-    partials[2 * blockIdx.x] = sa;
-    partials[2 * blockIdx.x + 1] = sb;
-  }
+  rhs_partial<32 * kFxWarps>(dr, dp, partials);
   if (!gw) return;
 
   // the six products and their forward transforms
@@ -675,16 +548,16 @@ __global__ void __launch_bounds__(32 * kFxWarps, H == 64 ? 4 : H < 64 ? 3 : 2) k
     const int eb = ib == 0 ? ex[0] : (ib == 1 ? ex[1] : ex[2]);
     const double pa = ia == 0 ? post[0] : (ia == 1 ? post[1] : post[2]);
     const double pb = ib == 0 ? post[0] : (ib == 1 ? post[1] : post[2]);
-    const int room = fx_room(fx_row_max<H>(fx_max_int(v)), G::pr);
+    const int room = fx_room(zrow_max<FxZG<H>::B>(fx_max_int(v)), G::pr);
     const FxShift sh = fx_shift_of(room);
 #pragma unroll
     for (int m = 0; m < A; ++m) v[m] = fx_shift(v[m], sh);
-    fx_z_forward<H>(v, t, xch, twh);
+    zrow_forward<NumFx, H>(v, t, xch, twh);
     fx2 xH;
-    fx_z_r2c_post<H>(v, t, gbase, twz, xH);
+    zrow_r2c_post<NumFx, H>(v, t, gbase, twz, xH);
     const int e = ea + eb + 64 - room + 4;
     if (valid) {
-      double2 *dst = (pr < 4 ? s6 + pr * sstride4 : s6b + (pr - 4) * sstride4) + row * (H + 1);
+      double2 *dst = s6 + pr * sstride + row * (H + 1);
       FxScale so;
       so.slow = slow;
       so.post = pa * pb;
@@ -741,18 +614,28 @@ static int fx_upload_twiddles(Ctx *c, void **dst, int L) {
   return IH_OK;
 }
 
-// derivative coefficients of one axis: c1[k] = k_f / 2^e1 (0 on Nyquist),
-// c2[k] = -k_f^2 / 2^e2 in Q62, k folded to [-L/2, L/2)
+// derivative coefficients of one axis: c1[k] = k_f / (odd 2^e1) (0 on Nyquist),
+// c2[k] = -k_f^2 / (odd 2^e2) in Q62, k folded to [-L/2, L/2); odd: the odd part
+// of the transforms' 1 / N factors, whose power of two goes into the exponents
 static void fx_coefs(std::vector<long long> &t, int L, int count, double unit, double unit2, int e1,
-                     int e2) {
+                     int e2, int odd1, int odd2) {
   for (int k = 0; k < count; ++k) {
     const int f = k > L / 2 ? k - L : k;
-    t.push_back(2 * k == L ? 0 : llrintl(ldexpl((long double)unit * f, 62 - e1)));
+    t.push_back(2 * k == L ? 0 : llrintl(ldexpl((long double)unit * f / odd1, 62 - e1)));
   }
   for (int k = 0; k < count; ++k) {
     const int f = k > L / 2 ? L - k : k;
-    t.push_back(-llrintl(ldexpl((long double)unit2 * f * f, 62 - e2)));
+    t.push_back(-llrintl(ldexpl((long double)unit2 * f * f / odd2, 62 - e2)));
   }
+}
+static int fx_odd(int n) {
+  while (n % 2 == 0) n /= 2;
+  return n;
+}
+static int fx_twos(int n) {
+  int s = 0;
+  for (; n % 2 == 0; n /= 2) ++s;
+  return s;
 }
 static int fx_exp(double v) {  // 2^e > v
   int e;
@@ -762,7 +645,8 @@ static int fx_exp(double v) {  // 2^e > v
 
 int fix_tables(Ctx *c) {
   const Geom &g = c->g;
-  if (c->mixed || !g.pow2) return IH_OK;
+  if (c->mixed) return IH_OK;
+  const bool px = pencil_length(g.nx), py = pencil_length(g.ny), pz = zrow_length(g.h);
   IH_TRY(fx_upload_twiddles(c, &c->fx_tw[0], g.nx));
   IH_TRY(fx_upload_twiddles(c, &c->fx_tw[1], g.ny));
   IH_TRY(fx_upload_twiddles(c, &c->fx_tw[2], g.h));
@@ -777,14 +661,16 @@ int fix_tables(Ctx *c) {
   for (int e : c->fx_e)  // a box whose k leave the exponent range of the passes
     if (e < -200 || e > 200) return IH_OK;
   std::vector<long long> t;
-  fx_coefs(t, g.nx, g.nx, g.kxu, g.kx2, c->fx_e[0], c->fx_e[1]);
-  fx_coefs(t, g.ny, g.ny, g.kyu, g.ky2, c->fx_e[2], c->fx_e[3]);
-  fx_coefs(t, g.nz, g.mz, g.kzu, g.kz2, c->fx_e[4], c->fx_e[3]);
+  const int oz = fx_odd(g.nz), ox = fx_odd(g.nx) * oz, oy = fx_odd(g.ny) * oz;
+  fx_coefs(t, g.nx, g.nx, g.kxu, g.kx2, c->fx_e[0], c->fx_e[1], ox, ox);
+  fx_coefs(t, g.ny, g.ny, g.kyu, g.ky2, c->fx_e[2], c->fx_e[3], oy, oy);
+  fx_coefs(t, g.nz, g.mz, g.kzu, g.kz2, c->fx_e[4], c->fx_e[3], oz, oy);
   IH_CUDA(c, cudaMalloc(&c->fx_coef, sizeof(long long) * t.size()));
   c->dev_bytes += sizeof(long long) * t.size();
   IH_CUDA(c, cudaMemcpy(c->fx_coef, t.data(), sizeof(long long) * t.size(),
                         cudaMemcpyHostToDevice));
-  c->fx_on = kFxAll;
+  c->fx_can = (px ? 1 : 0) | (py ? 2 : 0) | (px && py && pz ? 8 | 16 : 0) | (pz ? 64 : 0);
+  c->fx_on = c->fx_can;
   return IH_OK;
 }
 
@@ -798,6 +684,17 @@ static int fx_dispatch(int L, F &&f) {
     case 128: return f.template run<128>();
     case 256: return f.template run<256>();
     case 512: return f.template run<512>();
+    case 12: return f.template run<12>();
+    case 18: return f.template run<18>();
+    case 24: return f.template run<24>();
+    case 36: return f.template run<36>();
+    case 48: return f.template run<48>();
+    case 72: return f.template run<72>();
+    case 96: return f.template run<96>();
+    case 144: return f.template run<144>();
+    case 192: return f.template run<192>();
+    case 288: return f.template run<288>();
+    case 384: return f.template run<384>();
     default: return IH_ERR_ARG;
   }
 }
@@ -818,7 +715,7 @@ struct FxXY {
     const size_t sm = sizeof(fx2) * L * kFxB;
     const dim3 grid((mz + kFxB - 1) / kFxB, outer, count);
     auto kf = sign < 0 ? k_fx_xy<L, kFxB, -1> : k_fx_xy<L, kFxB, +1>;
-    cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    want_smem(kf, sm);
     kf<<<grid, fx_threads<L, kFxB>(), sm, c->stream>>>(data, stride, sj, so, mz, tw);
     return IH_OK;
   }
@@ -844,12 +741,12 @@ struct FxRT {
     const long long *cx = (const long long *)c->fx_coef, *cy = cx + 2 * g.nx,
                     *cz = cy + 2 * g.ny;
     const long long *c1 = axis == 0 ? cx : cy;
-    const int scale = clog2(L) + clog2(g.nz);  // 1 / (L nz)
+    const int scale = fx_twos(L) + fx_twos(g.nz);  // 1 / (L nz), its powers of two
     const int e1 = c->fx_e[2 * axis] - scale, e2 = c->fx_e[2 * axis + 1] - scale;
     const size_t sm = sizeof(fx2) * L * B * 2;
     const dim3 grid((g.mz + B - 1) / B, outer);
     auto kf = axis == 1 ? k_fx_rt<L, B, true> : k_fx_rt<L, B, false>;
-    cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    want_smem(kf, sm);
     kf<<<grid, fx_threads<L, B>(), sm, c->stream>>>(z, d1, d2, sj, so, g.mz, tw, c1, c1 + L,
                                                     cz + g.mz, e1, e2);
     return IH_OK;
@@ -893,6 +790,12 @@ static int fx_z_dispatch(int H, F &&f) {
     case 64: return f.template run<64>();
     case 128: return f.template run<128>();
     case 256: return f.template run<256>();
+    case 6: return f.template run<6>();
+    case 12: return f.template run<12>();
+    case 24: return f.template run<24>();
+    case 48: return f.template run<48>();
+    case 96: return f.template run<96>();
+    case 192: return f.template run<192>();
     default: return IH_ERR_ARG;
   }
 }
@@ -909,7 +812,7 @@ struct FxZRhs {
   double2 *s6;
   int gw;
   double *partials;
-  int *nblk_out, zsrc;
+  int zsrc;
   template <int H>
   int run() {
     const Geom &g = c->g;
@@ -923,19 +826,19 @@ struct FxZRhs {
     const long long *cz = (const long long *)c->fx_coef + 2 * g.nx + 2 * g.ny;
     auto kf = zsrc ? k_fx_z_rhs<H, true> : k_fx_z_rhs<H, false>;
     const size_t sm = sizeof(FxZSmem<H>);
-    cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    kf<<<nblk, 32 * kFxWarps, sm, c->stream>>>(d4, g.M, yfl, ysc, lap, p, rho, s6, g.M,
-                                               s6 + 5 * g.M, gw, partials, g, th, tz, cz,
-                                               c->fx_e[4], clog2(g.nz));
-    *nblk_out = (int)nblk;
+    want_smem(kf, sm);
+    c->z_blocks = (int)nblk;
+    kf<<<nblk, 32 * kFxWarps, sm, c->stream>>>(d4, g.M, yfl, ysc, lap, p, rho, s6, g.M, gw,
+                                               partials, g, th, tz, cz, c->fx_e[4],
+                                               fx_twos(g.nz));
     return IH_OK;
   }
 };
 int fix_z_rhs(Ctx *c, const void *d4, const void *yfl, const double *ysc, void *lap, void *p,
-              void *rho, void *s6, int gw, double *partials, int *nblk_out, int zsrc) {
+              void *rho, void *s6, int gw, double *partials, int zsrc) {
   return fx_z_dispatch(c->g.h, FxZRhs{c, (const double2 *)d4, (const double *)yfl, ysc,
                                       (double *)lap, (double *)p, (double *)rho, (double2 *)s6,
-                                      gw, partials, nblk_out, zsrc});
+                                      gw, partials, zsrc});
 }
 
 }  // namespace ih

@@ -137,37 +137,71 @@ __device__ __forceinline__ fx2 fx_rot32(fx2 v) {
   return v;
 }
 
-template <int R, int... K>
-__device__ __forceinline__ void fx_brev(fx2 (&v)[R], std::integer_sequence<int, K...>) {
-  const fx2 t[R] = {v[Brev<K, clog2(R)>::value]...};
-  ((v[K] = t[K]), ...);
-}
-
-// one radix-2 decimation-in-frequency stage of span LEN, butterfly J..
-template <int R, int LEN, int S, int J>
-__device__ __forceinline__ void fx_stage(fx2 (&v)[R]) {
-  if constexpr (J < LEN / 2) {
-#pragma unroll
-    for (int st = 0; st < R; st += LEN) {
-      const fx2 a = v[st + J], b = v[st + J + LEN / 2];
-      v[st + J] = a + b;
-      v[st + J + LEN / 2] = fx_rot32<S * J * (32 / LEN)>(a - b);
-    }
-    fx_stage<R, LEN, S, J + 1>(v);
+// a[j][k] <- a[j][k] exp(S 2 pi i j k / R)
+template <int R, int S, int J, int M, int I>
+__device__ __forceinline__ void fx_twist(fx2 (&a)[J][M]) {
+  if constexpr (I < J * M) {
+    constexpr int j = I / M, k = I % M;
+    if constexpr (j > 0 && k > 0) a[j][k] = fx_rot32<S * j * k * (32 / R)>(a[j][k]);
+    fx_twist<R, S, J, M, I + 1>(a);
   }
 }
-template <int R, int LEN, int S>
-__device__ __forceinline__ void fx_stages(fx2 (&v)[R]) {
-  if constexpr (LEN > 1) {
-    fx_stage<R, LEN, S, 0>(v);
-    fx_stages<R, LEN / 2, S>(v);
-  }
-}
-// in-register DFT of R <= 32 points, v[k] <- sum_n v[n] exp(S 2 pi i nk/R)
+// in-register DFT of R <= 32 points (a power of two, or three times one), v[k]
+// <- sum_n v[n] exp(S 2 pi i nk/R)
+constexpr long long kFxOneMinusSqrt34 = 0x224c28bd3d9aac62LL;  // 1 - sqrt(3)/2
 template <int R, int S>
 __device__ __forceinline__ void fx_dft(fx2 (&v)[R]) {
-  fx_stages<R, R, S>(v);
-  fx_brev<R>(v, std::make_integer_sequence<int, R>{});
+  if constexpr (R % 3 == 0) {
+    // Good and Thomas' index maps n = Q n1 + 3 n2, k = (k mod 3, k mod Q) leave no
+    // twiddles between the factors 3 and Q
+    constexpr int Q = R / 3;
+    fx2 a[3][Q];
+#pragma unroll
+    for (int n = 0; n < Q; ++n) {
+      const fx2 x0 = v[(3 * n) % R], x1 = v[(Q + 3 * n) % R], x2 = v[(2 * Q + 3 * n) % R];
+      const fx2 s = x1 + x2, d = x1 - x2;
+      const fx2 m = fx_mk(x0.x - ((s.x + 1) >> 1), x0.y - ((s.y + 1) >> 1));
+      const fx2 h = fx_rot90<S>(fx_mk(d.x - fx_mul(d.x, kFxOneMinusSqrt34),
+                                      d.y - fx_mul(d.y, kFxOneMinusSqrt34)));
+      a[0][n] = x0 + s;
+      a[1][n] = m + h;
+      a[2][n] = m - h;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) fx_dft<Q, S>(a[k]);
+#pragma unroll
+    for (int k = 0; k < R; ++k) v[k] = a[k % 3][k % Q];
+  } else if constexpr (R == 2) {
+    const fx2 a = v[0], b = v[1];
+    v[0] = a + b;
+    v[1] = a - b;
+  } else if constexpr (R == 4) {
+    const fx2 s02 = v[0] + v[2], d02 = v[0] - v[2], s13 = v[1] + v[3];
+    const fx2 j13 = fx_rot90<S>(v[1] - v[3]);
+    v[0] = s02 + s13;
+    v[2] = s02 - s13;
+    v[1] = d02 + j13;
+    v[3] = d02 - j13;
+  } else if constexpr (R > 1) {  // one twiddle per value, as in reg_dft
+    constexpr int J = R == 8 ? 2 : 4, M = R / J;
+    fx2 a[J][M];
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+#pragma unroll
+      for (int m = 0; m < M; ++m) a[j][m] = v[j + J * m];
+      fx_dft<M, S>(a[j]);
+    }
+    fx_twist<R, S, J, M, 0>(a);
+#pragma unroll
+    for (int k = 0; k < M; ++k) {
+      fx2 b[J];
+#pragma unroll
+      for (int j = 0; j < J; ++j) b[j] = a[j][k];
+      fx_dft<J, S>(b);
+#pragma unroll
+      for (int q = 0; q < J; ++q) v[k + M * q] = b[q];
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------

@@ -143,6 +143,8 @@ struct Ctx {
   int mixed = 0;                // IH_PREC_MIXED
   size_t tsize = 8;             // sizeof(T)
   cudaStream_t stream = nullptr;
+  cudaStream_t side = nullptr;  // work of an RHS beside the tensor sources' transforms
+  cudaEvent_t fork[3] = {};     // z pass done; scalars written; phi/psi written
   int num_sms = 0;              // multiprocessors of the device
   std::string err;
   size_t dev_bytes = 0;
@@ -159,6 +161,7 @@ struct Ctx {
   void *mask = nullptr;         // filter mask, M values of T
   double *partials = nullptr;   // partials_cap doubles
   long long partials_cap = 0;
+  int z_blocks = 0;             // blocks (pairs of partial sums) of the last z pass
   RhsScalars *rs = nullptr;     // device
   RhsScalars rs_host{};
   // device, 4 * bins + 128 doubles: 4 spectra, then (offsets after 4 * bins)
@@ -220,10 +223,12 @@ struct Ctx {
   double *dt_dev = nullptr;     // step size of the current try (device)
 
   // FFT engines of the x/y passes (per axis) and of the fused x pass, chosen
-  // by fft_autotune; Stockham with 128-byte tiles until tuned
-  int xy_var[2] = {0, 0};
-  int d4_var = 0;
-  int rt_var[2] = {FV_TWOSTEP_HALF, FV_TWOSTEP_HALF};  // x, y round trips (two-step forms)
+  // by fft_autotune; until tuned the register forms (ih_create: three-step in
+  // FP32), which are within 2% of the fastest at 256^3 and below (FP32, six
+  // arrays at 128^3: 21 us against 38 of the shared-memory Stockham engine)
+  int xy_var[2] = {FV_TWOSTEP_HALF, FV_TWOSTEP_HALF};
+  int d4_var = FV_TWOSTEP;
+  int rt_var[2] = {FV_TWOSTEP, FV_TWOSTEP_HALF};  // x, y round trips (two-step forms)
   int roundtrip = 1;  // RHS without filter/output: round trips instead of full spectra
   int tensor_fused = 0;  // update_h fused into the last x pass (autotuner's choice)
   int gw_plane = 0;      // tensor sources plane-major: 1 one cluster per plane, 2 persistent,
@@ -237,12 +242,12 @@ struct Ctx {
   int stage_fusion = 0;  // DOPRI853 stage inputs formed by the RHS of the previous stage
   int velocity_form = 1; // mixed form: stage combinations from the velocity halves only
   int skip_pos = 0;      // set during the stage evaluations of a velocity-form try
-  // FP64 form, power-of-two axes: transforms in 64-bit block fixed point
+  // FP64 form: transforms in 64-bit block fixed point
   // (ih_fix.cu).  fx_on: the passes that run so (bits as the passes of
   // ih_fft_set_engine: 0 x, 1 y, 3 / 4 the round trips, 6 the z passes);
   // fx_tw: twiddles of x, y, h, nz; fx_coef: derivative coefficients;
   // fx_e: their exponents (x first, x second, y first, y and z second, z first)
-  int fx_on = 0;
+  int fx_on = 0, fx_can = 0;    // fx_can: the passes that have the form on this grid
   void *fx_tw[4] = {};
   void *fx_coef = nullptr;
   int fx_e[5] = {};
@@ -296,7 +301,7 @@ int fft_zc2r(Ctx *c, const C2<T> *in, long long in_stride, T *out,
 template <typename T>
 int fft_xy(Ctx *c, C2<T> *data, long long stride, int count, int axis,
            int sign);
-// forward y then x passes of the six tensor sources (spec arrays 0..3, 5, 6),
+// forward y then x passes of the six tensor sources (spec arrays 0..5),
 // in kz slabs of width w (0: whole arrays)
 template <typename T>
 int fft_gw_yx(Ctx *c, C2<T> *spec, int w);
@@ -312,11 +317,10 @@ int fft_x_deriv4_inv(Ctx *c, const C2<T> *phihat, C2<T> *out,
 // d2 and -kz^2 Z / nz to d2 (the x round trip's), completing the laplacian.
 template <typename T>
 int fft_xy_roundtrip(Ctx *c, const C2<T> *z, C2<T> *d1, C2<T> *d2, int axis);
-// The forward x pass of the six S_ij spectra (arrays 0..3 at s03, 4..5 at
-// s45, stride M; z and y passes done) fused with update_h: writes the tensor
+// The forward x pass of the six S_ij spectra (stride M; z and y passes done) fused with update_h: writes the tensor
 // segments of out from those of y (toolbox.c:311-346, 363-397).
 template <typename T>
-int fft_x_tensor(Ctx *c, const C2<T> *s03, const C2<T> *s45, T *y, T *out, double *outsc,
+int fft_x_tensor(Ctx *c, const C2<T> *s6, T *y, T *out, double *outsc,
                  const NextLin *next);
 // Fused last inverse z pass for the RHS: c2r of the four derivative spectra,
 // then per point (grad phi)^2, rho, p (and their FP64 block sums), writes the
@@ -327,7 +331,7 @@ int fft_x_tensor(Ctx *c, const C2<T> *s03, const C2<T> *s45, T *y, T *out, doubl
 template <typename T>
 int fft_z_rhs_fused(Ctx *c, const C2<T> *d4, const T *yfl, const double *ysc,
                     T *lap, T *p, T *rho, C2<T> *s6, int gw, double *partials,
-                    int *nblocks_out, int zsrc, int plane = 0);
+                    int zsrc, int plane = 0);
 // The same pass on the wide-row engine (ih_zwide.cu): nz = 256, in the
 // context's precision (FP32 mixed form or FP64).
 bool fused_wide_ok(const Ctx *c);
@@ -335,7 +339,7 @@ bool fused_wide_ok(const Ctx *c);
 int zr2c_wide_launch(Ctx *c, const void *in, long long istride, void *out, long long ostride,
                      int count);
 int fused_wide_launch(Ctx *c, const void *d4, const void *yfl, const double *ysc, void *lap,
-                      void *p, void *rho, void *s6, int gw, double *partials, int *nblk_out,
+                      void *p, void *rho, void *s6, int gw, double *partials,
                       int zsrc, int plane);
 // plane-major tensor sources (ih_gwplane.cu): mixed form, 256^3, wide z pass;
 // the six sources live in Ctx::gwbuf (a plane-major write would otherwise
@@ -349,6 +353,27 @@ int update_h_tt(Ctx *c, const void *spec, const void *y, void *out, double *outs
 
 int fft_tables(Ctx *c);
 
+// pencils of the fixed-point passes along x and y: 2^a, 3 2^a and 9 2^a points
+// with two factors of at most 16 (32 for 512, 24 for 288 and 384)
+inline bool pencil_length(int L) {
+  switch (L) {
+    case 8: case 12: case 16: case 18: case 24: case 32: case 36: case 48: case 64: case 72:
+    case 96: case 128: case 144: case 192: case 256: case 288: case 384: case 512: return true;
+    default: return false;
+  }
+}
+// the FP32 z passes on the row engine (ih_zrow.cu): mixed form, power-of-two
+// rows other than the 128 complex points of ih_zwide.cu
+bool zrow_ok(const Ctx *c);
+int zrow_pass(Ctx *c, const void *in, long long istride, void *out, long long ostride, int count,
+              bool forward);
+int zrow_rhs(Ctx *c, const void *d4, const void *yfl, const double *ysc, void *lap, void *p,
+             void *rho, void *s6, int gw, double *partials, int zsrc);
+// whether the z pass of the RHS is one fused kernel, and whether the x and y
+// round trips exist (else the full-spectrum route)
+inline bool zfused_ok(const Ctx *c) { return c->g.pow2 || (c->fx_on >> 6 & 1); }
+inline bool roundtrip_ok(const Ctx *c) { return c->g.pow2 || (c->fx_on & 0x58) == 0x58; }
+
 // the fixed-point passes of the FP64 form (ih_fix.cu)
 int fix_tables(Ctx *c);
 int fix_xy(Ctx *c, void *data, long long stride, int count, int axis, int sign, int cols);
@@ -356,7 +381,7 @@ int fix_roundtrip(Ctx *c, const void *z, void *d1, void *d2, int axis);
 int fix_z(Ctx *c, const void *in, long long istride, void *out, long long ostride, int count,
           bool forward);
 int fix_z_rhs(Ctx *c, const void *d4, const void *yfl, const double *ysc, void *lap, void *p,
-              void *rho, void *s6, int gw, double *partials, int *nblk_out, int zsrc);
+              void *rho, void *s6, int gw, double *partials, int zsrc);
 // time every engine variant of the x/y passes and the fused x pass on the
 // context's scratch spectra and keep the fastest
 int fft_autotune(Ctx *c);
@@ -407,8 +432,19 @@ void dopri_tableau(double *cc, double *a, double *b, double *bhh, double *er);
 void dopri_dense_tableau(double *ad, double *d);
 int dopri_dense(Ctx *c, double t_out, int want_output);
 
+// dynamic shared memory of a launch: only above the default limit does a kernel
+// have to be told
+template <typename K>
+inline void want_smem(K *kernel, size_t bytes) {
+  if (bytes > 40 * 1024)  // the limit is 48 KB with the static part
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 // launch geometry helper: blocks for n items with `per` items per thread
+// (fewer where the grid would not give every SM four CTAs: a small grid's
+// kernels are as long as one thread's chain of items)
 inline unsigned grid_for(long long n, int threads, int per = 1) {
+  while (per > 1 && n < 152LL * 4 * threads * per) per /= 2;
   long long b = (n + (long long)threads * per - 1) / ((long long)threads * per);
   if (b < 1) b = 1;
   if (b > 152LL * 16) b = 152LL * 16;  // grid-stride beyond 16 CTAs per SM

@@ -309,7 +309,7 @@ __global__ void k_next_sc(const NextLin nl, const double *ksc, double *outsc) {
 
 // update_h with the TT projection (toolbox.c:311-346, 363-397), FP32: also the
 // next stage's input at the tensor entries of y (nl).  s holds the six S_ij
-// spectra, spectra 4 and 5 at s + 5M.
+// spectra.
 __global__ void __launch_bounds__(256, 3) k_update_h_next(
     const float2 *__restrict__ s, float *y, float *__restrict__ out, const RhsScalars *rs, Geom g,
     const NextLin nl, double *outsc) {
@@ -338,8 +338,8 @@ __global__ void __launch_bounds__(256, 3) k_update_h_next(
     C2<T> n0 = mk2c<T>(0, 0), n1 = mk2c<T>(0, 0);
     T ksq = 0;
     if (id != 0) {  // the zero mode has no sources (its spectra are not read)
-      const C2<T> v[6] = {s[id], s[M + id], s[2 * M + id], s[3 * M + id], s[5 * M + id],
-                          s[6 * M + id]};
+      const C2<T> v[6] = {s[id], s[M + id], s[2 * M + id], s[3 * M + id], s[4 * M + id],
+                          s[5 * M + id]};
       const ModeK<T> q = mode_k<T>(g, m);
       ksq = q.ksq;
       tensor_sources<T>(m, q, v, n0, n1);
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(128) k_update_h_tab(
         ((long long)(sx ? g.nx - i : i) * g.ny + (sy ? g.ny - j : j)) * g.mz + k;
     double2 v[6];
 #pragma unroll
-    for (int a = 0; a < 6; ++a) v[a] = s[(a < 4 ? a : a + 1) * M + id];
+    for (int a = 0; a < 6; ++a) v[a] = s[a * M + id];
     // a coefficient of S_ab in n_cd changes sign with kx (ky) when x (y)
     // occurs an odd number of times in a, b, c, d; n0 is xx (yy for kz = ky =
     // 0) and n1 xy (xz for kz = 0, yz for kz = ky = 0)
@@ -461,8 +461,8 @@ __global__ void __launch_bounds__(256, 3) k_update_h_pf(
       vv[1] = s[M + q];
       vv[2] = s[2 * M + q];
       vv[3] = s[3 * M + q];
-      vv[4] = s[5 * M + q];
-      vv[5] = s[6 * M + q];
+      vv[4] = s[4 * M + q];
+      vv[5] = s[5 * M + q];
     } else {
 #pragma unroll
       for (int a = 0; a < 6; ++a) vv[a] = mk2c<T>(0, 0);
@@ -510,8 +510,7 @@ __global__ void __launch_bounds__(256, 3) k_update_h_pf(
   dh_max_store<T>(mx, outsc);
 }
 
-// The last forward x pass of the six S_ij spectra (arrays 0..3, 5, 6 of
-// spec; z and y passes done) and update_h, writing the tensor segments of
+// The last forward x pass of the six S_ij spectra (z and y passes done) and update_h, writing the tensor segments of
 // out: x passes then k_update_h, or the fused k_fft_x_tensor, as the
 // autotuner chose (Ctx::tensor_fused).  next: the tensor entries of the next
 // stage input too (in y).
@@ -521,9 +520,8 @@ static int tensor_last_pass_t(Ctx *c, C2<T> *s, T *y, T *out, double *outsc,
   const Geom &g = c->g;
   const long long M = g.M;
   if (!x_done) {
-    if (c->tensor_fused && g.pow2) return fft_x_tensor<T>(c, s, s + 5 * M, y, out, outsc, next);
-    IH_TRY((fft_xy<T>(c, s, M, 4, 0, -1)));
-    IH_TRY((fft_xy<T>(c, s + 5 * M, M, 2, 0, -1)));
+    if (c->tensor_fused && g.pow2) return fft_x_tensor<T>(c, s, y, out, outsc, next);
+    IH_TRY((fft_xy<T>(c, s, M, 6, 0, -1)));
   }
   prof_begin(c, KK_UPDATE_H);
   if constexpr (sizeof(T) == 4) {
@@ -954,9 +952,10 @@ int variance_f64(Ctx *c, const double *arr, long long n, double mean, double *de
 }
 
 // The output flag (toolbox.c:251-270), in two parts around the fused z pass
-// (which reuses spec[0..3], spec[5], spec[6] for the GW products).
-// output_pre: psi power spectrum and the laplacian of psi (toolbox.c:172-184)
-// from spec[5] = psihat (filtered when the filter ran).
+// (which reuses spec[0..5] for the GW products).
+// output_pre: phi and psi power spectra from spec[4] = phihat and spec[5] =
+// psihat (filtered when the filter ran), and the laplacian of psi
+// (toolbox.c:172-184).
 template <typename T>
 static int output_pre(Ctx *c, const Vec &y, int psi_ready) {
   const Geom &g = c->g;
@@ -969,6 +968,8 @@ static int output_pre(Ctx *c, const Vec &y, int psi_ready) {
   const size_t hsm = sizeof(double) * bins;
   const unsigned gm = grid_for(M, 256, 8);
   if (!psi_ready) IH_TRY((fft_r2c<T>(c, yfl + 2 * N, 0, spec + 5 * M, 0, 1)));
+  k_power_spectrum<T><<<gm, 256, hsm, c->stream>>>(spec + 4 * M, g, d);
+  IH_TRY(check_launch(c, "k_power_spectrum"));
   k_power_spectrum<T><<<gm, 256, hsm, c->stream>>>(spec + 5 * M, g, d + bins);
   IH_TRY(check_launch(c, "k_power_spectrum"));
   k_lap_spectrum<T><<<gm, 256, 0, c->stream>>>(spec + 5 * M, spec + 6 * M, g);
@@ -976,8 +977,8 @@ static int output_pre(Ctx *c, const Vec &y, int psi_ready) {
   return fft_c2r<T>(c, spec + 6 * M, 0, (T *)c->rbuf[3], 0, 1);
 }
 
-// output_post: phi and rho power spectra, constraints, summaries, GW spectrum
-// (after the reductions; spec[4] = phihat is free once phi_ps is binned).
+// output_post: rho power spectrum, constraints, summaries, GW spectrum (after
+// the reductions; spec[6] is free beside the GW products).
 template <typename T>
 static int output_post(Ctx *c, const Vec &y, const Vec *smry_src) {
   const Geom &g = c->g;
@@ -989,10 +990,8 @@ static int output_post(Ctx *c, const Vec &y, const Vec *smry_src) {
   const int bins = g.bins;
   const size_t hsm = sizeof(double) * bins;
   const unsigned gm = grid_for(M, 256, 8);
-  k_power_spectrum<T><<<gm, 256, hsm, c->stream>>>(spec + 4 * M, g, d);
-  IH_TRY(check_launch(c, "k_power_spectrum"));
-  IH_TRY((fft_r2c<T>(c, rho, 0, spec + 4 * M, 0, 1)));
-  k_power_spectrum<T><<<gm, 256, hsm, c->stream>>>(spec + 4 * M, g, d + 2 * bins);
+  IH_TRY((fft_r2c<T>(c, rho, 0, spec + 6 * M, 0, 1)));
+  k_power_spectrum<T><<<gm, 256, hsm, c->stream>>>(spec + 6 * M, g, d + 2 * bins);
   IH_TRY(check_launch(c, "k_power_spectrum"));
   double *means = d + 4 * bins + 28;  // [phi_mean, dphi_mean]
   const int nb = nblk_reduce(N);
@@ -1051,7 +1050,7 @@ int read_output(Ctx *c, ih_output *out) {
 }
 
 // ---------------------------------------------------------------------------
-// The z part of the RHS for grids with a radix-3 factor, unfused: 4 c2r
+// The z part of the RHS for rows that no fused kernel takes, unfused: 4 c2r
 // passes (d/dx, d/dy, d/dz into the scratch, the laplacian into lap), one
 // pointwise pass (rho, p, their FP64 block sums, the six GW products d_i phi
 // d_j phi written over the derivatives and into the rest of the scratch) and
@@ -1059,11 +1058,12 @@ int read_output(Ctx *c, ih_output *out) {
 // 410-424).
 template <typename T, bool MIXED>
 __global__ void k_pointwise_g(const T *__restrict__ yfl, const double *ysc, T *g0, T *g1, T *g2,
-                              T *g3, T *g4, T *g5, T *pout, T *rhoout, int gw, long long N,
-                              double mass, double *partials) {
+                              T *g3, T *g4, T *g5, T *pout, T *rhoout, int gw, Geom g,
+                              double *partials) {
+  const long long N = g.N;
   const double a_sc = ysc[4];
   const T inv_a2 = (T)(1.0 / (a_sc * a_sc));
-  const T m2 = (T)(mass * mass);
+  const T m2 = (T)(g.mass * g.mass);
   const T third = (T)(1.0 / 3.0);
   const T phib = (T)ysc[0], pib = (T)ysc[1], psib = (T)ysc[2];
   double sr = 0.0, sp = 0.0;
@@ -1086,17 +1086,12 @@ __global__ void k_pointwise_g(const T *__restrict__ yfl, const double *ysc, T *g
       g5[i] = dz * dz;
     }
   }
-  sr = block_sum(sr);
-  sp = block_sum(sp);
-  if (threadIdx.x == 0) {
-    partials[2 * blockIdx.x] = sr;
-    partials[2 * blockIdx.x + 1] = sp;
-  }
+  rhs_partial<256>(sr, sp, partials);
 }
 
 template <typename T>
 static int z_pass_generic(Ctx *c, C2<T> *spec, const T *yfl, const double *ysc, T *lap, T *p,
-                          T *rho, int *nblk_out) {
+                          T *rho) {
   const Geom &g = c->g;
   const long long N = g.N, M = g.M;
   T *gs = (T *)c->gscratch;
@@ -1108,19 +1103,16 @@ static int z_pass_generic(Ctx *c, C2<T> *spec, const T *yfl, const double *ysc, 
   prof_begin(c, KK_Z_RHS_FUSED);
   if (c->mixed)
     k_pointwise_g<T, true><<<nb, 256, 0, c->stream>>>(yfl, ysc, gs, gs + N, gs + 2 * N, gs + 3 * N,
-                                                      gs + 4 * N, gs + 5 * N, p, rho, gw, N,
-                                                      g.mass, c->partials);
+                                                      gs + 4 * N, gs + 5 * N, p, rho, gw, g,
+                                                      c->partials);
   else
     k_pointwise_g<T, false><<<nb, 256, 0, c->stream>>>(yfl, ysc, gs, gs + N, gs + 2 * N,
                                                        gs + 3 * N, gs + 4 * N, gs + 5 * N, p, rho,
-                                                       gw, N, g.mass, c->partials);
+                                                       gw, g, c->partials);
+  c->z_blocks = (int)nb;
   prof_end(c, KK_Z_RHS_FUSED, (6.0 + (gw ? 6.0 : 0.0) + (rho ? 1.0 : 0.0)) * N * sizeof(T));
   IH_TRY(check_launch(c, "k_pointwise_g"));
-  *nblk_out = (int)nb;
-  if (gw) {  // xx, xy, xz, yy -> spec[0..3]; yz, zz -> spec[5], spec[6]
-    IH_TRY((fft_zr2c<T>(c, gs, N, spec, M, 4)));
-    IH_TRY((fft_zr2c<T>(c, gs + 4 * N, N, spec + 5 * M, M, 2)));
-  }
+  if (gw) IH_TRY((fft_zr2c<T>(c, gs, N, spec, M, 6)));  // xx, xy, xz, yy, yz, zz
   return IH_OK;
 }
 
@@ -1138,10 +1130,15 @@ static int rhs_t(Ctx *c, Vec &y, Vec &k, int filter, int output, const Vec *smry
   // the diagnostics stay those of the last RHS run with the output flag
   if (output == 1) c->have_output = 0;
   const int do_filter = (filter == 1) && c->p.enable_filter;
-  // without the filter and the output flag nothing needs the full spectrum
-  // of phi: the derivatives come from round trips along x and y on its z
-  // spectrum Z (spec[4]), the z parts from Z inside the fused z pass
-  const int use_rt = c->roundtrip && c->g.pow2 && !do_filter && output != 1;
+  // the derivatives come from round trips along x and y on the z spectrum Z
+  // of phi (spec[4]), the z parts from Z inside the fused z pass.  The filter
+  // and the output flag need the full spectrum anyway: the FP64 form then takes
+  // one more z pass and the round trips all the same (256^3: 0.84 ms against
+  // 2.4 ms for the derivatives of the full spectrum on the FP64 pipe), the
+  // mixed form the derivatives of the full spectrum.
+  const bool full = do_filter || output == 1;
+  const int use_rt = c->roundtrip && roundtrip_ok(c) &&
+                     (!full || (sizeof(T) == 8 && (c->fx_on & 0x18) == 0x18));
   const unsigned gm = grid_for(M, 256, 4);
   // 1. phihat (and with the filter: dphi, psi, dpsi spectra, mask, write back)
   if (do_filter) {
@@ -1158,12 +1155,11 @@ static int rhs_t(Ctx *c, Vec &y, Vec &k, int filter, int output, const Vec *smry
     prof_end(c, KK_FILTER, (double)M * (9 + (output ? 1 : 0)) * sizeof(C2<T>) + (double)M * sizeof(T));
     IH_TRY(check_launch(c, "k_filter_spectra"));
     IH_TRY((fft_c2r<T>(c, spec, M, yfl, N, 4)));
-  } else if (use_rt) {
-    IH_TRY((fft_zr2c<T>(c, yfl, 0, spec + 4 * M, 0, 1)));
-  } else {
+  } else if (!use_rt || full) {
     IH_TRY((fft_r2c<T>(c, yfl, 0, spec + 4 * M, 0, 1)));
   }
   if (output == 1) IH_TRY(output_pre<T>(c, y, do_filter));
+  if (use_rt) IH_TRY((fft_zr2c<T>(c, yfl, 0, spec + 4 * M, 0, 1)));
   // 2. derivative spectra in (x, y, kz): d/dx, d/dy, (d/dz), laplacian
   if (use_rt) {
     IH_TRY((fft_xy_roundtrip<T>(c, spec + 4 * M, spec, spec + 3 * M, 0)));
@@ -1175,61 +1171,66 @@ static int rhs_t(Ctx *c, Vec &y, Vec &k, int filter, int output, const Vec *smry
   // 3. fused inverse z + pointwise + GW products forward z (the products
   // plane-major where the one-pass plane transforms take them)
   const int plane = sizeof(T) == 4 && c->gw_plane && !next && gw_plane_ok(c);
-  int nblk = 0;
-  if (c->g.pow2)
+  if (zfused_ok(c))
     IH_TRY((fft_z_rhs_fused<T>(c, spec, yfl, y.sc, lap, p, output == 1 ? rho : nullptr,
-                               plane ? (C2<T> *)c->gwbuf : spec, c->p.enable_gw, c->partials,
-                               &nblk, use_rt, plane)));
+                               plane ? (C2<T> *)c->gwbuf : spec, c->p.enable_gw, c->partials, use_rt,
+                               plane)));
   else
-    IH_TRY((z_pass_generic<T>(c, spec, yfl, y.sc, lap, p, output == 1 ? rho : nullptr, &nblk)));
-  k_reduce_finish<<<1, 256, 0, c->stream>>>(c->partials, nblk, g, y.sc, k.sc, c->rs, c->mixed);
-  IH_TRY(check_launch(c, "k_reduce_finish"));
-  // 4. diagnostics that need <rho> and H
-  if (output == 1) IH_TRY(output_post<T>(c, y, smry_src));
-  // 5. tensor modes
-  if (c->p.enable_gw) {
-    // S_ij spectra: spec[0..3] and spec[5..6]; forward y and x passes
-    // (batched: per-array y-then-x ordering measured slower, no L2 reuse;
-    // kz slabs of all six arrays where the autotuner chose them)
-    if (plane && c->gw_plane == 3) {
-      IH_TRY(gw_tt_plane(c, c->gwbuf));
-      IH_TRY(update_h_tt(c, c->gwbuf, yfl, kfl, k.sc));
-    } else if (plane) {
-      IH_TRY(gw_plane_fft(c, c->gwbuf, c->gw_plane));
-      IH_TRY(update_h_plane(c, c->gwbuf, yfl, kfl, k.sc));
-    } else if (c->gw_slab > 0 && !c->tensor_fused && g.pow2) {
-      IH_TRY((fft_gw_yx<T>(c, spec, c->gw_slab)));
-      IH_TRY(tensor_last_pass(c, spec, yfl, kfl, k.sc, next, true));
-    } else {
-      IH_TRY((fft_xy<T>(c, spec, M, 4, 1, -1)));
-      IH_TRY((fft_xy<T>(c, spec + 5 * M, M, 2, 1, -1)));
-      IH_TRY(tensor_last_pass(c, spec, yfl, kfl, k.sc, next));
-    }
+    IH_TRY((z_pass_generic<T>(c, spec, yfl, y.sc, lap, p, output == 1 ? rho : nullptr)));
+  // 4. the scalars and the phi/psi equations of motion (and their part of the
+  // next stage input) beside the tensor sources' transforms, on a second stream:
+  // the reduction is one block and on small grids neither fills the GPU (32^3
+  // to 64^3: 10 to 15 us of an RHS).  The diagnostics and per-kernel timing run
+  // in one stream.
+  const bool fork = output != 1 && !c->prof_on && c->p.enable_gw;
+  const cudaStream_t st = fork ? c->side : c->stream;
+  if (fork) {
+    IH_CUDA(c, cudaEventRecord(c->fork[0], c->stream));
+    IH_CUDA(c, cudaStreamWaitEvent(c->side, c->fork[0], 0));
   }
-  // 6. phi/psi equations of motion (and the next stage input)
+  k_reduce_finish<<<1, 256, 0, st>>>(c->partials, c->z_blocks, g, y.sc, k.sc, c->rs, c->mixed);
+  IH_TRY(check_launch(c, "k_reduce_finish"));
+  if (fork) IH_CUDA(c, cudaEventRecord(c->fork[1], c->side));
+  if (output == 1) IH_TRY(output_post<T>(c, y, smry_src));
   prof_begin(c, KK_UPDATE_PHI_PSI);
   NextLin none{};
   none.skip_pos = c->skip_pos;
   const NextLin &nl = next ? *next : none;
   const unsigned gu = grid_for(N / VecW<T>::W, 256, 4);
-  if (c->mixed) {
-    if (next)
-      k_update_phi_psi<T, true, true><<<gu, 256, 0, c->stream>>>(yfl, y.sc, lap, p, kfl, c->rs, N,
-                                                                 g.mass, nl);
-    else
-      k_update_phi_psi<T, true, false><<<gu, 256, 0, c->stream>>>(yfl, y.sc, lap, p, kfl, c->rs, N,
-                                                                  g.mass, nl);
-  } else {
-    if (next)
-      k_update_phi_psi<T, false, true><<<gu, 256, 0, c->stream>>>(yfl, y.sc, lap, p, kfl, c->rs,
-                                                                  N, g.mass, nl);
-    else
-      k_update_phi_psi<T, false, false><<<gu, 256, 0, c->stream>>>(yfl, y.sc, lap, p, kfl, c->rs,
-                                                                   N, g.mass, nl);
-  }
+  constexpr bool MIXED = sizeof(T) == 4;
+  auto kf = next ? k_update_phi_psi<T, MIXED, true> : k_update_phi_psi<T, MIXED, false>;
+  kf<<<gu, 256, 0, st>>>(yfl, y.sc, lap, p, kfl, c->rs, N, g.mass, nl);
   prof_end(c, KK_UPDATE_PHI_PSI,
            ((nl.skip_pos ? 8.0 : 10.0) + (next ? 4.0 * (next->n + 2) : 0.0)) * N * sizeof(T));
   IH_TRY(check_launch(c, "k_update_phi_psi"));
+  if (fork) IH_CUDA(c, cudaEventRecord(c->fork[2], c->side));
+  // 5. tensor modes
+  if (c->p.enable_gw) {
+    auto join = [&]() {  // the equation of motion reads the scalars
+      return fork ? cudaStreamWaitEvent(c->stream, c->fork[1], 0) : cudaSuccess;
+    };
+    // S_ij spectra: spec[0..5]; forward y and x passes
+    // (batched: per-array y-then-x ordering measured slower, no L2 reuse;
+    // kz slabs of all six arrays where the autotuner chose them)
+    if (plane && c->gw_plane == 3) {
+      IH_TRY(gw_tt_plane(c, c->gwbuf));
+      IH_CUDA(c, join());
+      IH_TRY(update_h_tt(c, c->gwbuf, yfl, kfl, k.sc));
+    } else if (plane) {
+      IH_TRY(gw_plane_fft(c, c->gwbuf, c->gw_plane));
+      IH_CUDA(c, join());
+      IH_TRY(update_h_plane(c, c->gwbuf, yfl, kfl, k.sc));
+    } else if (c->gw_slab > 0 && !c->tensor_fused && g.pow2) {
+      IH_TRY((fft_gw_yx<T>(c, spec, c->gw_slab)));
+      IH_CUDA(c, join());
+      IH_TRY(tensor_last_pass(c, spec, yfl, kfl, k.sc, next, true));
+    } else {
+      IH_TRY((fft_xy<T>(c, spec, M, 6, 1, -1)));
+      IH_CUDA(c, join());
+      IH_TRY(tensor_last_pass(c, spec, yfl, kfl, k.sc, next));
+    }
+  }
+  if (fork) IH_CUDA(c, cudaStreamWaitEvent(c->stream, c->fork[2], 0));
   if (next) {
     k_next_sc<<<1, 32, 0, c->stream>>>(*next, k.sc, y.sc);
     IH_TRY(check_launch(c, "k_next_sc"));

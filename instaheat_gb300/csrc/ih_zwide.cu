@@ -66,7 +66,6 @@ template <typename T> struct WideSmem {
   C2<T> twz[2 * kH];                 // exp(-2 pi i k/nz)
   C2<T> xch[kWarpsW][kRowsW][kXch];
   Q4<T> grad[kWarpsW][2][8][32];     // d/dx, d/dy of each lane's 32 points: [q][lane]
-  double red[2][kWarpsW];
 };
 // with the prefetch: each row's next input spectrum row (kH + 1 values)
 template <typename T> struct WideSmemPF : WideSmem<T> {
@@ -189,7 +188,7 @@ __device__ __forceinline__ void zw_r2c_post(C2<T> (&v)[16], int t, int gbase, co
 template <typename T, bool ZSRC, bool PLANE, bool PF>
 __global__ void __launch_bounds__(32 * kWarpsW, (sizeof(T) == 4 ? (PF ? 3 : 4) : 2)) k_fft_z_rhs_wide(
     const C2<T> *d4, long long dstride, const T *__restrict__ yfl, const double *ysc, T *lap,
-    T *pout, T *rhoout, C2<T> *s6, long long sstride4, C2<T> *s6b, int gw, double *partials,
+    T *pout, T *rhoout, C2<T> *s6, long long sstride, int gw, double *partials,
     Geom g, const C2<T> *__restrict__ twhg, const C2<T> *__restrict__ twzg) {
   using V = C2<T>;
   constexpr bool MIXED = sizeof(T) == 4;  // FP32 fields are fluctuations (mixed form)
@@ -315,26 +314,7 @@ __global__ void __launch_bounds__(32 * kWarpsW, (sizeof(T) == 4 ? (PF ? 3 : 4) :
       dp += (double)((p4.x + p4.y) + (p4.z + p4.w));
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    dr += __shfl_down_sync(0xffffffffu, dr, o);
-    dp += __shfl_down_sync(0xffffffffu, dp, o);
-  }
-  if (lane == 0) {
-    sm.red[0][warp] = dr;
-    sm.red[1][warp] = dp;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    double sa = 0.0, sb = 0.0;
-#pragma unroll
-    for (int w = 0; w < kWarpsW; ++w) {
-      sa += sm.red[0][w];
-      sb += sm.red[1][w];
-    }
-    partials[2 * blockIdx.x] = sa;
-    partials[2 * blockIdx.x + 1] = sb;
-  }
+  rhs_partial<32 * kWarpsW>(dr, dp, partials);
   if (!gw) return;
 
   // 5. the six GW source products d_i phi d_j phi, forward transforms
@@ -355,7 +335,7 @@ __global__ void __launch_bounds__(32 * kWarpsW, (sizeof(T) == 4 ? (PF ? 3 : 4) :
     V xH;
     zw_r2c_post<T>(v, t, gbase, sm.twz, xH);
     if constexpr (PLANE) {
-      V *arr = pr < 4 ? s6 + pr * sstride4 : s6b + (pr - 4) * sstride4;
+      V *arr = s6 + pr * sstride;
 #pragma unroll
       for (int m = 0; m < 16; ++m) xch[t + 8 * m] = v[m];
       if (t == 0) xch[kH] = xH;
@@ -370,7 +350,7 @@ __global__ void __launch_bounds__(32 * kWarpsW, (sizeof(T) == 4 ? (PF ? 3 : 4) :
       }
       __syncwarp();
     } else {
-      V *dst = (pr < 4 ? s6 + pr * sstride4 : s6b + (pr - 4) * sstride4) + rs;
+      V *dst = s6 + pr * sstride + rs;
       if (valid) {
 #pragma unroll
         for (int m = 0; m < 16; ++m) dst[t + 8 * m] = v[m];
@@ -458,14 +438,10 @@ static void wide_launch_pf(Ctx *c, unsigned nblk, const void *d4, long long M, c
                            const double *ysc, void *lap, void *p, void *rho, void *s6, int gw,
                            double *partials, const Geom &g) {
   const size_t sm = PF ? sizeof(WideSmemPF<T>) : sizeof(WideSmem<T>);
-  cudaFuncSetAttribute(k_fft_z_rhs_wide<T, ZSRC, PLANE, PF>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  // row layout: the sources in spectra 0..3, 5, 6 of the RHS block; plane
-  // layout: six consecutive spectra of their own buffer
-  C2<T> *s = reinterpret_cast<C2<T> *>(s6);
+  want_smem(k_fft_z_rhs_wide<T, ZSRC, PLANE, PF>, sm);
   k_fft_z_rhs_wide<T, ZSRC, PLANE, PF><<<nblk, 32 * kWarpsW, sm, c->stream>>>(
-      (const C2<T> *)d4, M, (const T *)yfl, ysc, (T *)lap, (T *)p, (T *)rho, s, M,
-      s + (PLANE ? 4 : 5) * M, gw, partials, g, reinterpret_cast<const C2<T> *>(c->tw_h),
+      (const C2<T> *)d4, M, (const T *)yfl, ysc, (T *)lap, (T *)p, (T *)rho, (C2<T> *)s6, M, gw,
+      partials, g, reinterpret_cast<const C2<T> *>(c->tw_h),
       reinterpret_cast<const C2<T> *>(c->tw_z));
 }
 
@@ -487,7 +463,7 @@ static void wide_launch_t(Ctx *c, unsigned nblk, const void *d4, long long M, co
 }
 
 int fused_wide_launch(Ctx *c, const void *d4, const void *yfl, const double *ysc, void *lap,
-                      void *p, void *rho, void *s6, int gw, double *partials, int *nblk_out,
+                      void *p, void *rho, void *s6, int gw, double *partials,
                       int zsrc, int plane) {
   const Geom &g = c->g;
   const long long rows = (long long)g.nx * g.ny;
@@ -501,6 +477,7 @@ int fused_wide_launch(Ctx *c, const void *d4, const void *yfl, const double *ysc
     c->err = "plane-major tensor sources are a mixed-form path";
     return IH_ERR_STATE;
   }
+  c->z_blocks = (int)nblk;
   const long long M = g.M;
   if (c->mixed) {
     if (zsrc && plane)
@@ -517,7 +494,6 @@ int fused_wide_launch(Ctx *c, const void *d4, const void *yfl, const double *ysc
     else
       wide_launch_t<double, false, false>(c, nblk, d4, M, yfl, ysc, lap, p, rho, s6, gw, partials, g);
   }
-  *nblk_out = (int)nblk;
   return IH_OK;
 }
 

@@ -7,7 +7,9 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 # every pencil length 8..512 along x and y, every row length along z
-GRIDS = [(8, 8, 8), (16, 8, 8), (32, 16, 16), (64, 32, 32), (128, 128, 64), (256, 64, 8),
+GRIDS = [(12, 12, 12), (24, 18, 12), (48, 36, 24), (72, 72, 48), (96, 64, 48), (144, 96, 96),
+         (192, 192, 192), (288, 24, 24), (384, 384, 8), (384, 12, 12),
+         (8, 8, 8), (16, 8, 8), (32, 16, 16), (64, 32, 32), (128, 128, 64), (256, 64, 8),
          (512, 8, 8), (512, 512, 16), (128, 128, 128), (256, 256, 256), (512, 512, 512)]
 
 
@@ -33,7 +35,7 @@ def test_transforms(gpu_mod, n):
     off by about eps sqrt(log2 N) = 1.1e-16 * 4.9 = 5.4e-16, the fixed-point one
     by less; 2e-15 is twice their sum."""
     ctx = gpu_mod.Context(n=n)
-    assert ctx.L_.ih_fft_get_engine(ctx.h, 9) == gpu_mod.FFT_FIXED_ALL
+    assert ctx.L_.ih_fft_get_engine(ctx.h, 9) == gpu_mod.FFT_FIXED_ALL, "all passes"
     x = np.random.default_rng(sum(n)).standard_normal(n)
     X = np.fft.rfftn(x)
     assert norm(ctx.fft(x) - X) <= 2e-15 * norm(X)
@@ -122,7 +124,8 @@ def state(gpu_mod, ctx, seed, amp=1e-3):
 
 
 @pytest.mark.parametrize("n", [(8, 8, 8), (16, 16, 8), (64, 32, 16), (32, 32, 32), (128, 64, 64),
-                               (512, 16, 8), (256, 256, 256)])
+                               (512, 16, 8), (256, 256, 256), (24, 18, 12), (96, 64, 48),
+                               (144, 72, 48), (384, 12, 12), (54, 48, 24), (48, 48, 36)])
 @pytest.mark.parametrize("flag", [0, 1])
 def test_rhs_agrees_with_the_fp64_engines(gpu_mod, n, flag):
     """One right-hand side on the fixed-point passes and on the FP64 engines:
@@ -130,12 +133,13 @@ def test_rhs_agrees_with_the_fp64_engines(gpu_mod, n, flag):
     against the oracle; single passes pinned to an FP64 engine in between."""
     ctx = gpu_mod.Context(n=n, L=(20.0, 17.0, 13.0))
     f = state(gpu_mod, ctx, 5)
+    passes = ctx.L_.ih_fft_get_engine(ctx.h, 9)
     ctx.set_engine(9, 0)
     ref, _ = ctx.mk_rhs(f, filter=flag, output=flag)
-    ctx.set_engine(9, gpu_mod.FFT_FIXED_ALL)
+    ctx.set_engine(9, passes)
     runs = [ctx.mk_rhs(f, filter=flag, output=flag)[0]]
     for p, e in ((0, 1), (1, 2), (3, 2), (4, 1), (6, 1)):
-        ctx.set_engine(9, gpu_mod.FFT_FIXED_ALL)
+        ctx.set_engine(9, passes)
         ctx.set_engine(p, e)
         runs.append(ctx.mk_rhs(f, filter=flag, output=flag)[0])
     N, X = ctx.N, 2 * ctx.M
@@ -173,10 +177,15 @@ def test_rhs_of_waves_along_one_axis_and_at_rest(gpu_mod):
 
 
 def test_pass_9_is_refused_where_it_does_not_apply(gpu_mod):
-    for kw in (dict(n=(32, 32, 32), precision=gpu_mod.PREC_MIXED), dict(n=(48, 32, 32))):
+    """The mixed form; an axis of 54 points (27 x 2), a row of 36 (18 complex
+    values): the passes that remain are offered, the others refused."""
+    for kw, can in ((dict(n=(32, 32, 32), precision=gpu_mod.PREC_MIXED), 0),
+                    (dict(n=(54, 48, 24)), 2 | 64), (dict(n=(48, 48, 36)), 1 | 2),
+                    (dict(n=(48, 32, 32)), gpu_mod.FFT_FIXED_ALL)):
         ctx = gpu_mod.Context(**kw)
-        assert ctx.L_.ih_fft_get_engine(ctx.h, 9) == 0
-        with pytest.raises(gpu_mod.IHError):
-            ctx.set_engine(9, gpu_mod.FFT_FIXED_ALL)
+        assert ctx.L_.ih_fft_get_engine(ctx.h, 9) == can
+        if can != gpu_mod.FFT_FIXED_ALL:
+            with pytest.raises(gpu_mod.IHError):
+                ctx.set_engine(9, gpu_mod.FFT_FIXED_ALL)
         ctx.set_engine(9, 0)
         ctx.close()
