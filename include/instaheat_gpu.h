@@ -182,8 +182,8 @@ int ih_variance_host(ih_context *c, double mean, const double *f_host, size_t n,
  * pass, of the x and y derivative round trips, of the last tensor x pass and
  * the kz slab widths of the tensor sources' y/x passes and, where it
  * applies, the plane-major tail of the tensor sources (pass 8 below) of the
- * RHS on the context's scratch spectra and keeps the fastest per pass.  Until it is called the passes use the register two-step
- * engine.  Results are identical across variants up to rounding.  The report
+ * RHS on the context's scratch spectra and keeps the fastest per pass.  Until
+ * it is called the passes use the shared-memory Stockham engine.  Results are identical across variants up to rounding.  The report
  * lists the timings and the choice (valid until the next ih_autotune). */
 int ih_autotune(ih_context *c);
 const char *ih_autotune_report(const ih_context *c);

@@ -164,7 +164,6 @@ static int create(const ih_params *p, Ctx *c) {
   make_geom(p, &c->g);
   c->mixed = p->precision == IH_PREC_MIXED;
   c->tsize = c->mixed ? 4 : 8;
-  if (c->mixed) c->xy_var[0] = c->xy_var[1] = FV_THREESTEP;
   c->noise_eta = c->mixed ? kDefaultNoiseEta : 0.0;
   IH_CUDA(c, cudaSetDevice(p->device));
   IH_CUDA(c, cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, p->device));

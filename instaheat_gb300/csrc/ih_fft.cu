@@ -1786,8 +1786,6 @@ int fft_zr2c(Ctx *c, const T *in, long long in_stride, C2<T> *out, long long out
   prof_begin(c, KK_FFT_ZR2C);
   if (sizeof(T) == 8 && (c->fx_on >> 6 & 1)) {
     IH_TRY(fix_z(c, in, in_stride, out, out_stride, count, true));
-  } else if (zrow_ok(c)) {
-    IH_TRY(zrow_pass(c, in, in_stride, out, out_stride, count, true));
   } else if (fused_wide_ok(c)) {
     IH_TRY(zr2c_wide_launch(c, in, in_stride, out, out_stride, count));
   } else if (g.h & (g.h - 1)) {
@@ -1811,8 +1809,6 @@ int fft_zc2r(Ctx *c, const C2<T> *in, long long in_stride, T *out, long long out
   prof_begin(c, KK_FFT_ZC2R);
   if (sizeof(T) == 8 && (c->fx_on >> 6 & 1)) {
     IH_TRY(fix_z(c, in, in_stride, out, out_stride, count, false));
-  } else if (zrow_ok(c)) {
-    IH_TRY(zrow_pass(c, in, in_stride, out, out_stride, count, false));
   } else if (g.h & (g.h - 1)) {
     const long long rows = (long long)g.nx * g.ny;
     const size_t sm = zg_smem<T>(g.h);
@@ -2081,8 +2077,6 @@ int fft_z_rhs_fused(Ctx *c, const C2<T> *d4, const T *yfl, const double *ysc, T 
   prof_begin(c, KK_Z_RHS_FUSED);
   if (sizeof(T) == 8 && (c->fx_on >> 6 & 1)) {
     IH_TRY(fix_z_rhs(c, d4, yfl, ysc, lap, p, rho, s6, gw, partials, zsrc));
-  } else if (zrow_ok(c)) {
-    IH_TRY(zrow_rhs(c, d4, yfl, ysc, lap, p, rho, s6, gw, partials, zsrc));
   } else if (fused_wide_ok(c)) {  // nz = 256: the wide-row engine
     IH_TRY(fused_wide_launch(c, d4, yfl, ysc, lap, p, rho, s6, gw, partials, zsrc, plane));
   } else {

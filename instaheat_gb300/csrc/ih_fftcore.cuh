@@ -67,61 +67,52 @@ __device__ __forceinline__ C2<T> w16(int m) {
   }
 }
 
-// In-register DFT of R points (a power of two): v[k] <-
-// sum_n v[n] exp(sign 2 pi i nk/R).  Twiddles are compile-time constants for R <=
-// 16, else tw[m * ts] = exp(-2 pi i m/R).
+// bit reversal of K over BITS bits, as a compile-time constant
+template <int K, int BITS> struct Brev {
+  static constexpr int value = ((K & 1) << (BITS - 1)) | Brev<(K >> 1), BITS - 1>::value;
+};
+template <int K> struct Brev<K, 0> {
+  static constexpr int value = 0;
+};
+
+// v[k] <- v[brev(k)], every index a template constant (the registers are
+// renamed; nothing is staged in local memory)
+template <typename T, int R, int... K>
+__device__ __forceinline__ void brev_permute(C2<T> (&v)[R], std::integer_sequence<int, K...>) {
+  const C2<T> t[R] = {v[Brev<K, clog2(R)>::value]...};
+  ((v[K] = t[K]), ...);
+}
+
+// In-register DFT of R points: v[k] <- sum_n v[n] exp(sign 2 pi i nk/R).
+// Radix-2 decimation in frequency; the bit-reversed result order is undone by
+// a compile-time register permutation.  Twiddles are compile-time constants
+// for R <= 16, else tw[m * ts] = exp(-2 pi i m/R).
 template <typename T, int R>
 __device__ __forceinline__ void reg_dft(C2<T> (&v)[R], const C2<T> *tw, int ts, int sign) {
-  if constexpr (R == 1) {
-    return;
-  } else {
-    // R = J M: M-point DFTs over v[j + J m], the twiddle w_R^(j k1), J-point DFTs
-    // over j.  J = 4 (2 for R = 8): every value meets one twiddle, where radix-2
-    // stages give it up to log2 R - 2 of them (and 10 nontrivial ones instead of 8
-    // for R = 16)
-    if constexpr (R == 2) {
-      const C2<T> a = v[0], b = v[1];
-      v[0] = cadd(a, b);
-      v[1] = csub(a, b);
-    } else if constexpr (R == 4) {
-      const C2<T> s02 = cadd(v[0], v[2]), d02 = csub(v[0], v[2]);
-      const C2<T> s13 = cadd(v[1], v[3]), d13 = csub(v[1], v[3]);
-      const C2<T> j13 = mk2<T>(-(T)sign * d13.y, (T)sign * d13.x);  // sign i (x1 - x3)
-      v[0] = cadd(s02, s13);
-      v[2] = csub(s02, s13);
-      v[1] = cadd(d02, j13);
-      v[3] = csub(d02, j13);
-    } else {
-      constexpr int J = R == 8 ? 2 : 4, M = R / J;
-      C2<T> a[J][M];
+  constexpr int LOGR = clog2(R);
 #pragma unroll
-      for (int j = 0; j < J; ++j) {
+  for (int s = 0; s < LOGR; ++s) {
+    const int len = R >> s, half = len >> 1;
 #pragma unroll
-        for (int m = 0; m < M; ++m) a[j][m] = v[j + J * m];
-        reg_dft<T, M>(a[j], tw, ts * J, sign);
+    for (int st = 0; st < R; st += len) {
 #pragma unroll
-        for (int k = 1; k < M; ++k) {
-          if (j == 0) continue;
-          if (4 * j * k == R) {  // exp(sign i pi/2)
-            a[j][k] = mk2<T>(-(T)sign * a[j][k].y, (T)sign * a[j][k].x);
-          } else {
-            C2<T> w = (R <= 16) ? w16<T>(j * k * (16 / (R <= 16 ? R : 16))) : tw[j * k * ts];
-            if (sign > 0) w.y = -w.y;
-            a[j][k] = cmul(a[j][k], w);
-          }
+      for (int j = 0; j < half; ++j) {
+        const C2<T> a = v[st + j], b = v[st + j + half];
+        v[st + j] = cadd(a, b);
+        const C2<T> d = csub(a, b);
+        if (j == 0) {
+          v[st + j + half] = d;
+        } else if (4 * j == len) {  // exp(sign i pi/2) = sign * i
+          v[st + j + half] = mk2<T>(-(T)sign * d.y, (T)sign * d.x);
+        } else {
+          C2<T> w = (R <= 16) ? w16<T>(j * (16 / len)) : tw[j * (R / len) * ts];
+          if (sign > 0) w.y = -w.y;
+          v[st + j + half] = cmul(d, w);
         }
-      }
-#pragma unroll
-      for (int k = 0; k < M; ++k) {
-        C2<T> b[J];
-#pragma unroll
-        for (int j = 0; j < J; ++j) b[j] = a[j][k];
-        reg_dft<T, J>(b, tw, ts, sign);
-#pragma unroll
-        for (int q = 0; q < J; ++q) v[k + M * q] = b[q];
       }
     }
   }
+  brev_permute<T, R>(v, std::make_integer_sequence<int, R>{});
 }
 
 // conjugate for the inverse direction (S = +1)

@@ -223,12 +223,10 @@ struct Ctx {
   double *dt_dev = nullptr;     // step size of the current try (device)
 
   // FFT engines of the x/y passes (per axis) and of the fused x pass, chosen
-  // by fft_autotune; until tuned the register forms (ih_create: three-step in
-  // FP32), which are within 2% of the fastest at 256^3 and below (FP32, six
-  // arrays at 128^3: 21 us against 38 of the shared-memory Stockham engine)
-  int xy_var[2] = {FV_TWOSTEP_HALF, FV_TWOSTEP_HALF};
-  int d4_var = FV_TWOSTEP;
-  int rt_var[2] = {FV_TWOSTEP, FV_TWOSTEP_HALF};  // x, y round trips (two-step forms)
+  // by fft_autotune; Stockham with 128-byte tiles until tuned
+  int xy_var[2] = {0, 0};
+  int d4_var = 0;
+  int rt_var[2] = {FV_TWOSTEP_HALF, FV_TWOSTEP_HALF};  // x, y round trips (two-step forms)
   int roundtrip = 1;  // RHS without filter/output: round trips instead of full spectra
   int tensor_fused = 0;  // update_h fused into the last x pass (autotuner's choice)
   int gw_plane = 0;      // tensor sources plane-major: 1 one cluster per plane, 2 persistent,
@@ -362,13 +360,6 @@ inline bool pencil_length(int L) {
     default: return false;
   }
 }
-// the FP32 z passes on the row engine (ih_zrow.cu): mixed form, power-of-two
-// rows other than the 128 complex points of ih_zwide.cu
-bool zrow_ok(const Ctx *c);
-int zrow_pass(Ctx *c, const void *in, long long istride, void *out, long long ostride, int count,
-              bool forward);
-int zrow_rhs(Ctx *c, const void *d4, const void *yfl, const double *ysc, void *lap, void *p,
-             void *rho, void *s6, int gw, double *partials, int zsrc);
 // whether the z pass of the RHS is one fused kernel, and whether the x and y
 // round trips exist (else the full-spectrum route)
 inline bool zfused_ok(const Ctx *c) { return c->g.pow2 || (c->fx_on >> 6 & 1); }

@@ -1,5 +1,5 @@
-"""The FP32 transforms of every row and pencil length (power-of-two rows on the
-row engine, ih_zrow.cu) against numpy and the FP64 form."""
+"""The FP32 transforms of every row and pencil length against numpy, and the
+mixed right-hand side against the FP64 form."""
 import numpy as np
 import pytest
 
@@ -54,10 +54,9 @@ def test_longest_rows(gpu_mod, n):
                                (54, 48, 24), (48, 48, 36), (384, 12, 12)])
 @pytest.mark.parametrize("flag", [0, 1])
 def test_rhs_against_fp64(gpu_mod, n, flag):
-    """One right-hand side of the mixed form with the row engine and without
-    (pass 6 engine 0) against the FP64 form: the fluctuation part of each real
-    segment within 1e-5 of its magnitude, the tensor segments within 1e-4, the
-    bounds of the other engines."""
+    """One right-hand side of the mixed form with either z engine against the
+    FP64 form: the fluctuation part of each real segment within 1e-5 of its
+    magnitude, the tensor segments within 1e-4, the bounds of the other engines."""
     ref = gpu_mod.Context(n=n)
     ref.ic(seed=5, amp=1e-3)
     f = ref.get_state()
