@@ -64,6 +64,11 @@ struct RhsScalars {
   double rho_bar, p_bar;        // FP64 homogeneous parts (mixed form)
   double dphi_mean, phi_mean;   // full means (psi solve, constraints)
   double ddphi_mean;            // mean of the dphi-RHS (psi solve)
+  // the factors of the equations of motion, formed once: a thread of theirs
+  // handles few points, and an FP64 division and a few conversions per thread
+  // were a third of the FP32 kernels' time at 128^3
+  double inv_a2, two_inv_a2;    // 1 / a^2, 2 / a^2
+  float f_inv_a2, f_two_inv_a2, f_H, f_h3, f_pm, f_pm2;  // also 3 H, <p>, 2 <p>
   int nonfinite;                // set when a reduction saw NaN/Inf
   int pad;
 };

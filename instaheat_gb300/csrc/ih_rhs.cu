@@ -169,6 +169,14 @@ __global__ void k_reduce_finish(const double *partials, int nblk, Geom g,
   r.dphi_mean = 0.0;
   r.phi_mean = 0.0;
   r.ddphi_mean = 0.0;
+  r.inv_a2 = 1.0 / r.a2;
+  r.two_inv_a2 = 2.0 / r.a2;
+  r.f_inv_a2 = (float)r.inv_a2;
+  r.f_two_inv_a2 = (float)r.two_inv_a2;
+  r.f_H = (float)H;
+  r.f_h3 = (float)(3.0 * H);
+  r.f_pm = (float)p_mean;
+  r.f_pm2 = (float)(2.0 * p_mean);
   r.nonfinite = !(isfinite(rho_mean) && isfinite(p_mean));
   r.pad = 0;
   *rs = r;
@@ -220,12 +228,23 @@ __device__ __forceinline__ void st_w(T *p, const T (&v)[VecW<T>::W]) {
 template <typename T, bool MIXED, bool NEXT>
 __global__ void k_update_phi_psi(T *y, const double *ysc, const T *__restrict__ lap,
                                  const T *__restrict__ p, T *__restrict__ out,
-                                 const RhsScalars *rs, long long N, double mass,
-                                 const NextLin nl) {
+                                 const RhsScalars *rs, long long N, T m2, const NextLin nl) {
   constexpr int W = VecW<T>::W;
-  const double a2d = rs->a2, Hd = rs->H, pmd = rs->p_mean;
-  const T inv_a2 = (T)(1.0 / a2d), H = (T)Hd, h3 = (T)(3.0 * Hd), pm = (T)pmd;
-  const T m2 = (T)(mass * mass);
+  T inv_a2, H, h3, pm;
+  if constexpr (MIXED) {
+    inv_a2 = rs->f_inv_a2;
+    H = rs->f_H;
+    h3 = rs->f_h3;
+    pm = rs->f_pm;
+  } else {
+    inv_a2 = rs->inv_a2;
+    H = rs->H;
+    h3 = 3.0 * H;
+    pm = rs->p_mean;
+  }
+  // FP64: the factors of the fused multiply-adds below (10 FP64 instructions
+  // a point; the FP64 pipe bounds that form)
+  const T ia4 = (T)4 * inv_a2, m22 = (T)2 * m2, H4 = (T)4 * H;
   T phib = 0, pib = 0, psib = 0, dpsib = 0;
   if (MIXED) {
     phib = (T)ysc[0];
@@ -248,9 +267,11 @@ __global__ void k_update_phi_psi(T *y, const double *ysc, const T *__restrict__ 
 #pragma unroll
     for (int w = 0; w < W; ++w) {
       if (!MIXED) {
-        o1[w] = ((T)1.0 + (T)4.0 * ps[w]) * l[w] * inv_a2 - (h3 - (T)4.0 * dps[w]) * dph[w] -
-                ((T)1.0 + (T)2.0 * ps[w]) * (m2 * ph[w]);
-        o3[w] = (T)0.5 * pp[w] + (ps[w] - (T)0.5) * pm - (T)4.0 * H * dps[w];
+        // (1 + 4 psi) lap / a^2 - (3 H - 4 dpsi) dphi - (1 + 2 psi) m^2 phi and
+        // p / 2 + (psi - 1/2) <p> - 4 H dpsi
+        o1[w] = fma(fma(ps[w], ia4, inv_a2), l[w],
+                    -fma(fma(dps[w], (T)-4.0, h3), dph[w], fma(ps[w], m22, m2) * ph[w]));
+        o3[w] = fma((T)0.5, pp[w] - pm, fma(ps[w], pm, -(H4 * dps[w])));
       } else {
         T psf = psib + ps[w], dpsf = dpsib + dps[w];
         o1[w] = ((T)1.0 + (T)4.0 * psf) * l[w] * inv_a2 + (T)4.0 * dps[w] * pib -
@@ -1199,7 +1220,7 @@ static int rhs_t(Ctx *c, Vec &y, Vec &k, int filter, int output, const Vec *smry
   const unsigned gu = grid_for(N / VecW<T>::W, 256, 4);
   constexpr bool MIXED = sizeof(T) == 4;
   auto kf = next ? k_update_phi_psi<T, MIXED, true> : k_update_phi_psi<T, MIXED, false>;
-  kf<<<gu, 256, 0, st>>>(yfl, y.sc, lap, p, kfl, c->rs, N, g.mass, nl);
+  kf<<<gu, 256, 0, st>>>(yfl, y.sc, lap, p, kfl, c->rs, N, (T)(g.mass * g.mass), nl);
   prof_end(c, KK_UPDATE_PHI_PSI,
            ((nl.skip_pos ? 8.0 : 10.0) + (next ? 4.0 * (next->n + 2) : 0.0)) * N * sizeof(T));
   IH_TRY(check_launch(c, "k_update_phi_psi"));

@@ -54,9 +54,19 @@ __device__ __forceinline__ double ksq64(const Geom &g, int i, int j, int k) {
 // the RHS scalars the tensor equation of motion uses, in T
 template <typename T> struct TensorConsts {
   T inv_a2, two_inv_a2, h3, pm2;
-  __device__ __forceinline__ explicit TensorConsts(const RhsScalars *rs)
-      : inv_a2((T)(1.0 / rs->a2)), two_inv_a2((T)(2.0 / rs->a2)), h3((T)(3.0 * rs->H)),
-        pm2((T)(2.0 * rs->p_mean)) {}
+  __device__ __forceinline__ explicit TensorConsts(const RhsScalars *rs) {
+    if constexpr (sizeof(T) == 4) {
+      inv_a2 = rs->f_inv_a2;
+      two_inv_a2 = rs->f_two_inv_a2;
+      h3 = rs->f_h3;
+      pm2 = rs->f_pm2;
+    } else {
+      inv_a2 = rs->inv_a2;
+      two_inv_a2 = rs->two_inv_a2;
+      h3 = 3.0 * rs->H;
+      pm2 = 2.0 * rs->p_mean;
+    }
+  }
 };
 
 // k components of mode m in T (FP64: the reference's expressions; FP32: the
