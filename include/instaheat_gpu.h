@@ -256,9 +256,10 @@ int ih_velocity_form(ih_context *c, int on);
 
 /* CUDA graphs (no reference counterpart): each DOPRI853 try (its 11 stage
  * combinations and RHS evaluations, the final combination and the error
- * reduction) and each filtered post-step RHS without diagnostics is captured
- * once per combination of the vectors it touches and replayed as one graph
- * launch; the step size is read from device memory.  On by default; off
+ * reduction), each filtered post-step RHS without diagnostics and, from the
+ * second time it meets its vectors, each RK4 step without diagnostics is
+ * captured once per combination of the vectors it touches and replayed as one
+ * graph launch; the step size is read from device memory.  On by default; off
  * while per-kernel timing (ih_profile_enable) or the error breakdown is on.
  * Results are identical either way. */
 int ih_graphs_enable(ih_context *c, int on);

@@ -216,7 +216,7 @@ struct Ctx {
   // CUDA graphs of the DOPRI853 try and of the filtered post-step RHS, one per
   // combination of the vectors they touch (see ih_stepper.cu)
   struct Graph {
-    int kind = 0;               // 0 try, 1 post-step RHS
+    int kind = 0;               // 0 try, 1 post-step RHS, 2 RK4 step
     unsigned epoch = 0;
     const void *key[4] = {nullptr, nullptr, nullptr, nullptr};
     cudaGraphExec_t exec = nullptr;
@@ -225,6 +225,7 @@ struct Ctx {
   std::vector<Graph> graphs;
   unsigned graph_epoch = 0;     // advanced when a captured parameter changes
   int graphs_on = 1;
+  int rk4_seen = 0;             // orders of y and ynew that an RK4 step has run in
   double *dt_dev = nullptr;     // step size of the current try (device)
 
   // FFT engines of the x/y passes (per axis) and of the fused x pass, chosen
