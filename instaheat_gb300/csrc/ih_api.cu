@@ -221,6 +221,7 @@ static void destroy(Ctx *c) {
     if (p) cudaFree(p);
   if (c->fx_coef) cudaFree(c->fx_coef);
   if (c->tensor_coef) cudaFree(c->tensor_coef);
+  if (c->shell) cudaFree(c->shell);
   if (c->spec[0]) cudaFree(c->spec[0]);
   if (c->rbuf[0]) cudaFree(c->rbuf[0]);
   if (c->gscratch) cudaFree(c->gscratch);

@@ -580,8 +580,11 @@ int tensor_last_pass(Ctx *c, void *spec, void *y, void *out, double *outsc,
 
 // ---------------------------------------------------------------------------
 // generic FP64 reductions of T arrays (deterministic two-stage)
+// (rows of n values: blockIdx.y)
 template <typename T>
 __global__ void k_partial_sum(const T *a, long long n, double *partials) {
+  a += blockIdx.y * n;
+  partials += blockIdx.y * gridDim.x;
   double s = 0.0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
@@ -742,61 +745,110 @@ int vec_copy(Ctx *c, const Vec &src, Vec &dst) {
 
 // ---------------------------------------------------------------------------
 // diagnostics (toolbox.c:251-270, 435-484, 524-551, 567-582, 634-690)
+// Shell of every mode of the octant i <= nx/2, j <= ny/2 (the others share it):
+// the index of toolbox.c:479, 578 with the reference's operations (a square
+// root and a division in FP64 per mode, once instead of in each of the four
+// spectra of every output)
+__global__ void k_shell_table(int *shell, Geom g) {
+  const int nyh = g.ny / 2 + 1;
+  const long long Mo = (long long)(g.nx / 2 + 1) * nyh * g.mz;
+  for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < Mo;
+       o += (long long)gridDim.x * blockDim.x) {
+    const int k = (int)(o % g.mz), j = (int)(o / g.mz % nyh), i = (int)(o / g.mz / nyh);
+    const int idx = (int)trunc(g.bins * sqrt(ksq64(g, i, j, k)) / g.kmax - 1.0e-14);
+    shell[o] = min(max(idx, 0), g.bins - 1);
+  }
+}
+__device__ __forceinline__ int shell_of(const int *shell, const Geom &g, Mode m) {
+  const int i = m.i > g.nx / 2 ? g.nx - m.i : m.i, j = m.j > g.ny / 2 ? g.ny - m.j : m.j;
+  return shell[((long long)i * (g.ny / 2 + 1) + j) * g.mz + m.k];
+}
+// v into hist[key] for every lane of a full warp (key < 0: nothing).  Neighbouring
+// modes fall into the same or the next shell, and FP64 atomics on one address
+// of shared memory follow one another: runs of equal keys are added up in the
+// warp first.
+__device__ __forceinline__ void hist_add(double *hist, int key, double v) {
+  const int lane = threadIdx.x & 31;
+  const int before = __shfl_up_sync(0xffffffffu, key, 1);
+  const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || before != key);
+  const unsigned later = lane == 31 ? 0u : heads >> (lane + 1);
+  const int run = later ? __ffs((int)later) : 32 - lane;  // to the end of the lane's run
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double w = __shfl_down_sync(0xffffffffu, v, o);
+    if (o < run) v += w;
+  }
+  if ((heads >> lane & 1) && key >= 0) atomicAdd(&hist[key], v);
+}
+__device__ __forceinline__ void hist_out(const double *hist, int bins, double scale, double *out) {
+  __syncthreads();
+  for (int b = threadIdx.x; b < bins; b += blockDim.x) atomicAdd(&out[b], hist[b] * scale);
+}
+
+// power spectra of gridDim.y consecutive spectra into consecutive rows of out
 template <typename T>
-__global__ void k_power_spectrum(const C2<T> *c, Geom g, double *out) {
+__global__ void k_power_spectrum(const C2<T> *c, Geom g, const int *shell, double *out) {
   extern __shared__ double hist[];
   for (int b = threadIdx.x; b < g.bins; b += blockDim.x) hist[b] = 0.0;
   __syncthreads();
-  for (long long id = 1 + blockIdx.x * (long long)blockDim.x + threadIdx.x; id < g.M;
-       id += (long long)gridDim.x * blockDim.x) {
-    Mode m = mode_of(id, g);
-    C2<T> v = c[id];
-    double p2 = (double)v.x * (double)v.x + (double)v.y * (double)v.y;
-    if (fabs(kz_deriv(g, m.k)) > DBL_EPSILON) p2 *= 2.0;
-    int idx = (int)trunc(g.bins * sqrt(ksq64(g, m.i, m.j, m.k)) / g.kmax - 1.0e-14);
-    idx = min(max(idx, 0), g.bins - 1);
-    atomicAdd(&hist[idx], p2 / (double)g.N);
+  c += blockIdx.y * g.M;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long base = blockIdx.x * (long long)blockDim.x; base < g.M; base += stride) {
+    const long long id = base + threadIdx.x;
+    double p2 = 0.0;
+    int key = -1;
+    if (id > 0 && id < g.M) {
+      const Mode m = mode_of(id, g);
+      const C2<T> v = c[id];
+      p2 = (double)v.x * (double)v.x + (double)v.y * (double)v.y;
+      if (m.k != 0 && 2 * m.k != g.nz) p2 *= 2.0;  // kz_deriv != 0
+      key = shell_of(shell, g, m);
+    }
+    hist_add(hist, key, p2);
   }
-  __syncthreads();
-  for (int b = threadIdx.x; b < g.bins; b += blockDim.x) atomicAdd(&out[b], hist[b]);
+  hist_out(hist, g.bins, 1.0 / (double)g.N, out + blockIdx.y * g.bins);
 }
 
 template <typename T>
-__global__ void k_gw_spectrum(const T *y, const RhsScalars *rs, Geom g, double rat,
-                              double *out) {
+__global__ void k_gw_spectrum(const T *y, const RhsScalars *rs, Geom g, const int *shell,
+                              double rat, double *out) {
   extern __shared__ double hist[];
   for (int b = threadIdx.x; b < g.bins; b += blockDim.x) hist[b] = 0.0;
   __syncthreads();
   const long long N = g.N, Next = g.Next;
-  const long long Ndh1 = 4 * N + 2 * Next, Ndh2 = Ndh1 + Next;
-  const double H = rs->H;
-  const double fac = kPi * rat / (3.0 * H * H * g.lx * g.ly * g.lz);
-  for (long long id = 1 + blockIdx.x * (long long)blockDim.x + threadIdx.x; id < g.M;
-       id += (long long)gridDim.x * blockDim.x) {
-    Mode m = mode_of(id, g);
-    double kx = kxf_of(g, m.i), ky = kyf_of(g, m.j), kz = kzf_of(g, m.k);
-    double kx2 = kx * kx, ky2 = ky * ky, kz2 = kz * kz;
-    double k2 = ksq64(g, m.i, m.j, m.k), k = sqrt(k2);
-    double d1r = y[Ndh1 + 2 * id], d2r = y[Ndh2 + 2 * id];
-    double d1i = y[Ndh1 + 2 * id + 1], d2i = y[Ndh2 + 2 * id + 1];
-    double pw;
-    if (fabs(kz) > DBL_EPSILON) {
-      pw = 2.0 * k2 / (kz2 * (ky2 + kz2)) *
-           ((kx2 + kz2) * (d1r * d1r + d1i * d1i) + 2.0 * kx * ky * (d1r * d2r + d1i * d2i) +
-            (ky2 + kz2) * (d2r * d2r + d2i * d2i));
-    } else if (fabs(ky) > DBL_EPSILON) {
-      pw = 2.0 * (kx2 + ky2) / (ky2 * ky2) *
-           ((kx2 + ky2) * (d1r * d1r + d1i * d1i) + ky2 * (d2r * d2r + d2i * d2i));
-    } else {
-      pw = 2.0 * (d1r * d1r + d1i * d1i + d2r * d2r + d2i * d2i);
+  const C2<T> *dh1 = reinterpret_cast<const C2<T> *>(y + 4 * N + 2 * Next);
+  const C2<T> *dh2 = reinterpret_cast<const C2<T> *>(y + 4 * N + 3 * Next);
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long base = blockIdx.x * (long long)blockDim.x; base < g.M; base += stride) {
+    const long long id = base + threadIdx.x;
+    double pw = 0.0;
+    int key = -1;
+    if (id > 0 && id < g.M) {
+      const Mode m = mode_of(id, g);
+      const double kx = kxf_of(g, m.i), ky = kyf_of(g, m.j), kz = kzf_of(g, m.k);
+      const double kx2 = kx * kx, ky2 = ky * ky, kz2 = kz * kz;
+      const double k2 = ksq64(g, m.i, m.j, m.k);
+      const C2<T> d1 = dh1[id], d2 = dh2[id];
+      const double d1r = d1.x, d1i = d1.y, d2r = d2.x, d2i = d2.y;
+      const double p11 = d1r * d1r + d1i * d1i, p22 = d2r * d2r + d2i * d2i;
+      if (m.k != 0) {
+        const double q = ky2 + kz2;
+        pw = 2.0 * k2 / (kz2 * q) *
+             ((kx2 + kz2) * p11 + 2.0 * kx * ky * (d1r * d2r + d1i * d2i) + q * p22);
+      } else if (m.j != 0) {
+        const double q = kx2 + ky2;
+        pw = 2.0 * q / (ky2 * ky2) * (q * p11 + ky2 * p22);
+      } else {
+        pw = 2.0 * (p11 + p22);
+      }
+      if (m.k != 0 && 2 * m.k != g.nz) pw *= 2.0;  // kz_deriv != 0
+      pw *= k2 * sqrt(k2);
+      key = shell_of(shell, g, m);
     }
-    if (fabs(kz_deriv(g, m.k)) > DBL_EPSILON) pw *= 2.0;
-    int idx = (int)trunc(g.bins * k / g.kmax - 1.0e-14);
-    idx = min(max(idx, 0), g.bins - 1);
-    atomicAdd(&hist[idx], fac * k2 * k * pw / (double)N);
+    hist_add(hist, key, pw);
   }
-  __syncthreads();
-  for (int b = threadIdx.x; b < g.bins; b += blockDim.x) atomicAdd(&out[b], hist[b]);
+  const double H = rs->H;
+  hist_out(hist, g.bins, kPi * rat / (3.0 * H * H * g.lx * g.ly * g.lz) / (double)g.N, out);
 }
 
 // -k^2 psihat / N (toolbox.c:177-184) into a work spectrum
@@ -870,30 +922,45 @@ __global__ void k_constraints_finish(const double *partials, int nb, long long N
   }
 }
 
-// summary of a field x_i = add + a[i] (mean, corrected variance, min, max;
-// toolbox.c:676-690, 744-754).  Two passes.
+// Summaries (mean, corrected variance, min, max; toolbox.c:676-690, 744-754) of
+// six fields at once, blockIdx.y the field: phi, dphi, psi, dpsi of a state, rho
+// and p, each an array of fluctuations about its homogeneous part (0 in the
+// plain form).  Two passes over the fields with a block per field after each.
+struct SmryArgs {
+  const void *a[6];
+  const double *sc;       // homogeneous parts of the state
+  const RhsScalars *rs;   // of rho and p
+  __device__ __forceinline__ double add(int f) const {
+    return f < 4 ? sc[f] : (f == 4 ? rs->rho_bar : rs->p_bar);
+  }
+};
 template <typename T>
-__global__ void k_smry1(const T *a, double add, long long n, double *partials) {
-  double s = 0.0, mn = INFINITY, mx = -INFINITY;
+__global__ void k_smry1(const SmryArgs s, long long n, double *partials) {
+  const T *a = reinterpret_cast<const T *>(s.a[blockIdx.y]);
+  double sum = 0.0;
+  T mn = INFINITY, mx = -INFINITY;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
-    double v = add + (double)a[i];
-    s += v;
+    const T v = a[i];
+    sum += (double)v;
     mn = fmin(mn, v);
     mx = fmax(mx, v);
   }
-  s = block_sum(s);
+  sum = block_sum(sum);
   __syncthreads();
-  mn = block_min(mn);
+  const double lo = block_min((double)mn);
   __syncthreads();
-  mx = block_max(mx);
+  const double hi = block_max((double)mx);
   if (threadIdx.x == 0) {
-    partials[3 * blockIdx.x] = s;
-    partials[3 * blockIdx.x + 1] = mn;
-    partials[3 * blockIdx.x + 2] = mx;
+    double *p = partials + 3 * (blockIdx.y * gridDim.x + blockIdx.x);
+    p[0] = sum;
+    p[1] = lo;
+    p[2] = hi;
   }
 }
-__global__ void k_smry1_finish(const double *partials, int nb, long long n, double *out) {
+__global__ void k_smry1_finish(const double *partials, int nb, const SmryArgs a, long long n,
+                               double *out) {
+  partials += 3 * (long long)blockIdx.x * nb;
   double s = 0, mn = INFINITY, mx = -INFINITY;
   for (int i = threadIdx.x; i < nb; i += blockDim.x) {
     s += partials[3 * i];
@@ -906,10 +973,41 @@ __global__ void k_smry1_finish(const double *partials, int nb, long long n, doub
   __syncthreads();
   mx = block_max(mx);
   if (threadIdx.x == 0) {
-    out[0] = s / (double)n;
-    out[2] = mn;
-    out[3] = mx;
+    const double add = a.add(blockIdx.x);
+    out += 4 * blockIdx.x;
+    out[0] = add + s / (double)n;
+    out[2] = add + mn;
+    out[3] = add + mx;
   }
+}
+template <typename T>
+__global__ void k_smry_var(const SmryArgs s, long long n, const double *out, double *partials) {
+  const T *a = reinterpret_cast<const T *>(s.a[blockIdx.y]);
+  const double mean = out[4 * blockIdx.y] - s.add(blockIdx.y);
+  double s1 = 0.0, s2 = 0.0;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    const double d = (double)a[i] - mean;
+    s1 += d * d;
+    s2 += d;
+  }
+  s1 = block_sum(s1);
+  __syncthreads();
+  s2 = block_sum(s2);
+  if (threadIdx.x == 0) {
+    double *p = partials + 2 * (blockIdx.y * gridDim.x + blockIdx.x);
+    p[0] = s1;
+    p[1] = s2;
+  }
+}
+// means of gridDim.x consecutive fields of n values (k_partial_sum in rows) plus
+// their homogeneous parts
+__global__ void k_finish_means(const double *partials, int nb, long long n, const double *add,
+                               double *out) {
+  double s = 0.0;
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) s += partials[blockIdx.x * nb + b];
+  s = block_sum(s);
+  if (threadIdx.x == 0) out[blockIdx.x] = add[blockIdx.x] + s * (1.0 / (double)n);
 }
 template <typename T>
 __global__ void k_smry2(const T *a, double add, long long n, const double *meanp,
@@ -930,7 +1028,10 @@ __global__ void k_smry2(const T *a, double add, long long n, const double *meanp
     partials[2 * blockIdx.x + 1] = s2;
   }
 }
+// (rows of partial sums and of results: blockIdx.x the field)
 __global__ void k_smry2_finish(const double *partials, int nb, long long n, double *out) {
+  partials += 2 * (long long)blockIdx.x * nb;
+  out += 4 * blockIdx.x;
   double s1 = 0, s2 = 0;
   for (int i = threadIdx.x; i < nb; i += blockDim.x) {
     s1 += partials[2 * i];
@@ -942,21 +1043,16 @@ __global__ void k_smry2_finish(const double *partials, int nb, long long n, doub
   if (threadIdx.x == 0) out[1] = (s1 - s2 * s2 / (double)n) / (double)(n - 1);
 }
 
-// homogeneous add for a per-point field whose FP64 part lives in a scalar
-__global__ void k_copy_scalar(const double *src, double *dst) { *dst = *src; }
-
 template <typename T>
-static int summary(Ctx *c, const T *a, const double *add_dev_unused, double add, long long n,
-                   double *out) {
-  (void)add_dev_unused;
+static int summaries(Ctx *c, const SmryArgs &a, long long n, double *out) {
   const int nb = nblk_reduce(n);
-  k_smry1<T><<<nb, 256, 0, c->stream>>>(a, add, n, c->partials);
+  k_smry1<T><<<dim3(nb, 6), 256, 0, c->stream>>>(a, n, c->partials);
   IH_TRY(check_launch(c, "k_smry1"));
-  k_smry1_finish<<<1, 256, 0, c->stream>>>(c->partials, nb, n, out);
+  k_smry1_finish<<<6, 256, 0, c->stream>>>(c->partials, nb, a, n, out);
   IH_TRY(check_launch(c, "k_smry1_finish"));
-  k_smry2<T><<<nb, 256, 0, c->stream>>>(a, add, n, out, c->partials);
-  IH_TRY(check_launch(c, "k_smry2"));
-  k_smry2_finish<<<1, 256, 0, c->stream>>>(c->partials, nb, n, out);
+  k_smry_var<T><<<dim3(nb, 6), 256, 0, c->stream>>>(a, n, out, c->partials);
+  IH_TRY(check_launch(c, "k_smry_var"));
+  k_smry2_finish<<<6, 256, 0, c->stream>>>(c->partials, nb, n, out);
   return check_launch(c, "k_smry2_finish");
 }
 
@@ -988,10 +1084,15 @@ static int output_pre(Ctx *c, const Vec &y, int psi_ready) {
   IH_CUDA(c, cudaMemsetAsync(d, 0, sizeof(double) * (4 * bins + 4 + 24), c->stream));
   const size_t hsm = sizeof(double) * bins;
   const unsigned gm = grid_for(M, 256, 8);
+  if (!c->shell) {  // at the first output
+    const size_t n = (size_t)(g.nx / 2 + 1) * (g.ny / 2 + 1) * g.mz;
+    IH_CUDA(c, cudaMalloc((void **)&c->shell, sizeof(int) * n));
+    c->dev_bytes += sizeof(int) * n;
+    k_shell_table<<<grid_for((long long)n, 256, 1), 256, 0, c->stream>>>(c->shell, g);
+    IH_TRY(check_launch(c, "k_shell_table"));
+  }
   if (!psi_ready) IH_TRY((fft_r2c<T>(c, yfl + 2 * N, 0, spec + 5 * M, 0, 1)));
-  k_power_spectrum<T><<<gm, 256, hsm, c->stream>>>(spec + 4 * M, g, d);
-  IH_TRY(check_launch(c, "k_power_spectrum"));
-  k_power_spectrum<T><<<gm, 256, hsm, c->stream>>>(spec + 5 * M, g, d + bins);
+  k_power_spectrum<T><<<dim3(gm, 2), 256, hsm, c->stream>>>(spec + 4 * M, g, c->shell, d);
   IH_TRY(check_launch(c, "k_power_spectrum"));
   k_lap_spectrum<T><<<gm, 256, 0, c->stream>>>(spec + 5 * M, spec + 6 * M, g);
   IH_TRY(check_launch(c, "k_lap_spectrum"));
@@ -1012,15 +1113,14 @@ static int output_post(Ctx *c, const Vec &y, const Vec *smry_src) {
   const size_t hsm = sizeof(double) * bins;
   const unsigned gm = grid_for(M, 256, 8);
   IH_TRY((fft_r2c<T>(c, rho, 0, spec + 6 * M, 0, 1)));
-  k_power_spectrum<T><<<gm, 256, hsm, c->stream>>>(spec + 6 * M, g, d + 2 * bins);
+  k_power_spectrum<T><<<gm, 256, hsm, c->stream>>>(spec + 6 * M, g, c->shell, d + 2 * bins);
   IH_TRY(check_launch(c, "k_power_spectrum"));
   double *means = d + 4 * bins + 28;  // [phi_mean, dphi_mean]
   const int nb = nblk_reduce(N);
-  for (int s = 0; s < 2; ++s) {
-    IH_TRY(mean_into<T>(c, yfl + s * N, N, means + s));
-    k_add_scalar<<<1, 1, 0, c->stream>>>(means + s, y.sc + s);
-    IH_TRY(check_launch(c, "k_add_scalar"));
-  }
+  k_partial_sum<T><<<dim3(nb, 2), 256, 0, c->stream>>>(yfl, N, c->partials);
+  IH_TRY(check_launch(c, "k_partial_sum"));
+  k_finish_means<<<2, 256, 0, c->stream>>>(c->partials, nb, N, y.sc, means);
+  IH_TRY(check_launch(c, "k_finish_means"));
   k_constraints<T><<<nb, 256, 0, c->stream>>>(yfl, y.sc, lappsi, rho, c->rs, means, N,
                                               c->partials);
   IH_TRY(check_launch(c, "k_constraints"));
@@ -1028,22 +1128,15 @@ static int output_post(Ctx *c, const Vec &y, const Vec *smry_src) {
   IH_TRY(check_launch(c, "k_constraints_finish"));
   // summaries: phi, dphi, psi, dpsi of the summary source, then rho and p
   const Vec &src = smry_src ? *smry_src : y;
-  IH_CUDA(c, cudaMemcpyAsync(c->hpin, c->rs, sizeof(RhsScalars), cudaMemcpyDeviceToHost,
-                             c->stream));
-  IH_CUDA(c, cudaMemcpyAsync(c->hpin + 32, src.sc, sizeof(double) * kSc,
-                             cudaMemcpyDeviceToHost, c->stream));
-  IH_CUDA(c, cudaStreamSynchronize(c->stream));
-  RhsScalars rs_h;
-  double sc_h[kSc];
-  memcpy(&rs_h, c->hpin, sizeof rs_h);
-  memcpy(sc_h, c->hpin + 32, sizeof sc_h);
-  const T *sfl = (const T *)src.fl;
-  for (int s = 0; s < 4; ++s)
-    IH_TRY(summary<T>(c, sfl + s * N, nullptr, sc_h[s], N, d + 4 * bins + 4 + 4 * s));
-  IH_TRY(summary<T>(c, rho, nullptr, rs_h.rho_bar, N, d + 4 * bins + 4 + 16));
-  IH_TRY(summary<T>(c, (const T *)c->rbuf[1], nullptr, rs_h.p_bar, N, d + 4 * bins + 4 + 20));
+  SmryArgs sa;
+  for (int f = 0; f < 4; ++f) sa.a[f] = (const T *)src.fl + f * N;
+  sa.a[4] = rho;
+  sa.a[5] = c->rbuf[1];
+  sa.sc = src.sc;
+  sa.rs = c->rs;
+  IH_TRY(summaries<T>(c, sa, N, d + 4 * bins + 4));
   if (c->p.enable_gw) {
-    k_gw_spectrum<T><<<gm, 256, hsm, c->stream>>>(yfl, c->rs, g, pow(0.01, 1.0 / 3.0),
+    k_gw_spectrum<T><<<gm, 256, hsm, c->stream>>>(yfl, c->rs, g, c->shell, pow(0.01, 1.0 / 3.0),
                                                  d + 3 * bins);
     IH_TRY(check_launch(c, "k_gw_spectrum"));
   }
