@@ -259,6 +259,153 @@ __device__ __forceinline__ void load_table(V *dst, const V *src, int n, int tid,
 }
 
 // ---------------------------------------------------------------------------
+// The Stockham stages in registers (FP32).  The shared-memory engine was bound
+// by its exchanges: a barrier pair, a round trip through shared memory and index
+// divisions per stage, three or four stages a pass.  Here: value by value the
+// operations of smem_fft and smem_fft_g in their order, so that the results are
+// the same to the bit, but several stages per thread and one exchange in all.  With elements q + st p of a stage of remaining length Lc
+// (p < Lc, st = L / Lc), a radix-r stage takes p = pp + t Lc/r to q + st (r pp +
+// t') with the twiddle w_L^(t' pp st); radix 4 while 4 divides Lc, then 2, then
+// 3.  Step 1: the first stage or the first two, S1 = 4 or 16 values: thread pp
+// over p = pp + i L/S1.  Step 2: the rest, thread q over all p of its S2 = L/S1.
+template <int L> struct StkFac {
+  static constexpr int S1 = L % 16 == 0 && L >= 48 ? 16 : 4, S2 = L / S1;
+};
+template <int L, int B> __host__ __device__ constexpr int stk_threads() {
+  return ((StkFac<L>::S1 > StkFac<L>::S2 ? StkFac<L>::S1 : StkFac<L>::S2) * B + 31) / 32 * 32;
+}
+template <int S1> __device__ __forceinline__ int stk_row(int r) {
+  // row of the exchange buffer: with 64-byte rows, rows S1 apart are written
+  // together and consecutive ones read, so neighbours swap on alternate blocks
+  return r ^ ((r >> (S1 == 16 ? 4 : 2)) & 1);
+}
+template <typename T>
+__device__ __forceinline__ void stk_bfly(C2<T> (&x)[4], int sign) {
+  C2<T> s02 = cadd(x[0], x[2]), d02 = csub(x[0], x[2]);
+  C2<T> s13 = cadd(x[1], x[3]), d13 = csub(x[1], x[3]);
+  C2<T> j13 = mk2<T>(-(T)sign * d13.y, (T)sign * d13.x);
+  x[0] = cadd(s02, s13);
+  x[2] = csub(s02, s13);
+  x[1] = cadd(d02, j13);
+  x[3] = csub(d02, j13);
+}
+template <typename T>
+__device__ __forceinline__ C2<T> stk_mul(C2<T> v, const C2<T> *tw, int i, int sign) {
+  C2<T> w = tw[i];
+  if (sign > 0) w.y = -w.y;
+  return cmul(v, w);
+}
+// step 1 of thread pp = q: v[i] = element q + S2 i -> element S1 q + i
+template <typename T, int L>
+__device__ __forceinline__ void stk_first(C2<T> (&v)[StkFac<L>::S1], const C2<T> *tw, int q,
+                                          int sign) {
+  constexpr int S1 = StkFac<L>::S1, S2 = StkFac<L>::S2;
+  if constexpr (S1 == 4) {
+    stk_bfly<T>(v, sign);
+#pragma unroll
+    for (int r = 1; r < 4; ++r)
+      if (q != 0) v[r] = stk_mul<T>(v[r], tw, r * q, sign);
+  } else {
+    // first stage: pp = q + S2 u over t (v index u + 4 t); second: pp = q over u
+    C2<T> a[4][4];  // [r][u]
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      C2<T> x[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) x[t] = v[u + 4 * t];
+      stk_bfly<T>(x, sign);
+      const int pp = q + S2 * u;
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        a[r][u] = (r == 0 || pp == 0) ? x[r] : stk_mul<T>(x[r], tw, r * pp, sign);
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      stk_bfly<T>(a[r], sign);
+#pragma unroll
+      for (int r2 = 0; r2 < 4; ++r2)
+        v[r + 4 * r2] =
+            (r2 == 0 || q == 0) ? a[r][r2] : stk_mul<T>(a[r][r2], tw, r2 * q * 4, sign);
+    }
+  }
+}
+// the stages from remaining length LC on over the R values of one thread, the
+// element p in v[p] at LC = R; st: the stride of that first stage
+template <typename T, int R, int LC>
+__device__ __forceinline__ void stk_stages(C2<T> (&v)[R], const C2<T> *tw, int st, int sign) {
+  if constexpr (LC > 1) {
+    constexpr int r = LC % 4 == 0 ? 4 : (LC % 2 == 0 ? 2 : 3), m = LC / r;
+    constexpr int ls = R / LC;  // stride among the thread's values
+    C2<T> w[R];
+#pragma unroll
+    for (int pp = 0; pp < m; ++pp) {
+#pragma unroll
+      for (int q = 0; q < ls; ++q) {
+        C2<T> y[4];
+        if constexpr (r == 4) {
+#pragma unroll
+          for (int t = 0; t < 4; ++t) y[t] = v[q + ls * (pp + t * m)];
+          stk_bfly<T>(y, sign);
+        } else if constexpr (r == 2) {
+          const C2<T> a = v[q + ls * pp], c = v[q + ls * (pp + m)];
+          y[0] = cadd(a, c);
+          y[1] = csub(a, c);
+        } else {
+          const T h3 = (T)0.86602540378443864676;
+          const C2<T> x0 = v[q + ls * pp], x1 = v[q + ls * (pp + m)], x2 = v[q + ls * (pp + 2 * m)];
+          const C2<T> s12 = cadd(x1, x2), d12 = csub(x1, x2);
+          const C2<T> tq = mk2<T>(x0.x - (T)0.5 * s12.x, x0.y - (T)0.5 * s12.y);
+          const C2<T> jd = mk2<T>(-(T)sign * h3 * d12.y, (T)sign * h3 * d12.x);
+          y[0] = cadd(x0, s12);
+          y[1] = cadd(tq, jd);
+          y[2] = csub(tq, jd);
+        }
+#pragma unroll
+        for (int t = 0; t < r; ++t)
+          w[q + ls * (r * pp + t)] =
+              (pp == 0 || t == 0) ? y[t] : stk_mul<T>(y[t], tw, t * pp * ls * st, sign);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) v[i] = w[i];
+    stk_stages<T, R, m>(v, tw, st, sign);
+  }
+}
+// B pencils of length L in s[L][P], in place, by at least stk_threads<L, B>
+// threads of one block
+template <typename T, int L, int B>
+__device__ __forceinline__ void smem_stk(C2<T> *s, int P, const C2<T> *tw, int sign, int tid) {
+  constexpr int S1 = StkFac<L>::S1, S2 = StkFac<L>::S2, LB = clog2(B);
+  const int b = tid & (B - 1), q = tid >> LB;
+  C2<T> v[S1];
+  if (q < S2) {
+#pragma unroll
+    for (int i = 0; i < S1; ++i) v[i] = s[(q + S2 * i) * P + b];
+    stk_first<T, L>(v, tw, q, sign);
+  }
+  __syncthreads();
+  if (q < S2) {
+#pragma unroll
+    for (int i = 0; i < S1; ++i) s[(S1 * q + i) * P + b] = v[i];
+  }
+  __syncthreads();
+  if (q < S1) {  // a thread's rows are its own
+    C2<T> u[S2];
+#pragma unroll
+    for (int p = 0; p < S2; ++p) u[p] = s[(q + S1 * p) * P + b];
+    stk_stages<T, S2, S2>(u, tw, S1, sign);
+#pragma unroll
+    for (int i = 0; i < S2; ++i) s[(q + S1 * i) * P + b] = u[i];
+  }
+  __syncthreads();
+}
+// lengths with a factor 3 that the register stages take
+inline bool stk_length3(int L) {
+  return L == 12 || L == 24 || L == 36 || L == 48 || L == 72 || L == 96 || L == 144 || L == 192 ||
+         L == 288 || L == 384;
+}
+
+// ---------------------------------------------------------------------------
 // Complex passes along x (axis 0) or y (axis 1), in place, batched over
 // arrays (blockIdx.z).  A CTA transforms a tile of B pencils: columns
 // z0..z0+B-1 of one plane, element j of a pencil at j * sj.  Two engines,
@@ -295,6 +442,48 @@ __global__ void k_fft_xy_st(C2<T> *data, long long astride, int L, long long sj,
   for (int idx = tid; idx < L * B; idx += nt) {
     const int b = idx & (B - 1), j = idx >> LB;
     if (b < bv) base[(long long)j * sj + b] = s[j * P + b];
+  }
+}
+
+// The Stockham stages in registers (stk_first, stk_stages), half-line tiles (8
+// columns: 64-byte lines, twice the resident CTAs of 16).  Taken for every
+// length that has an instantiation; the shared-memory kernel above keeps the
+// others (2, 4, 6, 18, ...) and FP64.  31 passes of a mixed DOPRI853 step, each
+// the same to the bit: 38.6 -> 27.2 us a pass at 128^3, 9.4 -> 9.3 at 64^3; at
+// 96^3 (64 passes) 26.2 -> 11.8, at 192^3 -> 44.9 us.
+template <typename T, int L, int B>
+__global__ void __launch_bounds__(stk_threads<L, B>()) k_fft_xy_stk(
+    C2<T> *data, long long astride, long long sj, long long so, int mz, int sign,
+    const C2<T> *__restrict__ twg) {
+  constexpr int S1 = StkFac<L>::S1, S2 = StkFac<L>::S2;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  C2<T> *tw = reinterpret_cast<C2<T> *>(smraw);
+  C2<T> *ex = tw + L;  // [L][B]
+  const int tid = threadIdx.x, b = tid & (B - 1), q = tid / B;
+  const int z0 = blockIdx.x * B;
+  const bool col = b < mz - z0;
+  C2<T> *base = data + blockIdx.z * astride + (long long)blockIdx.y * so + z0 + b;
+  load_table(tw, twg, L, tid, (int)blockDim.x);
+  __syncthreads();
+  if (q < S2) {
+    C2<T> v[S1];
+#pragma unroll
+    for (int i = 0; i < S1; ++i)
+      v[i] = col ? base[(long long)(q + S2 * i) * sj] : mk2<T>(0, 0);
+    stk_first<T, L>(v, tw, q, sign);
+#pragma unroll
+    for (int i = 0; i < S1; ++i) ex[stk_row<S1>(S1 * q + i) * B + b] = v[i];
+  }
+  __syncthreads();
+  if (q < S1) {
+    C2<T> u[S2];
+#pragma unroll
+    for (int p = 0; p < S2; ++p) u[p] = ex[stk_row<S1>(q + S1 * p) * B + b];
+    stk_stages<T, S2, S2>(u, tw, S1, sign);
+    if (col) {
+#pragma unroll
+      for (int i = 0; i < S2; ++i) base[(long long)(q + S1 * i) * sj] = u[i];
+    }
   }
 }
 
@@ -827,7 +1016,7 @@ __global__ void __launch_bounds__(32 * zwarps<T>()) k_fft_zc2r(const C2<T> *in, 
 // Two engines, as for the plain passes: Stockham (the phihat tile stays in
 // shared memory for the four variants) and two-step (each step-1 thread keeps
 // its R2 values of phihat in registers for the four variants).
-template <typename T, int B, bool GEN = false>
+template <typename T, int B, bool GEN = false, int LT = 0>
 __global__ void k_fft_x_deriv4_st(const C2<T> *phihat, C2<T> *out, long long ostride, Geom g,
                                    const C2<T> *twg) {
   constexpr int P = B + 1;
@@ -875,7 +1064,9 @@ __global__ void k_fft_x_deriv4_st(const C2<T> *phihat, C2<T> *out, long long ost
                              : mk2<T>(-pre.x * f, -pre.y * f);  // -pre * k^2
     }
     __syncthreads();
-    if constexpr (GEN)
+    if constexpr (LT > 0)
+      smem_stk<T, LT, B>(s, P, tw, +1, tid);
+    else if constexpr (GEN)
       smem_fft_g<T, B, kFftK>(s, L, P, tw, +1, tid, nt);
     else
       smem_fft<T, B, kFftK>(s, L, P, tw, +1, tid, nt);
@@ -1073,10 +1264,11 @@ template <typename T> constexpr size_t zg_smem(int H) {
   return sizeof(C2<T>) * ((size_t)H + 2 * (size_t)H + (size_t)H * (kZB + 1));
 }
 
-template <typename T>
+template <typename T, int HT = 0>
 __global__ void k_fft_zr2c_g(const T *in, long long istride, C2<T> *out, long long ostride,
-                             long long rows, int H, const C2<T> *twhg, const C2<T> *twzg) {
+                             long long rows, int Hrt, const C2<T> *twhg, const C2<T> *twzg) {
   constexpr int P = kZB + 1;
+  const int H = HT > 0 ? HT : Hrt;  // HT: the register stages, H known to the compiler
   extern __shared__ __align__(16) unsigned char smraw[];
   C2<T> *twh = reinterpret_cast<C2<T> *>(smraw);  // exp(-2 pi i k/H)
   C2<T> *twz = twh + H;                           // exp(-2 pi i k/nz)
@@ -1094,7 +1286,10 @@ __global__ void k_fft_zr2c_g(const T *in, long long istride, C2<T> *out, long lo
                               : mk2<T>(0, 0);
   }
   __syncthreads();
-  smem_fft_g<T, kZB, kFftK>(s, H, P, twh, -1, tid, nt);
+  if constexpr (HT > 0)
+    smem_stk<T, HT, kZB>(s, P, twh, -1, tid);
+  else
+    smem_fft_g<T, kZB, kFftK>(s, H, P, twh, -1, tid, nt);
   // X_k = E_k + exp(-2 pi i k/nz) O_k, E = (Z_k + conj Z_(H-k))/2,
   // O = (Z_k - conj Z_(H-k))/(2i), k = 0..H (Z_H = Z_0)
   for (int idx = tid; idx < (H + 1) * kZB; idx += nt) {
@@ -1109,10 +1304,11 @@ __global__ void k_fft_zr2c_g(const T *in, long long istride, C2<T> *out, long lo
   }
 }
 
-template <typename T>
+template <typename T, int HT = 0>
 __global__ void k_fft_zc2r_g(const C2<T> *in, long long istride, T *out, long long ostride,
-                             long long rows, int H, const C2<T> *twhg, const C2<T> *twzg) {
+                             long long rows, int Hrt, const C2<T> *twhg, const C2<T> *twzg) {
   constexpr int P = kZB + 1;
+  const int H = HT > 0 ? HT : Hrt;  // HT: the register stages, H known to the compiler
   extern __shared__ __align__(16) unsigned char smraw[];
   C2<T> *twh = reinterpret_cast<C2<T> *>(smraw);
   C2<T> *twz = twh + H;
@@ -1141,7 +1337,10 @@ __global__ void k_fft_zc2r_g(const C2<T> *in, long long istride, T *out, long lo
     s[k * P + b] = zv;
   }
   __syncthreads();
-  smem_fft_g<T, kZB, kFftK>(s, H, P, twh, +1, tid, nt);
+  if constexpr (HT > 0)
+    smem_stk<T, HT, kZB>(s, P, twh, +1, tid);
+  else
+    smem_fft_g<T, kZB, kFftK>(s, H, P, twh, +1, tid, nt);
   for (int idx = tid; idx < H * kZB; idx += nt) {  // z_j = reals 2j, 2j+1
     const int j = idx % H, b = idx / H;
     const long long r = r0 + b;
@@ -1581,6 +1780,24 @@ static int dispatch_len(int L, F &&f, bool allow512) {
   return IH_ERR_ARG;
 }
 
+// the same for the L of stk_length3
+template <typename F>
+static int dispatch_len3(int L, F &&f) {
+  switch (L) {
+    case 12: return f.template run_reg<12>();
+    case 24: return f.template run_reg<24>();
+    case 36: return f.template run_reg<36>();
+    case 48: return f.template run_reg<48>();
+    case 72: return f.template run_reg<72>();
+    case 96: return f.template run_reg<96>();
+    case 144: return f.template run_reg<144>();
+    case 192: return f.template run_reg<192>();
+    case 288: return f.template run_reg<288>();
+    case 384: return f.template run_reg<384>();
+    default: return IH_ERR_ARG;
+  }
+}
+
 // 512-point passes in both precisions (FP64 ones spill in some forms; the
 // autotuner times them like the rest)
 template <typename T> constexpr bool allow512() { return true; }
@@ -1606,6 +1823,14 @@ struct XYLaunch {
     want_smem(k_fft_xy_st<T, B, GEN>, sm);
     k_fft_xy_st<T, B, GEN><<<grid, threads_st(L, B), sm, c->stream>>>(data, stride, L, sj, so,
                                                                        mzv(), sign, tw);
+    return IH_OK;
+  }
+  template <int L, int B>
+  int run_stk(dim3 grid, long long sj, long long so, const C2<T> *tw) {
+    const size_t sm = sizeof(C2<T>) * ((size_t)L + (size_t)L * B);
+    want_smem(k_fft_xy_stk<T, L, B>, sm);
+    k_fft_xy_stk<T, L, B><<<grid, stk_threads<L, B>(), sm, c->stream>>>(data, stride, sj, so,
+                                                                        mzv(), sign, tw);
     return IH_OK;
   }
   template <int L, int B>
@@ -1653,6 +1878,16 @@ struct XYLaunch {
     return IH_OK;
   }
   template <int L>
+  int run_reg() {
+    constexpr int B = tileB<T>() / 2;
+    const int outer = axis == 0 ? c->g.ny : c->g.nx, mz = mzv();
+    const Geom &g = c->g;
+    return run_stk<L, B>(dim3((mz + B - 1) / B, outer, count),
+                         axis == 0 ? (long long)g.ny * g.mz : g.mz,
+                         axis == 0 ? g.mz : (long long)g.ny * g.mz,
+                         tab<T>(axis == 0 ? c->tw_x : c->tw_y));
+  }
+  template <int L>
   int run() {
     if constexpr (L == 512 && !allow512<T>()) {
       return IH_ERR_ARG;
@@ -1683,6 +1918,10 @@ struct XYLaunch {
           return run_2s<L, B / 2>(grid, sj, so, tw);
         }
       }
+      if constexpr (sizeof(T) == 4 && L >= 8) {
+        constexpr int Bh = B / 2;
+        return run_stk<L, Bh>(dim3((mz + Bh - 1) / Bh, outer, count), sj, so, tw);
+      }
       return run_st<B>(L, grid, sj, so, tw);
     }
   }
@@ -1695,6 +1934,9 @@ int fft_xy(Ctx *c, C2<T> *data, long long stride, int count, int axis, int sign)
   prof_begin(c, KK_FFT_XY);
   if (sizeof(T) == 8 && (c->fx_on >> axis & 1)) {
     IH_TRY(fix_xy(c, data, stride, count, axis, sign, 0));
+  } else if (sizeof(T) == 4 && stk_length3(L)) {
+    if constexpr (sizeof(T) == 4)
+      IH_TRY(dispatch_len3(L, XYLaunch<T>{c, data, stride, count, axis, sign, 0}));
   } else if (L & (L - 1)) {  // 2^a 3^b: the Stockham engine with a radix-3 stage
     constexpr int B = tileB<T>();
     const long long sj = axis == 0 ? (long long)g.ny * g.mz : g.mz;
@@ -1746,6 +1988,39 @@ int fft_gw_yx(Ctx *c, C2<T> *spec, int w) {
   return IH_OK;
 }
 
+// the z passes of rows with a factor 3 on the register stages; 96^3: r2c 25.0 ->
+// 19.0 us, c2r 17.6 -> 13.5 us a pass (the lengths without an instantiation stay
+// with smem_fft_g)
+template <typename T>
+struct Z3Launch {
+  Ctx *c;
+  const void *in;
+  long long istride;
+  void *out;
+  long long ostride;
+  int count;
+  bool forward;
+  template <int H>
+  int run_reg() {
+    const long long rows = (long long)c->g.nx * c->g.ny;
+    const size_t sm = zg_smem<T>(H);
+    const dim3 grid((unsigned)((rows + kZB - 1) / kZB), count);
+    constexpr int nt = stk_threads<H, kZB>();
+    if (forward) {
+      auto kf = k_fft_zr2c_g<T, H>;
+      want_smem(kf, sm);
+      kf<<<grid, nt, sm, c->stream>>>((const T *)in, istride, (C2<T> *)out, ostride, rows, H,
+                                      tab<T>(c->tw_h), tab<T>(c->tw_z));
+    } else {
+      auto kf = k_fft_zc2r_g<T, H>;
+      want_smem(kf, sm);
+      kf<<<grid, nt, sm, c->stream>>>((const C2<T> *)in, istride, (T *)out, ostride, rows, H,
+                                      tab<T>(c->tw_h), tab<T>(c->tw_z));
+    }
+    return IH_OK;
+  }
+};
+
 template <typename T>
 struct ZLaunch {
   Ctx *c;
@@ -1788,6 +2063,9 @@ int fft_zr2c(Ctx *c, const T *in, long long in_stride, C2<T> *out, long long out
     IH_TRY(fix_z(c, in, in_stride, out, out_stride, count, true));
   } else if (fused_wide_ok(c)) {
     IH_TRY(zr2c_wide_launch(c, in, in_stride, out, out_stride, count));
+  } else if (sizeof(T) == 4 && stk_length3(g.h)) {
+    if constexpr (sizeof(T) == 4)
+      IH_TRY(dispatch_len3(g.h, Z3Launch<T>{c, in, in_stride, out, out_stride, count, true}));
   } else if (g.h & (g.h - 1)) {
     const long long rows = (long long)g.nx * g.ny;
     const size_t sm = zg_smem<T>(g.h);
@@ -1809,6 +2087,9 @@ int fft_zc2r(Ctx *c, const C2<T> *in, long long in_stride, T *out, long long out
   prof_begin(c, KK_FFT_ZC2R);
   if (sizeof(T) == 8 && (c->fx_on >> 6 & 1)) {
     IH_TRY(fix_z(c, in, in_stride, out, out_stride, count, false));
+  } else if (sizeof(T) == 4 && stk_length3(g.h)) {
+    if constexpr (sizeof(T) == 4)
+      IH_TRY(dispatch_len3(g.h, Z3Launch<T>{c, in, in_stride, out, out_stride, count, false}));
   } else if (g.h & (g.h - 1)) {
     const long long rows = (long long)g.nx * g.ny;
     const size_t sm = zg_smem<T>(g.h);
@@ -1891,6 +2172,17 @@ struct D4Launch {
     return IH_OK;
   }
   template <int L>
+  int run_reg() {
+    constexpr int B = tileB<T>() / 2;
+    const Geom &g = c->g;
+    dim3 grid((g.mz + B - 1) / B, g.ny, 1);
+    const size_t sm = sizeof(C2<T>) * ((size_t)L + 2 * (size_t)L * (B + 1));
+    auto kf = k_fft_x_deriv4_st<T, B, true, L>;
+    want_smem(kf, sm);
+    kf<<<grid, stk_threads<L, B>(), sm, c->stream>>>(phihat, out, out_stride, g, tab<T>(c->tw_x));
+    return IH_OK;
+  }
+  template <int L>
   int run() {
     if constexpr (L == 512 && !allow512<T>()) {
       return IH_ERR_ARG;
@@ -1899,6 +2191,7 @@ struct D4Launch {
       if (var == FV_PIPELINED) return run_pipe<L, B>();
       if (var == FV_TWOSTEP) return run_2s<L, B>();
       if (var == FV_TWOSTEP_HALF) return run_2s<L, B / 2>();
+      if constexpr (sizeof(T) == 4 && L >= 8) return run_reg<L>();
       return run_st(L);
     }
   }
@@ -1908,7 +2201,10 @@ template <typename T>
 int fft_x_deriv4_inv(Ctx *c, const C2<T> *phihat, C2<T> *out, long long out_stride) {
   const Geom &g = c->g;
   prof_begin(c, KK_X_DERIV4);
-  if (g.nx & (g.nx - 1))
+  if (sizeof(T) == 4 && stk_length3(g.nx)) {
+    if constexpr (sizeof(T) == 4)
+      IH_TRY(dispatch_len3(g.nx, D4Launch<T>{c, phihat, out, out_stride, 0}));
+  } else if (g.nx & (g.nx - 1))
     IH_TRY((D4Launch<T>{c, phihat, out, out_stride, FV_STOCKHAM}.template run_st<true>(g.nx)));
   else
     IH_TRY(dispatch_len(g.nx, D4Launch<T>{c, phihat, out, out_stride, c->d4_var}, allow512<T>()));
