@@ -396,19 +396,28 @@ __global__ void __launch_bounds__(32 * kFxWarps) k_fx_zc2r(
 // their FP64 sums, the six products d_i phi d_j phi and their r2c.  d/dx,
 // d/dy, d/dz stay integers with a shared exponent per row, brought to 2^62;
 // products of two rows are the upper 64 bits and go into the forward transform
-// without a conversion.  rho and p are FP64.  At 256^3: 2.44 ms against 5.90 ms
-// on the FP64 pipe (wide rows); at 128^3 0.181 against 0.915 ms (a warp per
-// row).  It takes about 2500 instructions per complex point and issues on 0.3
-// to 0.4 of the cycles: latency, with the few warps that the three derivative
-// rows leave room for (H = 64: 8 resident warps 221 us, 12 201, 16 181; H = 128
-// is held to 8 by its 96 KB per CTA).  Outputs convert on the integer pipe.
+// without a conversion.  rho and p are FP64.
+//
+// It takes about 2500 instructions per complex point; what bounds it is latency,
+// so the three integer rows are not kept on the chip (96 KB of shared memory per
+// CTA at H = 128, 8 warps an SM issuing on a third of the cycles) but written
+// where the spectra of S_xz, S_yz and S_zz come to lie, each element by the
+// thread that reads it back and at last overwrites it: they stay in the L2 (58 MB
+// in flight), and the CTAs per SM below fit the registers.  At 256^3 2.47 -> 1.53
+// ms (5.90 on the FP64 pipe), 192^3 1.61 -> 0.86, 128^3 0.182 -> 0.170, 96^3
+// 0.115 -> 0.102 ms.  CTAs tried: A = 24 2 / 3: 969 / 855 us; A = 16 3 / 4 / 5:
+// 1704 / 1528 / 1606; A = 12 3 / 4 / 5: 102 / 108 / 115; A = 8 5 / 6 / 8: 170 /
+// 185 / 170 (128^3), 61 / 64 / 74 (64^3).
 template <int H> struct FxZSmem {
   fx2 xs[kFxWarps][FxZG<H>::G * FxZG<H>::X];
-  fx2 grad[kFxWarps][2][FxZG<H>::A][32];  // d/dx, d/dy: thread-private
 };
+template <int H> constexpr int fx_z_ctas() {
+  constexpr int A = FxZG<H>::A;
+  return A == 24 || A == 12 ? 3 : A == 16 ? 4 : A == 8 ? 5 : 6;
+}
 
 template <int H, bool ZSRC>
-__global__ void __launch_bounds__(32 * kFxWarps, H == 64 ? 4 : H < 64 ? 3 : 2) k_fx_z_rhs(
+__global__ void __launch_bounds__(32 * kFxWarps, fx_z_ctas<H>()) k_fx_z_rhs(
     const double2 *d4, long long dstride, const double *__restrict__ yfl, const double *ysc,
     double *lap, double *pout, double *rhoout, double2 *s6, long long sstride, int gw,
     double *partials, Geom g, FxTab twh, FxTab twz, const long long *__restrict__ ckz,
@@ -423,12 +432,15 @@ __global__ void __launch_bounds__(32 * kFxWarps, H == 64 ? 4 : H < 64 ? 3 : 2) k
   const long long row = ((long long)blockIdx.x * kFxWarps + warp) * G::G + grp;
   const bool valid = row < rows;
   fx2 *xch = &sm.xs[warp][grp * G::X];
-  fx2 dz[A];
+  // the thread's own elements of the three integer rows
+  auto grad = [&](int a) {
+    return reinterpret_cast<fx2 *>(s6 + (a == 0 ? 2 : a + 3) * sstride + row * (H + 1)) + t;
+  };
   int ex[3];       // exponents of the three derivative rows
   double post[3];  // their slow factors (1 but for extreme rows)
 #pragma unroll 1
   for (int i = 0; i < 4; ++i) {
-    const int a = (i + 3) & 3;  // the laplacian, then d/dx, d/dy, d/dz
+    const int a = i < 2 ? 3 - i : i - 2;  // the laplacian, d/dz, d/dx, d/dy
     double2 x[A], xH;
     fx2 v[A], vH;
     FxScale sc;
@@ -467,12 +479,10 @@ __global__ void __launch_bounds__(32 * kFxWarps, H == 64 ? 4 : H < 64 ? 3 : 2) k
 #pragma unroll
       for (int m = 0; m < A; ++m) v[m] = fx_shift(v[m], sh);
       e -= room;
-      if (a < 2) {
+      if (valid) {
+        fx2 *gr = grad(a);
 #pragma unroll
-        for (int m = 0; m < A; ++m) sm.grad[warp][a][m][lane] = v[m];
-      } else {
-#pragma unroll
-        for (int m = 0; m < A; ++m) dz[m] = v[m];
+        for (int m = 0; m < A; ++m) gr[B * m] = v[m];
       }
       if (a == 0) { ex[0] = e; post[0] = sc.post; }
       if (a == 1) { ex[1] = e; post[1] = sc.post; }
@@ -483,7 +493,7 @@ __global__ void __launch_bounds__(32 * kFxWarps, H == 64 ? 4 : H < 64 ? 3 : 2) k
   // rho and p; |grad phi|^2 from the integer squares at the largest exponent
   const double a_sc = ysc[4];
   const double inv_a2 = 1.0 / (a_sc * a_sc);
-  const double m2 = g.mass * g.mass, third = 1.0 / 3.0;
+  const double hm2 = 0.5 * (g.mass * g.mass), third = 1.0 / 3.0;
   const long long N = g.N;
   const bool slow = post[0] != 1.0 || post[1] != 1.0 || post[2] != 1.0;
   const int em = max(ex[0], max(ex[1], ex[2]));
@@ -511,17 +521,17 @@ __global__ void __launch_bounds__(32 * kFxWarps, H == 64 ? 4 : H < 64 ? 3 : 2) k
         const int i = E * q + j;
         const long long at = E * t + j + A * q;
         const double2 ph = yp[at], dph = yd[at], ps = ys[at];
-        const fx2 gx = sm.grad[warp][0][i][lane], gy = sm.grad[warp][1][i][lane];
+        const fx2 gx = grad(0)[B * i], gy = grad(1)[B * i], gz = grad(2)[B * i];
         double rx, ry, px, py;
         auto point = [&](double grad, double f, double d, double s, double &rho, double &p) {
-          const double t1 = (0.5 - s) * d * d;
-          const double t2 = (0.5 + s) * grad * inv_a2;
-          const double V = m2 * f * f * 0.5;
-          rho = t1 + t2 + V;
-          p = t1 - t2 * third - V;
+          const double h = 0.5 - s, d2 = d * d, gi = grad * inv_a2;
+          const double u = fma(-h, gi, gi);  // (1/2 + psi) |grad phi|^2 / a^2
+          const double V = hm2 * f * f;
+          rho = fma(h, d2, V) + u;
+          p = fma(-third, u, fma(h, d2, -V));
         };
-        point(grad2(gx.x, gy.x, dz[i].x), ph.x, dph.x, ps.x, rx, px);
-        point(grad2(gx.y, gy.y, dz[i].y), ph.y, dph.y, ps.y, ry, py);
+        point(grad2(gx.x, gy.x, gz.x), ph.x, dph.x, ps.x, rx, px);
+        point(grad2(gx.y, gy.y, gz.y), ph.y, dph.y, ps.y, ry, py);
         po[at] = make_double2(px, py);
         if (rhoout) ro[at] = make_double2(rx, ry);
         dr += rx + ry;
@@ -538,10 +548,10 @@ __global__ void __launch_bounds__(32 * kFxWarps, H == 64 ? 4 : H < 64 ? 3 : 2) k
     const int ia = pr < 3 ? 0 : (pr < 5 ? 1 : 2);
     const int ib = pr < 3 ? pr : (pr < 5 ? pr - 2 : 2);
     fx2 v[A];
+    const fx2 *ga = grad(ia), *gb = grad(ib);
 #pragma unroll
     for (int m = 0; m < A; ++m) {
-      const fx2 a = ia < 2 ? sm.grad[warp][ia][m][lane] : dz[m];
-      const fx2 b = ib < 2 ? sm.grad[warp][ib][m][lane] : dz[m];
+      const fx2 a = valid ? ga[B * m] : fx_mk(0, 0), b = valid ? gb[B * m] : fx_mk(0, 0);
       v[m] = fx_mk(fx_mul(a.x, b.x), fx_mul(a.y, b.y));
     }
     const int ea = ia == 0 ? ex[0] : (ia == 1 ? ex[1] : ex[2]);
