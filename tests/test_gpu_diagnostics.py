@@ -13,9 +13,9 @@ def gpu_mod():
     return gpu
 
 
-@pytest.mark.parametrize("n,L", [((8, 8, 8), (20.0, 20.0, 20.0)), ((12, 8, 18), (9.0, 20.0, 14.0)),
+@pytest.mark.parametrize("n,L", [((8, 8, 8), (20.0, 20.0, 20.0)), ((18, 12, 8), (14.0, 9.0, 20.0)),
                                  ((54, 36, 24), (20.0, 20.0, 20.0)),
-                                 ((16, 8, 128), (20.0, 5.0, 40.0)),
+                                 ((128, 16, 8), (40.0, 20.0, 5.0)),
                                  ((64, 48, 32), (11.0, 20.0, 17.0))])
 @pytest.mark.parametrize("prec", [0, 1])
 def test_every_bin(gpu_mod, oracle_mod, n, L, prec):
