@@ -353,4 +353,18 @@ __device__ __forceinline__ fx2 fx_shift(fx2 v, const FxShift &f) {
   return fx_mk(fx_shift(v.x, f), fx_shift(v.y, f));
 }
 
+// host side: a twiddle table of n entries, and the power of two in n
+inline FxTab fx_tab(const void *p, int n) {
+  FxTab t;
+  t.a = reinterpret_cast<const int4 *>(p);
+  t.b = reinterpret_cast<const int2 *>(t.a + n);
+  return t;
+}
+
+inline int fx_twos(int n) {
+  int s = 0;
+  for (; n % 2 == 0; n /= 2) ++s;
+  return s;
+}
+
 }  // namespace ih

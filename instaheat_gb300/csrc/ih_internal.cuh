@@ -372,7 +372,7 @@ inline bool pencil_length(int L) {
 inline bool zfused_ok(const Ctx *c) { return c->g.pow2 || (c->fx_on >> 6 & 1); }
 inline bool roundtrip_ok(const Ctx *c) { return c->g.pow2 || (c->fx_on & 0x58) == 0x58; }
 
-// the fixed-point passes of the FP64 form (ih_fix.cu)
+// the fixed-point passes of the FP64 form (ih_fix.cu, ih_fixz.cu)
 int fix_tables(Ctx *c);
 int fix_xy(Ctx *c, void *data, long long stride, int count, int axis, int sign, int cols);
 int fix_roundtrip(Ctx *c, const void *z, void *d1, void *d2, int axis);

@@ -1,5 +1,5 @@
 // ih_zrow.cuh -- the z engine of the fixed-point passes of the FP64 form
-// (ih_fix.cu): a row of H = nz/2 complex values (z_j = x_2j + i x_2j+1) on B
+// (ih_fixz.cu): a row of H = nz/2 complex values (z_j = x_2j + i x_2j+1) on B
 // lanes with A values each, H = A B, the structure of the wide-row engine of
 // ih_zwide.cu for other lengths.
 //   spectral side: lane t holds Z[t + B m], m < A;
