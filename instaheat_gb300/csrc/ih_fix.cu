@@ -248,11 +248,6 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 384 /
 
 // ---------------------------------------------------------------------------
 // host side
-static void fx_split(long long v, int &h, int &l) {
-  l = (int)(unsigned)(unsigned long long)v;
-  h = (int)((v - l) >> 32);
-}
-
 // exp(-2 pi i k / L), k < L, as FxTab entries
 static int fx_upload_twiddles(Ctx *c, void **dst, int L) {
   std::vector<int> host(6 * (size_t)L);

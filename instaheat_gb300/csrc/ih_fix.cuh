@@ -260,16 +260,18 @@ __device__ __forceinline__ double fx_out_pipe(long long v, int e) {
 // ... and on the integer pipe (about 3.5 per clock and SM): the mantissa, its
 // leading one put in, shifted to the pencil's exponent, and back by a count of
 // leading zeros; both round to nearest
-__device__ __forceinline__ long long fx_in_bits(double a, const FxScale &s) {
+__device__ __forceinline__ long long fx_in_shift(double a, int r) {
   const unsigned hi = (unsigned)__double2hiint(a), lo = (unsigned)__double2loint(a);
   // a = m 2^(e - 1075) with m < 2^53; m 2^10 is below 2^63 and goes right by
   // r > 0 bits, one of them in the rounding
-  const int e = (int)((hi >> 20) & 0x7ff);
   unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 10;
   // (shr clamps: a count of 64 or more, as for zeros, gives 0)
-  asm("shr.u64 %0, %0, %1;" : "+l"(m) : "r"(1084 - s.in - e));
+  asm("shr.u64 %0, %0, %1;" : "+l"(m) : "r"(r));
   const long long t = (long long)((m + 1) >> 1);
   return (int)hi < 0 ? -t : t;
+}
+__device__ __forceinline__ long long fx_in_bits(double a, const FxScale &s) {
+  return fx_in_shift(a, 1084 - s.in - (int)(((unsigned)__double2hiint(a) >> 20) & 0x7ff));
 }
 __device__ __forceinline__ double fx_out_bits(long long v, int e) {
   const unsigned long long u = (unsigned long long)(v < 0 ? -v : v);
@@ -353,6 +355,35 @@ __device__ __forceinline__ fx2 fx_shift(fx2 v, const FxShift &f) {
   return fx_mk(fx_shift(v.x, f), fx_shift(v.y, f));
 }
 
+// ---------------------------------------------------------------------------
+// Sums sum_j c_j x_j of a few FP64 numbers per element, off the FP64 pipe:
+// c_j = C_j 2^(k_j - 62) with |C_j| <= 2^62, the x_j 2^(k_j) as integers at the
+// exponent of the largest of them (2^61), the upper halves of the products added
+// up.  With n <= 15 terms the sum stays below 2^63, and its error is at most a
+// unit per term, 2^-57 of the largest product: below that of an FP64 sum, whose
+// terms each round to 2^-53 of a partial sum.
+struct FxCoef {
+  int h, l, k;
+};
+__device__ __forceinline__ long long fx_mul(int ah, int al, FxCoef c) {
+  return fx_mul(ah, al, c.h, c.l);
+}
+__device__ __forceinline__ int fx_exponent(double x, int k) {  // biased, of x 2^k
+  return ((__double2hiint(x) >> 20) & 0x7ff) + k;
+}
+struct FxPoint {
+  bool fast;  // every x_j finite, the sums' exponents in range (k_j within 64)
+  int in;     // integer = x_j 2^(k_j + in)
+  __device__ __forceinline__ explicit FxPoint(int E) {  // the largest fx_exponent
+    fast = E >= 200 && E <= 1900;
+    in = 61 + 1022 - E;
+  }
+  __device__ __forceinline__ long long get(double x, int e) const {
+    return fx_in_shift(x, 1084 - in - e);
+  }
+  __device__ __forceinline__ double put(long long v) const { return fx_out_bits(v, 2 - in); }
+};
+
 // host side: a twiddle table of n entries, and the power of two in n
 inline FxTab fx_tab(const void *p, int n) {
   FxTab t;
@@ -365,6 +396,24 @@ inline int fx_twos(int n) {
   int s = 0;
   for (; n % 2 == 0; n /= 2) ++s;
   return s;
+}
+inline void fx_split(long long v, int &h, int &l) {
+  l = (int)(unsigned)(unsigned long long)v;
+  h = (int)((v - l) >> 32);
+}
+// the exponent of a coefficient, kFxNone for one that FxPoint does not take
+// (zero, or outside 2^-64 .. 2^64); c as a fraction of 2^k
+constexpr int kFxNone = 1 << 20;
+inline int fx_coef_exp(double c) {
+  int e = 0;
+  const double m = frexp(c, &e);
+  return fabs(m) >= 0.5 && fabs(m) < 1.0 && e >= -64 && e <= 64 ? e : kFxNone;
+}
+inline FxCoef fx_coef(double c, int k) {
+  FxCoef f;
+  fx_split(llrint(ldexp(c, 62 - k)), f.h, f.l);
+  f.k = k;
+  return f;
 }
 
 }  // namespace ih

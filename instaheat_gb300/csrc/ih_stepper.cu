@@ -17,6 +17,7 @@
 #include <string.h>
 #include <mutex>
 #include "ih_internal.cuh"
+#include "ih_fix.cuh"
 
 namespace ih {
 
@@ -221,6 +222,8 @@ struct LinArgs {
   int n;
   double scale;            // out = base + scale * sum coef_j in_j
   const double *scale_dev;  // if set, the scale is read from device memory
+  FxCoef fx[kMaxTerms];     // FP64: the coefficients as fractions
+  int fxn;                  // how many of them FxPoint takes
 };
 
 template <typename T> struct Vec4;
@@ -256,9 +259,12 @@ __device__ __forceinline__ void vstore(T *p, const T *v) {
 // the number of terms.  A term behind a run-time test (12 of them, whatever
 // the stage) still takes its issue slot when the test is a predicate, and in
 // FP64 the slots are what there is: 143 DFMA slots per element over the 11
-// stages of a step against 61 with the count known.  FP64 256^3, the 11
-// combinations of a step: 15.9 ms against 35.7, 4.9 TB/s (bound by the FP64
-// pipe, 13 ms of DFMA, and HBM, 11.6 ms, together).
+// stages of a step against 61 with the count known.  From three terms on the
+// DFMAs take longer than HBM, so FP64 elements are summed in integers (FxPoint;
+// the FP64 sum stays for values that it does not take).  FP64 256^3, the 11
+// combinations of a step: 35.7 ms, 15.9 with the count known (4.9 TB/s), 14.2
+// with every other element in integers, 12.2 with all (6.4 TB/s, HBM).
+template <typename T> constexpr int kFxTerms = sizeof(T) == 8 ? 3 : 1 << 20;
 template <typename T, int NT>
 __global__ void __launch_bounds__(256) k_lincomb(const T *__restrict__ base, const double *basesc,
                                                  T *__restrict__ out, double *outsc, LinArgs args,
@@ -277,14 +283,31 @@ __global__ void __launch_bounds__(256) k_lincomb(const T *__restrict__ base, con
     for (int j = 0; j < NT; ++j) vload<T>((const T *)args.in[j] + v * W, x[j]);
     vload<T>(base + v * W, x[NT]);
 #pragma unroll
-    for (int w = 0; w < W; ++w) acc[w] = 0;
+    for (int w = 0; w < W; ++w) {
+      acc[w] = 0;
+      if constexpr (NT >= kFxTerms<T>) {
+        int e[NT], em = 0;
 #pragma unroll
-    for (int j = 0; j < NT; ++j) {
+        for (int j = 0; j < NT; ++j) {
+          e[j] = fx_exponent(x[j][w], args.fx[j].k);
+          em = max(em, e[j]);
+        }
+        const FxPoint pt(em);
+        if (pt.fast && args.fxn == NT) {
+          long long s = 0;
 #pragma unroll
-      for (int w = 0; w < W; ++w) acc[w] += cf[j] * x[j][w];
+          for (int j = 0; j < NT; ++j) {
+            const long long xi = pt.get(x[j][w], e[j]);
+            s += fx_mul(fx_hi(xi), (int)xi, args.fx[j]);
+          }
+          acc[w] = x[NT][w] + sc * pt.put(s);
+          continue;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < NT; ++j) acc[w] += cf[j] * x[j][w];
+      acc[w] = x[NT][w] + sc * acc[w];
     }
-#pragma unroll
-    for (int w = 0; w < W; ++w) acc[w] = x[NT][w] + sc * acc[w];
     vstore<T>(out + v * W, acc);
   }
   if (blockIdx.x == 0 && threadIdx.x < 5) {
@@ -306,11 +329,27 @@ struct FinalArgs {
   double rtol, atol;
   double noise;               // eta * eps32 (mixed form), 0 for FP64
   long long next;             // Next (tensor segment length)
+  FxCoef fb[8], fe3[8], fbhh[3];  // FP64: b, e3 and bhh as fractions, one exponent a stage
   double *diag;               // per-segment sums [phi, dphi, psi, dpsi, h, dh] x (e5, e3), or null
 };
 
+// 1 / x with three FP64 operations: an FP32 reciprocal of the upper 20 bits of
+// the mantissa (relative error e below 2^-19) and one third-order step of
+// Householder's iteration, y (1 + e + e^2), e = 1 - x y: 2^-57 before its
+// rounding.  Outside of FP32's normal range the division.
+__device__ __forceinline__ double recip(double x) {
+  constexpr int kBias = 896 << 20;  // between the exponents of the two formats
+  const int h = __double2hiint(x);
+  if (h < kBias + (2 << 20) || h > kBias + (252 << 20)) return 1.0 / x;
+  const int r = __float_as_int(__fdividef(1.0f, __int_as_float((h - kBias) << 3)));
+  const double y = __hiloint2double((r >> 3) + kBias, r << 29);
+  const double e = fma(-x, y, 1.0);
+  return fma(fma(e, e, e), y, y);
+}
+
 // The final combination and both embedded error sums in one pass
-// (dopri853.c:436-458, error() 469-486).  The FP64 homogeneous parts of the
+// (dopri853.c:436-458, error() 469-486).  FP64: the three sums in integers as in
+// k_lincomb, 256^3 7.78 -> 3.14 ms.  The FP64 homogeneous parts of the
 // three combinations are formed once per CTA in shared memory; per element
 // the work is FP32 (mixed form, rounding floor removed) or FP64, and the
 // squared ratios are accumulated in FP64 per thread.
@@ -377,11 +416,34 @@ __global__ void __launch_bounds__(256) k_dopri_final(const T *__restrict__ y, co
 #pragma unroll
     for (int j = 0; j < 8; ++j) vload<T>((const T *)a.k[j] + v * W, x[j]);
 #pragma unroll
-    for (int w = 0; w < W; ++w) ab[w] = a5[w] = a3[w] = t5[w] = t3[w] = 0;
+    for (int w = 0; w < W; ++w) {
+      ab[w] = a5[w] = a3[w] = t5[w] = t3[w] = 0;
+      if constexpr (sizeof(T) == 8) {
+        int e[8], em = 0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < 8; ++j) {
+          e[j] = fx_exponent(x[j][w], a.fb[j].k);
+          em = max(em, e[j]);
+        }
+        const FxPoint pt(em);
+        if (pt.fast) {
+          long long sb = 0, s3 = 0, sh = 0;
 #pragma unroll
-      for (int w = 0; w < W; ++w) {
+          for (int j = 0; j < 8; ++j) {
+            const long long xi = pt.get(x[j][w], e[j]);
+            const int xh = fx_hi(xi), xl = (int)xi;
+            sb += fx_mul(xh, xl, a.fb[j]);
+            s3 += fx_mul(xh, xl, a.fe3[j]);
+            if (j == 0 || j == 4 || j == 7) sh += fx_mul(xh, xl, a.fbhh[j == 0 ? 0 : j == 4 ? 1 : 2]);
+          }
+          ab[w] = pt.put(sb);
+          a5[w] = pt.put(sb - sh);
+          a3[w] = pt.put(s3);
+          continue;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
         ab[w] += cb[j] * x[j][w];
         a3[w] += c3[j] * x[j][w];
         if constexpr (sizeof(T) == 4) {
@@ -390,12 +452,9 @@ __global__ void __launch_bounds__(256) k_dopri_final(const T *__restrict__ y, co
           t3[w] += fabsf(c3[j] * x[j][w]);
         }
       }
-    }
-    if constexpr (sizeof(T) == 8) {
       // the 3rd-order difference as the reference forms it (dopri853.c:451),
       // three terms off the 8th-order sum instead of eight of its own
-#pragma unroll
-      for (int w = 0; w < W; ++w)
+      if constexpr (sizeof(T) == 8)
         a5[w] = ab[w] - a.bhh[0] * x[0][w] - a.bhh[1] * x[4][w] - a.bhh[2] * x[7][w];
     }
     T yv[W], yn[W];
@@ -429,15 +488,15 @@ __global__ void __launch_bounds__(256) k_dopri_final(const T *__restrict__ y, co
       acc3d = (double)acc3;
     } else {
       // the homogeneous parts of the plain form are 0; one reciprocal for both
-      // ratios; |y| compared as bits, off the FP64 pipe, which bounds this
-      // kernel (256^3: 8.2 ms against 12.3 with the sums and divisions apart)
+      // ratios; |y| compared as bits, off the FP64 pipe, which has the rest: 9 operations an element with recip, 17 with a division
+      // (256^3: 8.24 and 7.78 ms with the sums on the FP64 pipe)
       acc5d = 0.0;
       acc3d = 0.0;
 #pragma unroll
       for (int w = 0; w < W; ++w) {
         const long long m = max(__double_as_longlong(fabs((double)yv[w])),
                                 __double_as_longlong(fabs((double)yn[w])));
-        const double isk = 1.0 / (a.atol + a.rtol * __longlong_as_double(m));
+        const double isk = recip(a.atol + a.rtol * __longlong_as_double(m));
         const double r5 = (double)a5[w] * isk, r3 = (double)a3[w] * isk;
         acc5d += r5 * r5;
         acc3d += r3 * r3;
@@ -866,8 +925,17 @@ static int lincomb(Ctx *c, const Vec &base, Vec &out, const LinArgs &args) {
   prof_begin(c, KK_LINCOMB);
   if (c->mixed)
     lincomb_launch<float, kMaxTerms>(c, base, out, args);
-  else
-    lincomb_launch<double, kMaxTerms>(c, base, out, args);
+  else {
+    LinArgs a = args;
+    a.fxn = 0;
+    for (int j = 0; j < a.n; ++j) {
+      const int k = fx_coef_exp(a.coef[j]);
+      if (k == kFxNone) continue;
+      a.fx[j] = fx_coef(a.coef[j], k);
+      ++a.fxn;
+    }
+    lincomb_launch<double, kMaxTerms>(c, base, out, a);
+  }
   prof_end(c, KK_LINCOMB, (double)(args.n + 2) * c->g.Nf * c->tsize);
   return check_launch(c, "k_lincomb");
 }
@@ -1201,6 +1269,16 @@ static int try_body(Ctx *c) {
     f.e3[j] = DE3[sidx];
   }
   for (int i = 0; i < 3; ++i) f.bhh[i] = DBHH[i];
+  for (int j = 0; j < 8; ++j) {
+    const int i = j == 0 ? 0 : (j == 4 ? 1 : 2);
+    const bool hh = j == 0 || j == 4 || j == 7;
+    int k = fx_coef_exp(f.b[j]);
+    if (fx_coef_exp(f.e3[j]) > k) k = fx_coef_exp(f.e3[j]);
+    if (hh && fx_coef_exp(f.bhh[i]) > k) k = fx_coef_exp(f.bhh[i]);
+    f.fb[j] = fx_coef(f.b[j], k);
+    f.fe3[j] = fx_coef(f.e3[j], k);
+    if (hh) f.fbhh[i] = fx_coef(f.bhh[i], k);
+  }
   f.dt = c->dt_dev;
   f.rtol = c->cfg.rtol;
   f.atol = c->cfg.atol;
