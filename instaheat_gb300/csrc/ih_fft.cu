@@ -2032,7 +2032,7 @@ struct ZLaunch {
   bool forward;
   template <int H>
   int run() {
-    if constexpr (H > 256) {
+    if constexpr (H > 256 || (sizeof(T) == 4 && H <= 64)) {  // (FP32: ih_zreg.cu)
       return IH_ERR_ARG;
     } else {
       constexpr int RB = zrows<T, H>();
@@ -2063,6 +2063,8 @@ int fft_zr2c(Ctx *c, const T *in, long long in_stride, C2<T> *out, long long out
     IH_TRY(fix_z(c, in, in_stride, out, out_stride, count, true));
   } else if (fused_wide_ok(c)) {
     IH_TRY(zr2c_wide_launch(c, in, in_stride, out, out_stride, count));
+  } else if (zreg_ok(c)) {
+    IH_TRY(zreg_pass(c, in, in_stride, out, out_stride, count, true));
   } else if (sizeof(T) == 4 && stk_length3(g.h)) {
     if constexpr (sizeof(T) == 4)
       IH_TRY(dispatch_len3(g.h, Z3Launch<T>{c, in, in_stride, out, out_stride, count, true}));
@@ -2087,6 +2089,8 @@ int fft_zc2r(Ctx *c, const C2<T> *in, long long in_stride, T *out, long long out
   prof_begin(c, KK_FFT_ZC2R);
   if (sizeof(T) == 8 && (c->fx_on >> 6 & 1)) {
     IH_TRY(fix_z(c, in, in_stride, out, out_stride, count, false));
+  } else if (zreg_ok(c)) {
+    IH_TRY(zreg_pass(c, in, in_stride, out, out_stride, count, false));
   } else if (sizeof(T) == 4 && stk_length3(g.h)) {
     if constexpr (sizeof(T) == 4)
       IH_TRY(dispatch_len3(g.h, Z3Launch<T>{c, in, in_stride, out, out_stride, count, false}));
@@ -2341,7 +2345,7 @@ struct FusedLaunch {
   }
   template <int H>
   int run() {
-    if constexpr (H > 256) {
+    if constexpr (H > 256 || (sizeof(T) == 4 && H <= 64)) {  // (FP32: ih_zreg.cu)
       return IH_ERR_ARG;
     } else {
       constexpr int RB = zrows<T, H>();
@@ -2380,9 +2384,12 @@ int fft_z_rhs_fused(Ctx *c, const C2<T> *d4, const T *yfl, const double *ysc, T 
       c->err = "plane-major tensor sources need the wide-row z pass";
       return IH_ERR_STATE;
     }
-    IH_TRY(dispatch_len(
-        g.h, FusedLaunch<T>{c, d4, yfl, ysc, lap, p, rho, s6, gw, partials, zsrc},
-        false));
+    if (zreg_ok(c))
+      IH_TRY(zreg_rhs(c, d4, yfl, ysc, lap, p, rho, s6, gw, partials, zsrc));
+    else
+      IH_TRY(dispatch_len(
+          g.h, FusedLaunch<T>{c, d4, yfl, ysc, lap, p, rho, s6, gw, partials, zsrc},
+          false));
   }
   prof_end(c, KK_Z_RHS_FUSED,
            (double)(4 + (gw ? 6 : 0)) * g.M * sizeof(C2<T>) +

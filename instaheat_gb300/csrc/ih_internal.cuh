@@ -367,6 +367,13 @@ inline bool pencil_length(int L) {
     default: return false;
   }
 }
+// the z passes of the mixed form for power-of-two rows of up to 128 reals, in
+// registers (ih_zreg.cu); the same to the bit as the warp-row engine of ih_fft.cu
+bool zreg_ok(const Ctx *c);
+int zreg_pass(Ctx *c, const void *in, long long istride, void *out, long long ostride, int count,
+              bool forward);
+int zreg_rhs(Ctx *c, const void *d4, const void *yfl, const double *ysc, void *lap, void *p,
+             void *rho, void *s6, int gw, double *partials, int zsrc);
 // whether the z pass of the RHS is one fused kernel, and whether the x and y
 // round trips exist (else the full-spectrum route)
 inline bool zfused_ok(const Ctx *c) { return c->g.pow2 || (c->fx_on >> 6 & 1); }
