@@ -314,7 +314,9 @@ struct FxZOut {
 // ms (5.90 on the FP64 pipe), 192^3 1.61 -> 0.86, 128^3 0.182 -> 0.170, 96^3
 // 0.115 -> 0.102 ms.  CTAs tried: A = 24 2 / 3: 969 / 855 us; A = 16 3 / 4 / 5:
 // 1704 / 1528 / 1606; A = 12 3 / 4 / 5: 102 / 108 / 115; A = 8 5 / 6 / 8: 170 /
-// 185 / 170 (128^3).
+// 185 / 170 (128^3).  The points two at a time in a loop instead of unrolled: 1.58 ->
+// 1.39 ms at 256^3, 895 -> 827 us at 192^3, 172 -> 169 at 128^3 (the unrolled kernel
+// waited for instructions).
 template <int H> constexpr int fx_z_ctas() {
   constexpr int A = FxZG<H>::A;
   return A == 24 || A == 12 ? 3 : A == 16 ? 4 : A == 8 ? 5 : 6;
@@ -363,8 +365,8 @@ __global__ void __launch_bounds__(32 * kFxWarps, fx_z_ctas<H>()) k_fx_z_rhs(
   pt.init(ysc[4], mass);
   double dr = 0.0, dp = 0.0;
   if (ln.valid) {
-#pragma unroll
-    for (int i = 0; i < A; ++i)
+#pragma unroll 2
+    for (int i = 0; i < A; ++i)  // (unrolled, the kernel waits for instructions)
       out.point<H>(pt, ln, i, grad(0)[B * i], grad(1)[B * i], grad(2)[B * i], dr, dp);
   }
   rhs_partial<32 * kFxWarps>(dr, dp, partials);
