@@ -183,45 +183,45 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 384 /
   const int room = fx_room(mu, fx_p<L>() + 2);
   const FxShift sh = fx_shift_of(room);
   // the spectrum waits in the thread's own slots of ex1 between the two
-  // inverse transforms (in registers it would halve the resident CTAs)
+  // inverse transforms (in registers it would halve the resident CTAs).  From 16
+  // points a thread on the two share their code: unrolled, the kernel waited for
+  // instructions more than for anything else (128^3 57.3 -> 53.3 us, 96^3
+  // 33.0 -> 31.6, 256^3 351 -> 344; 64^3 the other way, 13.5 -> 14.3).
+  constexpr int kShare = R1 >= 16 || R2 >= 16 || R1 % 3 == 0 ? 1 : 2;
   auto slot = [&](int k1) { return (k1 * R2 + q) * B + b; };
-  fx2 w[R1];
   if (q < R2) {
 #pragma unroll
-    for (int k1 = 0; k1 < R1; ++k1) {
-      const fx2 v = fx_shift(u[k1], sh);
-      ex1[slot(k1)] = v;
-      const long long c = __ldg(c1 + q + R2 * k1);
-      const int ch = fx_hi(c), cl = (int)c;
-      w[k1] = fx_mk(-fx_mul(v.y, ch, cl), fx_mul(v.x, ch, cl));  // i k X
-    }
-    fx_dft<R1, +1>(w);
-#pragma unroll
-    for (int n1 = 0; n1 < R1; ++n1)
-      ex0[fx_row<L, B>(q * R1 + n1) * B + b] =
-          n1 == 0 ? fx_quarter(w[n1]) : fx_cmul<+1>(w[n1], fx_tw(tw, n1 * q));
-    const long long z2 = ACC ? __ldg(cz + min(z0 + b, mz - 1)) : 0;
-#pragma unroll
-    for (int k1 = 0; k1 < R1; ++k1) {
-      const fx2 v = ex1[slot(k1)];
-      const long long c = __ldg(c2 + q + R2 * k1) + z2;
-      const int ch = fx_hi(c), cl = (int)c;
-      w[k1] = fx_mk(fx_mul(v.x, ch, cl), fx_mul(v.y, ch, cl));  // -k^2 X
-    }
-    fx_dft<R1, +1>(w);
+    for (int k1 = 0; k1 < R1; ++k1) ex1[slot(k1)] = fx_shift(u[k1], sh);
   }
-  __syncthreads();  // every slot of ex1 is read
-  if (q < R2) {
+#pragma unroll kShare
+  for (int o = 0; o < 2; ++o) {
+    if (q < R2) {
+      const long long *cc = o ? c2 : c1;
+      const long long z2 = ACC && o ? __ldg(cz + min(z0 + b, mz - 1)) : 0;
 #pragma unroll
-    for (int n1 = 0; n1 < R1; ++n1)
-      ex1[fx_row<L, B>(q * R1 + n1) * B + b] =
-          n1 == 0 ? fx_quarter(w[n1]) : fx_cmul<+1>(w[n1], fx_tw(tw, n1 * q));
+      for (int k1 = 0; k1 < R1; ++k1) {
+        const fx2 v = ex1[slot(k1)];
+        const long long c = __ldg(cc + q + R2 * k1) + z2;
+        const int ch = fx_hi(c), cl = (int)c;
+        const long long cx = fx_mul(v.x, ch, cl), cy = fx_mul(v.y, ch, cl);
+        u[k1] = o ? fx_mk(cx, cy) : fx_mk(-cy, cx);  // -k^2 X, i k X
+      }
+      fx_dft<R1, +1>(u);
+    }
+    if (o) __syncthreads();  // every slot of ex1 is read
+    fx2 *ex = o ? ex1 : ex0;
+    if (q < R2) {
+#pragma unroll
+      for (int n1 = 0; n1 < R1; ++n1)
+        ex[fx_row<L, B>(q * R1 + n1) * B + b] =
+            n1 == 0 ? fx_quarter(u[n1]) : fx_cmul<+1>(u[n1], fx_tw(tw, n1 * q));
+    }
   }
   __syncthreads();
   if (q < R1) {
     // forward twiddle, coefficient and inverse twiddle took 2 bits each
     const int e = sc.out + 6 - room;
-#pragma unroll
+#pragma unroll kShare
     for (int o = 0; o < 2; ++o) {
       const fx2 *ex = o ? ex1 : ex0;
       fx2 v[R2];
