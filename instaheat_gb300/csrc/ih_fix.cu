@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 512 /
 // in Q62 (first derivative 0 on the Nyquist index).  ACC (the y round trip):
 // the coefficient of d2 takes -kz^2 too (cz, at the scale of c2), so that d2
 // is the y and z part of the laplacian, and the x part in out1 is added.
-// At 256^3: 347 us a round trip against 1359 us on the FP64 pipe, 128^3 58 us
+// At 256^3: 344 us a round trip against 1359 us on the FP64 pipe, 128^3 53 us
 // against 178.  Inputs convert on the FP64 pipe, outputs (two per input) on the
 // integer pipe: 375 us with both on the former, 388 on the latter.
 // Between the transforms the spectrum is brought to 2 bits above the inverse

@@ -362,9 +362,7 @@ __device__ __forceinline__ fx2 fx_shift(fx2 v, const FxShift &f) {
 // up.  With n <= 15 terms the sum stays below 2^63, and its error is at most a
 // unit per term, 2^-57 of the largest product: below that of an FP64 sum, whose
 // terms each round to 2^-53 of a partial sum.
-struct FxCoef {
-  int h, l, k;
-};
+constexpr int kFxSum = 3;  // terms from which FP64 sums of vectors are summed so
 __device__ __forceinline__ long long fx_mul(int ah, int al, FxCoef c) {
   return fx_mul(ah, al, c.h, c.l);
 }
@@ -381,7 +379,10 @@ struct FxPoint {
   __device__ __forceinline__ long long get(double x, int e) const {
     return fx_in_shift(x, 1084 - in - e);
   }
-  __device__ __forceinline__ double put(long long v) const { return fx_out_bits(v, 2 - in); }
+  // (k: of coefficients that share one exponent, which get() then leaves out)
+  __device__ __forceinline__ double put(long long v, int k = 0) const {
+    return fx_out_bits(v, 2 + k - in);
+  }
 };
 
 // host side: a twiddle table of n entries, and the power of two in n

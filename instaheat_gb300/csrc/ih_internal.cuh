@@ -78,6 +78,11 @@ struct Vec {                    // one state-shaped vector
   double *sc = nullptr;         // double[kSc] (device)
 };
 
+// an FP64 coefficient as a fraction of 2^k, split (ih_fix.cuh)
+struct FxCoef {
+  int h, l, k;
+};
+
 // Terms of a DOPRI853/RK4 stage combination (dopri853.c:340-436).
 constexpr int kMaxTerms = 12;
 // The next stage's input formed by the kernels that write the stage being
@@ -93,6 +98,10 @@ struct NextLin {
   int n;
   double self;                    // the coefficient of k_s (0: none)
   float selff;
+  // FP64: the coefficients for sums in integers as in k_lincomb (FxPoint); fxn:
+  // the number of terms if they are summed so, else 0
+  FxCoef fx[kMaxTerms], fxself;
+  int fxn;
   const void *base;               // the step's start state (T[Nf])
   const double *basesc;
   const double *dt;               // the step size (device memory)

@@ -291,24 +291,31 @@ __global__ void k_update_phi_psi(T *y, const double *ysc, const T *__restrict__ 
       for (int seg = 0; seg < 4; ++seg) {
         const T *o = seg == 0 ? dph : seg == 1 ? o1 : seg == 2 ? dps : o3;
         const long long e = seg * N + i0;
-        T acc[W], x[W];
+        T x[W];
+        if constexpr (sizeof(T) == 8) {
+          const double2 r = nl_sum2(nl, dt, e, make_double2(o[0], o[1]));
+          x[0] = r.x;
+          x[1] = r.y;
+        } else {
+          T acc[W];
 #pragma unroll
-        for (int w = 0; w < W; ++w) acc[w] = 0;
+          for (int w = 0; w < W; ++w) acc[w] = 0;
 #pragma unroll
-        for (int j = 0; j < kMaxTerms; ++j) {
-          if (j < nl.n) {
-            ld_w<T>(reinterpret_cast<const T *>(nl.k[j]) + e, x);
-            const T cj = nl_coef<T>(nl, j);
+          for (int j = 0; j < kMaxTerms; ++j) {
+            if (j < nl.n) {
+              ld_w<T>(reinterpret_cast<const T *>(nl.k[j]) + e, x);
+              const T cj = nl_coef<T>(nl, j);
 #pragma unroll
-            for (int w = 0; w < W; ++w) acc[w] += cj * x[w];
+              for (int w = 0; w < W; ++w) acc[w] += cj * x[w];
+            }
           }
+          const T cs = nl_self<T>(nl);
+#pragma unroll
+          for (int w = 0; w < W; ++w) acc[w] += cs * o[w];
+          ld_w<T>(reinterpret_cast<const T *>(nl.base) + e, x);
+#pragma unroll
+          for (int w = 0; w < W; ++w) x[w] = x[w] + dt * acc[w];
         }
-        const T cs = nl_self<T>(nl);
-#pragma unroll
-        for (int w = 0; w < W; ++w) acc[w] += cs * o[w];
-        ld_w<T>(reinterpret_cast<const T *>(nl.base) + e, x);
-#pragma unroll
-        for (int w = 0; w < W; ++w) x[w] = x[w] + dt * acc[w];
         st_w<T>(y + e, x);
       }
     }

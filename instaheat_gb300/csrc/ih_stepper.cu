@@ -264,7 +264,7 @@ __device__ __forceinline__ void vstore(T *p, const T *v) {
 // the FP64 sum stays for values that it does not take).  FP64 256^3, the 11
 // combinations of a step: 35.7 ms, 15.9 with the count known (4.9 TB/s), 14.2
 // with every other element in integers, 12.2 with all (6.4 TB/s, HBM).
-template <typename T> constexpr int kFxTerms = sizeof(T) == 8 ? 3 : 1 << 20;
+template <typename T> constexpr int kFxTerms = sizeof(T) == 8 ? kFxSum : 1 << 20;
 template <typename T, int NT>
 __global__ void __launch_bounds__(256) k_lincomb(const T *__restrict__ base, const double *basesc,
                                                  T *__restrict__ out, double *outsc, LinArgs args,
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(256) k_lincomb(const T *__restrict__ base, con
             const long long xi = pt.get(x[j][w], e[j]);
             s += fx_mul(fx_hi(xi), (int)xi, args.fx[j]);
           }
-          acc[w] = x[NT][w] + sc * pt.put(s);
+          acc[w] = fma(sc, (T)pt.put(s), x[NT][w]);
           continue;
         }
       }
@@ -1214,6 +1214,18 @@ static void stage_terms(Ctx *c, int s, bool self, LinArgs *a, NextLin *nl) {
     nl->n = n;
     nl->self = DA[s][s - 1];
     nl->selff = (float)DA[s][s - 1];
+    const bool with = nl->self != 0.0;
+    nl->fxn = n + (with ? 1 : 0);
+    for (int j = 0; j < n + (with ? 1 : 0); ++j) {
+      const double cj = j < n ? nl->coef[j] : nl->self;
+      const int k = fx_coef_exp(cj);
+      if (k == kFxNone) {
+        nl->fxn = 0;
+        break;
+      }
+      (j < n ? nl->fx[j] : nl->fxself) = fx_coef(cj, k);
+    }
+    if (nl->fxn < kFxSum) nl->fxn = 0;
     nl->base = c->y.fl;
     nl->basesc = c->y.sc;
     nl->dt = c->dt_dev;

@@ -4,6 +4,7 @@
 // update_h kernel and the x pass that fuses it.
 #pragma once
 #include "ih_internal.cuh"
+#include "ih_fix.cuh"
 
 namespace ih {
 
@@ -182,27 +183,81 @@ __device__ __forceinline__ T nl_self(const NextLin &nl) {
     return nl.self;
   }
 }
+// FP64, two consecutive elements e, e + 1 (e even): what k_lincomb makes of them
+// with o as the last term
+__device__ __forceinline__ double2 nl_sum2(const NextLin &nl, double dt, long long e, double2 o) {
+  auto load = [&](const void *p) {
+    return *reinterpret_cast<const double2 *>((const double *)p + e);
+  };
+  double2 r = load(nl.base);
+  bool fx = false, fy = false;
+  if (nl.fxn) {
+    const bool self = nl.self != 0.0;
+    int ex = self ? fx_exponent(o.x, nl.fxself.k) : 0;
+    int ey = self ? fx_exponent(o.y, nl.fxself.k) : 0;
+#pragma unroll 1
+    for (int j = 0; j < nl.n; ++j) {
+      const double2 v = load(nl.k[j]);
+      ex = max(ex, fx_exponent(v.x, nl.fx[j].k));
+      ey = max(ey, fx_exponent(v.y, nl.fx[j].k));
+    }
+    const FxPoint px(ex), py(ey);
+    long long sx = 0, sy = 0;
+    auto add = [&](double2 v, FxCoef c) {
+      const long long x = px.get(v.x, fx_exponent(v.x, c.k));
+      const long long y = py.get(v.y, fx_exponent(v.y, c.k));
+      sx += fx_mul(fx_hi(x), (int)x, c);
+      sy += fx_mul(fx_hi(y), (int)y, c);
+    };
+#pragma unroll 1
+    for (int j = 0; j < nl.n; ++j) add(load(nl.k[j]), nl.fx[j]);
+    if (self) add(o, nl.fxself);
+    fx = px.fast;
+    fy = py.fast;
+    if (fx) r.x = fma(dt, px.put(sx), r.x);
+    if (fy) r.y = fma(dt, py.put(sy), r.y);
+  }
+  if (!fx || !fy) {
+    double ax = 0, ay = 0;
+#pragma unroll 1
+    for (int j = 0; j < nl.n; ++j) {
+      const double2 v = load(nl.k[j]);
+      ax = fma(nl.coef[j], v.x, ax);
+      ay = fma(nl.coef[j], v.y, ay);
+    }
+    ax = fma(nl.self, o.x, ax);
+    ay = fma(nl.self, o.y, ay);
+    if (!fx) r.x = fma(dt, ax, r.x);
+    if (!fy) r.y = fma(dt, ay, r.y);
+  }
+  return r;
+}
 // next-stage input at complex element e of the state (V = C2<T>): base +
 // dt (sum_j coef_j k_j + self o), written to y
 template <typename T>
 __device__ __forceinline__ void nl_apply_c(const NextLin &nl, T dt, long long e, C2<T> o,
                                            C2<T> *y) {
   typedef C2<T> V;
-  T ax = 0, ay = 0;
+  if constexpr (sizeof(T) == 8) {
+    const double2 r = nl_sum2(nl, dt, 2 * e, make_double2(o.x, o.y));
+    y[e] = mk2c<T>(r.x, r.y);
+  } else {
+    T ax = 0, ay = 0;
 #pragma unroll
-  for (int j = 0; j < kMaxTerms; ++j) {
-    if (j < nl.n) {
-      const V kv = reinterpret_cast<const V *>(nl.k[j])[e];
-      const T cj = nl_coef<T>(nl, j);
-      ax += cj * kv.x;
-      ay += cj * kv.y;
+    for (int j = 0; j < kMaxTerms; ++j) {
+      if (j < nl.n) {
+        const V kv = reinterpret_cast<const V *>(nl.k[j])[e];
+        const T cj = nl_coef<T>(nl, j);
+        ax += cj * kv.x;
+        ay += cj * kv.y;
+      }
     }
+    const T cs = nl_self<T>(nl);
+    ax += cs * o.x;
+    ay += cs * o.y;
+    const V bv = reinterpret_cast<const V *>(nl.base)[e];
+    y[e] = mk2c<T>(bv.x + dt * ax, bv.y + dt * ay);
   }
-  const T cs = nl_self<T>(nl);
-  ax += cs * o.x;
-  ay += cs * o.y;
-  const V bv = reinterpret_cast<const V *>(nl.base)[e];
-  y[e] = mk2c<T>(bv.x + dt * ax, bv.y + dt * ay);
 }
 
 // The equation of motion of mode id from its sources n0, n1 (zero for the
