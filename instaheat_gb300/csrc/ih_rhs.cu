@@ -23,6 +23,7 @@
 #include "ih_internal.cuh"
 #include "ih_tensor.cuh"
 #include "ih_fftcore.cuh"
+#include "ih_fix.cuh"
 
 namespace ih {
 
@@ -242,9 +243,9 @@ __global__ void k_update_phi_psi(T *y, const double *ysc, const T *__restrict__ 
     h3 = 3.0 * H;
     pm = rs->p_mean;
   }
-  // FP64: the factors of the fused multiply-adds below (10 FP64 instructions
+  // FP64: the factors of the fused multiply-adds below (9 FP64 instructions
   // a point; the FP64 pipe bounds that form)
-  const T ia4 = (T)4 * inv_a2, m22 = (T)2 * m2, H4 = (T)4 * H;
+  const T ia4 = (T)4 * inv_a2, m22 = (T)2 * m2, H4 = (T)4 * H, pm2 = (T)0.5 * pm;
   T phib = 0, pib = 0, psib = 0, dpsib = 0;
   if (MIXED) {
     phib = (T)ysc[0];
@@ -271,7 +272,7 @@ __global__ void k_update_phi_psi(T *y, const double *ysc, const T *__restrict__ 
         // p / 2 + (psi - 1/2) <p> - 4 H dpsi
         o1[w] = fma(fma(ps[w], ia4, inv_a2), l[w],
                     -fma(fma(dps[w], (T)-4.0, h3), dph[w], fma(ps[w], m22, m2) * ph[w]));
-        o3[w] = fma((T)0.5, pp[w] - pm, fma(ps[w], pm, -(H4 * dps[w])));
+        o3[w] = fma(ps[w], pm, fma(-H4, dps[w], fma((T)0.5, pp[w], -pm2)));
       } else {
         T psf = psib + ps[w], dpsf = dpsib + dps[w];
         o1[w] = ((T)1.0 + (T)4.0 * psf) * l[w] * inv_a2 + (T)4.0 * dps[w] * pib -
@@ -384,11 +385,16 @@ __global__ void __launch_bounds__(256, 3) k_update_h_next(
 // instructions of a mode, and the FP64 pipe is what bounds this kernel.  The
 // table holds alpha, beta and |k|^2 of the octant kx, ky, kz >= 0; a thread
 // reads one entry and handles the up to four modes (+-kx, +-ky, kz) that share
-// it: 26 bytes of table per mode beside 224 of data.  256^3: 0.594 ms against
+// it: 28 bytes of table per mode beside 224 of data.  256^3: 0.594 ms against
 // 1.592 ms with the coefficients formed per mode (3.2 TB/s; 37 FP64
 // instructions per mode are 0.59 ms); 64^3: 21 us against 42.
-constexpr int kTensorCoefs = 13;
-__global__ void k_tensor_table(double *coef, long long Mo, Geom g) {
+//
+// The twelve products of a mode's real and of its imaginary parts are summed in
+// integers (FxPoint, ih_fix.cuh: 13 FP64 instructions a mode are left): 256^3 555
+// -> 387 us (4.9 TB/s), 128^3 80 -> 62.  The coefficients are stored for that, as
+// fractions of 2^k, alpha and beta with a k each.
+constexpr int kTensorCoefs = 14;
+__global__ void k_tensor_table(long long *coef, long long Mo, Geom g) {
   const int nyh = g.ny / 2 + 1;
   for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < Mo;
        o += (long long)gridDim.x * blockDim.x) {
@@ -397,25 +403,74 @@ __global__ void k_tensor_table(double *coef, long long Mo, Geom g) {
                  ksq = ksq64(g, i, j, k);
     const double inv = o ? 1.0 / ksq : 0.0;
     const int branch = k ? 0 : (j ? 1 : 2);
-    for (int a = 0; a < 6; ++a) {
-      double al = 0.0, be = 0.0;  // the zero mode has no sources
-      if (o) tensor_coef<double>(a, branch, kx, ky, kz, kx * inv, ky * inv, kz * inv, al, be);
-      coef[a * Mo + o] = al;
-      coef[(6 + a) * Mo + o] = be;
+    double c[2][6];
+    int e[2];
+    for (int n = 0; n < 2; ++n) {
+      double m = 0.0;
+      for (int a = 0; a < 6; ++a) {
+        double al = 0.0, be = 0.0;  // the zero mode has no sources
+        if (o) tensor_coef<double>(a, branch, kx, ky, kz, kx * inv, ky * inv, kz * inv, al, be);
+        c[n][a] = n ? be : al;
+        m = fmax(m, fabs(c[n][a]));
+      }
+      frexp(m, &e[n]);
+      for (int a = 0; a < 6; ++a)
+        coef[(6 * n + a) * Mo + o] = __double2ll_rn(ldexp(c[n][a], 62 - e[n]));
     }
-    coef[12 * Mo + o] = ksq;
+    coef[12 * Mo + o] = __double_as_longlong(ksq);
+    coef[13 * Mo + o] = (long long)e[1] << 32 | (unsigned)e[0];
   }
 }
 // v, negated where f
-__device__ __forceinline__ double flip(double v, int f) {
-  return __hiloint2double(__double2hiint(v) ^ (f << 31), __double2loint(v));
+__device__ __forceinline__ long long flip(long long v, int f) { return (v ^ -(long long)f) + f; }
+// sum_a al_a x_a and sum_a be_a x_a, the coefficients fractions of 2^k0 and 2^k1
+__device__ __forceinline__ void tensor_sums(const double (&x)[6], const long long (&al)[6],
+                                            const long long (&be)[6], int k0, int k1, double &n0,
+                                            double &n1) {
+  int e[6], em = 0;
+#pragma unroll
+  for (int a = 0; a < 6; ++a) {
+    e[a] = fx_exponent(x[a], 0);
+    em = max(em, e[a]);
+  }
+  const FxPoint pt(em);
+  if (pt.fast) {
+    long long s0 = 0, s1 = 0;
+#pragma unroll
+    for (int a = 0; a < 6; ++a) {
+      const long long xi = pt.get(x[a], e[a]);
+      const int xh = fx_hi(xi), xl = (int)xi;
+      s0 += fx_mul(xh, xl, fx_hi(al[a]), (int)al[a]);
+      s1 += fx_mul(xh, xl, fx_hi(be[a]), (int)be[a]);
+    }
+    n0 = pt.put(s0, k0);
+    n1 = pt.put(s1, k1);
+  } else {
+    const double u0 = ldexp(1.0, k0 - 62), u1 = ldexp(1.0, k1 - 62);
+    n0 = n1 = 0.0;
+#pragma unroll 1
+    for (int a = 0; a < 6; ++a) {
+      double xa = x[0];
+      long long ca = al[0], cb = be[0];
+#pragma unroll
+      for (int b = 1; b < 6; ++b) {
+        if (a == b) {
+          xa = x[b];
+          ca = al[b];
+          cb = be[b];
+        }
+      }
+      n0 += u0 * __ll2double_rn(ca) * xa;
+      n1 += u1 * __ll2double_rn(cb) * xa;
+    }
+  }
 }
 // per: modes of an octant entry per thread (4, or fewer with the rest on
 // gridDim.y where the grid would otherwise leave SMs idle)
 template <bool NEXT>
 __global__ void __launch_bounds__(128) k_update_h_tab(
     const double2 *__restrict__ s, double *y, double *__restrict__ out, const RhsScalars *rs,
-    Geom g, const double *__restrict__ coef, int Mo, const NextLin nl, int per) {
+    Geom g, const long long *__restrict__ coef, int Mo, const NextLin nl, int per) {
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= Mo) return;
   const int nyh = g.ny / 2 + 1;
@@ -423,13 +478,17 @@ __global__ void __launch_bounds__(128) k_update_h_tab(
   const long long M = g.M;
   const TensorConsts<double> tc(rs);
   const double dt = NEXT ? *nl.dt : 0.0;
-  double al[6], be[6];
+  long long al[6], be[6];
 #pragma unroll
   for (int a = 0; a < 6; ++a) {
     al[a] = coef[(long long)a * Mo + o];
     be[a] = coef[(long long)(6 + a) * Mo + o];
   }
-  const double ksq = coef[(long long)12 * Mo + o];
+  const double ksq = __longlong_as_double(coef[(long long)12 * Mo + o]);
+  const long long ks = coef[(long long)13 * Mo + o];
+  const int k0 = (int)ks, k1 = (int)(ks >> 32);
+  int px = 0, py = 0;  // the signs that al and be have
+#pragma unroll 1
   for (int q = blockIdx.y * per; q < (int)(blockIdx.y + 1) * per; ++q) {
     const int sx = q & 1, sy = q >> 1;
     if ((sx && (i == 0 || 2 * i == g.nx)) || (sy && (j == 0 || 2 * j == g.ny))) continue;
@@ -441,18 +500,22 @@ __global__ void __launch_bounds__(128) k_update_h_tab(
     // a coefficient of S_ab in n_cd changes sign with kx (ky) when x (y)
     // occurs an odd number of times in a, b, c, d; n0 is xx (yy for kz = ky =
     // 0) and n1 xy (xz for kz = 0, yz for kz = ky = 0)
-    const int sxy = sx ^ sy;
-    const int f1[6] = {sxy, 0, k ? sy : 0, sxy, k ? sx : (j ? sxy : 0), sxy};
-    const int f0[6] = {0, sxy, sx, 0, sy, 0};
-    double2 n0 = make_double2(0.0, 0.0), n1 = n0;
+    const int fx = sx ^ px, fy = sy ^ py, fxy = fx ^ fy;
+    px = sx;
+    py = sy;
+    const int f1[6] = {fxy, 0, k ? fy : 0, fxy, k ? fx : (j ? fxy : 0), fxy};
+    const int f0[6] = {0, fxy, fx, 0, fy, 0};
+    double xr[6], xi[6];
 #pragma unroll
     for (int a = 0; a < 6; ++a) {
-      const double ca = flip(al[a], f0[a]), cb = flip(be[a], f1[a]);
-      n0.x += ca * v[a].x;
-      n0.y += ca * v[a].y;
-      n1.x += cb * v[a].x;
-      n1.y += cb * v[a].y;
+      al[a] = flip(al[a], f0[a]);
+      be[a] = flip(be[a], f1[a]);
+      xr[a] = v[a].x;
+      xi[a] = v[a].y;
     }
+    double2 n0, n1;
+    tensor_sums(xr, al, be, k0, k1, n0.x, n1.x);
+    tensor_sums(xi, al, be, k0, k1, n0.y, n1.y);
     if (id == 0) n0 = n1 = make_double2(0.0, 0.0);
     tensor_eom<double, NEXT>(g, id, n0, n1, ksq, tc, y, out, nl, dt);
   }
@@ -462,7 +525,7 @@ int tensor_table(Ctx *c) {
   const long long Mo = (long long)(g.nx / 2 + 1) * (g.ny / 2 + 1) * g.mz;
   IH_CUDA(c, cudaMalloc(&c->tensor_coef, sizeof(double) * kTensorCoefs * Mo));
   c->dev_bytes += sizeof(double) * kTensorCoefs * Mo;
-  k_tensor_table<<<grid_for(Mo, 256, 1), 256, 0, c->stream>>>((double *)c->tensor_coef, Mo, g);
+  k_tensor_table<<<grid_for(Mo, 256, 1), 256, 0, c->stream>>>((long long *)c->tensor_coef, Mo, g);
   return check_launch(c, "k_tensor_table");
 }
 
@@ -569,7 +632,7 @@ static int tensor_last_pass_t(Ctx *c, C2<T> *s, T *y, T *out, double *outsc,
     const int per = nb >= wave ? 4 : (2 * nb >= wave ? 2 : 1);
     auto kf = next ? k_update_h_tab<true> : k_update_h_tab<false>;
     kf<<<dim3(nb, 4 / per), 128, 0, c->stream>>>(s, y, out, c->rs, g,
-                                                 (const double *)c->tensor_coef, Mo, nl, per);
+                                                 (const long long *)c->tensor_coef, Mo, nl, per);
   }
   prof_end(c, KK_UPDATE_H,
            6.0 * M * sizeof(C2<T>) +

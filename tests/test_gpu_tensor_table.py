@@ -57,3 +57,25 @@ def test_stage_fusion_is_identical_at_odd_sizes(gpu_mod):
         runs.append(ctx.get_state())
         ctx.close()
     assert np.array_equal(*runs)
+
+
+@pytest.mark.parametrize("n", [(16, 12, 8), (32, 32, 32)])
+def test_sources_outside_the_integer_range(gpu_mod, n):
+    """The projection of sources of 2^-960 the size (summed in FP64): the same
+    values but for the scale, to 1e-13 of the norm."""
+    rng = np.random.default_rng(5)
+    x = None
+    runs = []
+    for s in (0, -480):
+        ctx = gpu_mod.Context(n=n)
+        x = rng.standard_normal(ctx.N) if x is None else x
+        f = np.zeros(ctx.Ntot)
+        f[:ctx.N] = np.ldexp(1e-2 * x, s)
+        f[ctx.N:2 * ctx.N] = -0.8
+        f[-1] = 1.3
+        r, _ = ctx.mk_rhs(f)
+        runs.append(np.ldexp(r[4 * ctx.N + 4 * ctx.M:-1], -2 * s))
+        ctx.close()
+    a, b = runs
+    assert np.linalg.norm(a) > 0
+    assert np.linalg.norm(a - b) <= 1e-13 * np.linalg.norm(a)
