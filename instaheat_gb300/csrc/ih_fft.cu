@@ -1725,6 +1725,111 @@ __global__ void __launch_bounds__(32 * zwarps<T>(), (sizeof(T) == 4 && H <= 128 
 }
 
 // ---------------------------------------------------------------------------
+// The z part of the mixed form's RHS for rows with a factor 3 in one kernel, the
+// passes of z_pass_generic (ih_rhs.cu) for kZB rows per CTA: 4 c2r, rho and p and
+// their FP64 sums, 6 products and their r2c, each value with the operations of
+// k_fft_zc2r_g, k_pointwise_g and k_fft_zr2c_g.  Unfused it moved 33 arrays of the
+// grid through memory instead of 15: 96^3 94 us (4 + 1 + 6 launches) -> 49.5, step 2.16
+// -> 1.92 ms; 192^3 step 11.6 -> 9.7 ms.  Spectra d4 (d/dx, d/dy, d/dz, laplacian) and
+// s6 may share their rows: a CTA reads all of its own before it writes.
+template <int H>
+__global__ void __launch_bounds__(stk_threads<H, kZB>()) k_fft_z_rhs_g(
+    const C2<float> *d4, long long stride, const float *__restrict__ yfl,
+    const double *__restrict__ ysc, float *__restrict__ lap, float *__restrict__ pout,
+    float *__restrict__ rhoout, C2<float> *s6, int gw, double *partials, Geom g,
+    const C2<float> *__restrict__ twhg, const C2<float> *__restrict__ twzg) {
+  using F2 = C2<float>;
+  constexpr int P = kZB + 1, NT = stk_threads<H, kZB>();
+  extern __shared__ __align__(16) unsigned char smraw[];
+  F2 *twh = reinterpret_cast<F2 *>(smraw), *twz = twh + H, *tile = twz + 2 * H;
+  F2 *w = tile + 3 * H * P;  // the laplacian, then the products
+  const int tid = threadIdx.x;
+  load_table(twh, twhg, H, tid, NT);
+  load_table(twz, twzg, 2 * H, tid, NT);
+  __syncthreads();
+  const long long r0 = (long long)blockIdx.x * kZB, rows = (long long)g.nx * g.ny;
+  for (int idx = tid; idx < H * kZB; idx += NT) {
+    const int k = idx % H, b = idx / H;
+    const long long r = r0 + b;
+    F2 wn = twz[k];
+    wn.y = -wn.y;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      F2 zv = mk2<float>(0, 0);
+      if (r < rows) {
+        const F2 *src = d4 + a * stride + r * (H + 1);
+        const F2 x = src[k], xp = src[H - k];
+        const F2 pc = mk2<float>(xp.x, -xp.y);
+        const F2 e = cadd(x, pc), d = csub(x, pc);
+        const F2 o = cmul(d, wn);
+        zv = mk2<float>(e.x - o.y, e.y + o.x);
+      }
+      tile[(a * H + k) * P + b] = zv;
+    }
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int a = 0; a < 4; ++a) smem_stk<float, H, kZB>(tile + a * H * P, P, twh, +1, tid);
+  const long long N = g.N;
+  const double a_sc = ysc[4];
+  const float inv_a2 = (float)(1.0 / (a_sc * a_sc)), m2 = (float)(g.mass * g.mass);
+  const float third = (float)(1.0 / 3.0);
+  const float phib = (float)ysc[0], pib = (float)ysc[1], psib = (float)ysc[2];
+  double sr = 0.0, sp = 0.0;
+  // (the separate pass stores the squares: each is rounded before the sum)
+  auto square = [](float x, float y, float z) {
+    return __fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z));
+  };
+  for (int idx = tid; idx < H * kZB; idx += NT) {  // value j = reals 2j, 2j+1
+    const int j = idx % H, b = idx / H;
+    const long long r = r0 + b;
+    if (r >= rows) continue;
+    const long long e = r * 2 * H + 2 * j;
+    const F2 dx = tile[j * P + b], dy = tile[(H + j) * P + b], dz = tile[(2 * H + j) * P + b];
+    const F2 ph = *reinterpret_cast<const F2 *>(yfl + e);
+    const F2 dp = *reinterpret_cast<const F2 *>(yfl + N + e);
+    const F2 ps = *reinterpret_cast<const F2 *>(yfl + 2 * N + e);
+    F2 rho, p;
+    rho_p_of_grad<float, true>(square(dx.x, dy.x, dz.x), ph.x, dp.x, ps.x, inv_a2, m2, third, phib, pib, psib,
+                               rho.x, p.x);
+    rho_p_of_grad<float, true>(square(dx.y, dy.y, dz.y), ph.y, dp.y, ps.y, inv_a2, m2, third, phib, pib, psib,
+                               rho.y, p.y);
+    *reinterpret_cast<F2 *>(lap + e) = w[j * P + b];
+    *reinterpret_cast<F2 *>(pout + e) = p;
+    if (rhoout) *reinterpret_cast<F2 *>(rhoout + e) = rho;
+    sr += (double)rho.x + (double)rho.y;
+    sp += (double)p.x + (double)p.y;
+  }
+  rhs_partial<NT>(sr, sp, partials);
+  if (!gw) return;
+#pragma unroll 1
+  for (int pr = 0; pr < 6; ++pr) {
+    const int ia = pr < 3 ? 0 : (pr < 5 ? 1 : 2);
+    const int ib = pr < 3 ? pr : (pr < 5 ? pr - 2 : 2);
+    const F2 *ta = tile + ia * H * P, *tb = tile + ib * H * P;
+    __syncthreads();  // w is read
+    for (int idx = tid; idx < H * kZB; idx += NT) {
+      const int at = idx / kZB * P + (idx & (kZB - 1));
+      const F2 x = ta[at], y = tb[at];
+      w[at] = mk2<float>(__fmul_rn(x.x, y.x), __fmul_rn(x.y, y.y));
+    }
+    __syncthreads();
+    smem_stk<float, H, kZB>(w, P, twh, -1, tid);
+    F2 *dst = s6 + pr * stride;
+    for (int idx = tid; idx < (H + 1) * kZB; idx += NT) {
+      const int k = idx % (H + 1), b = idx / (H + 1);
+      const long long r = r0 + b;
+      if (r >= rows) continue;
+      const F2 z = w[(k % H) * P + b], zp = w[((H - k) % H) * P + b];
+      const F2 zc = mk2<float>(zp.x, -zp.y);
+      const F2 e = mk2<float>(0.5f * (z.x + zc.x), 0.5f * (z.y + zc.y));
+      const F2 o = mk2<float>(0.5f * (z.y - zc.y), -0.5f * (z.x - zc.x));
+      dst[r * (H + 1) + k] = cadd(e, cmul(o, twz[k]));
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // host launchers
 
 // rows of a z-pass CTA
@@ -2395,6 +2500,43 @@ int fft_z_rhs_fused(Ctx *c, const C2<T> *d4, const T *yfl, const double *ysc, T 
            (double)(4 + (gw ? 6 : 0)) * g.M * sizeof(C2<T>) +
                (double)(3 + 2 + (rho ? 1 : 0)) * g.N * sizeof(T));
   return check_launch(c, "k_fft_z_rhs_fused");
+}
+
+struct ZRhs3Launch {
+  Ctx *c;
+  C2<float> *spec;
+  const float *yfl;
+  const double *ysc;
+  float *lap, *p, *rho;
+  template <int H>
+  int run_reg() {
+    if constexpr (H > 192) {  // (nz <= 512)
+      return IH_ERR_ARG;
+    } else {
+      const Geom &g = c->g;
+      const long long rows = (long long)g.nx * g.ny;
+      const unsigned nblk = (unsigned)((rows + kZB - 1) / kZB);
+      const size_t sm = sizeof(C2<float>) * (3 * (size_t)H + 4 * (size_t)H * (kZB + 1));
+      want_smem(k_fft_z_rhs_g<H>, sm);
+      c->z_blocks = (int)nblk;
+      k_fft_z_rhs_g<H><<<nblk, stk_threads<H, kZB>(), sm, c->stream>>>(
+          spec, g.M, yfl, ysc, lap, p, rho, spec, c->p.enable_gw, c->partials, g,
+          tab<float>(c->tw_h), tab<float>(c->tw_z));
+      return IH_OK;
+    }
+  }
+};
+bool z_rhs_g_ok(const Ctx *c) { return c->mixed && stk_length3(c->g.h); }
+int z_rhs_g(Ctx *c, void *spec, const void *yfl, const double *ysc, void *lap, void *p, void *rho) {
+  const Geom &g = c->g;
+  const int gw = c->p.enable_gw;
+  prof_begin(c, KK_Z_RHS_FUSED);
+  IH_TRY(dispatch_len3(g.h, ZRhs3Launch{c, (C2<float> *)spec, (const float *)yfl, ysc, (float *)lap,
+                                        (float *)p, (float *)rho}));
+  prof_end(c, KK_Z_RHS_FUSED,
+           (double)(4 + (gw ? 6 : 0)) * g.M * sizeof(C2<float>) +
+               (double)(3 + 2 + (rho ? 1 : 0)) * g.N * sizeof(float));
+  return check_launch(c, "k_fft_z_rhs_g");
 }
 
 // twiddle tables, computed in FP64 on the host

@@ -212,13 +212,10 @@ __device__ __forceinline__ void rhs_partial(double dr, double dp, double *partia
 // gradient dx, dy, dz, phi, dphi and psi.  FP64 form: full values.  Mixed form
 // (MIXED): the arguments are fluctuations about the FP64 homogeneous parts
 // phib, pib (= <dphi>), psib, and rho, p are the fluctuation parts, expanded
-// so that no O(1) background cancels in FP32.
+// so that no O(1) background cancels in FP32.  _of_grad: from |grad phi|^2.
 template <typename T, bool MIXED>
-__device__ __forceinline__ void rho_p(T dx, T dy, T dz, T phi, T dph, T ps, T inv_a2, T m2, T third,
-                                      T phib, T pib, T psib, T &rho, T &p) {
-  T grad = dx * dx;
-  grad += dy * dy;
-  grad += dz * dz;
+__device__ __forceinline__ void rho_p_of_grad(T grad, T phi, T dph, T ps, T inv_a2, T m2, T third,
+                                              T phib, T pib, T psib, T &rho, T &p) {
   if (!MIXED) {
     T t1 = ((T)0.5 - ps) * dph * dph;
     T t2 = ((T)0.5 + ps) * grad * inv_a2;
@@ -233,6 +230,15 @@ __device__ __forceinline__ void rho_p(T dx, T dy, T dz, T phi, T dph, T ps, T in
     rho = kin + grd + pot;
     p = kin - grd * third - pot;
   }
+}
+
+template <typename T, bool MIXED>
+__device__ __forceinline__ void rho_p(T dx, T dy, T dz, T phi, T dph, T ps, T inv_a2, T m2, T third,
+                                      T phib, T pib, T psib, T &rho, T &p) {
+  T grad = dx * dx;
+  grad += dy * dy;
+  grad += dz * dz;
+  rho_p_of_grad<T, MIXED>(grad, phi, dph, ps, inv_a2, m2, third, phib, pib, psib, rho, p);
 }
 
 }  // namespace ih

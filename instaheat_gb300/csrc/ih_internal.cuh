@@ -383,6 +383,9 @@ int zreg_pass(Ctx *c, const void *in, long long istride, void *out, long long os
               bool forward);
 int zreg_rhs(Ctx *c, const void *d4, const void *yfl, const double *ysc, void *lap, void *p,
              void *rho, void *s6, int gw, double *partials, int zsrc);
+// the z part of the mixed form's RHS in one kernel for rows with a factor 3
+bool z_rhs_g_ok(const Ctx *c);
+int z_rhs_g(Ctx *c, void *spec, const void *yfl, const double *ysc, void *lap, void *p, void *rho);
 // whether the z pass of the RHS is one fused kernel, and whether the x and y
 // round trips exist (else the full-spectrum route)
 inline bool zfused_ok(const Ctx *c) { return c->g.pow2 || (c->fx_on >> 6 & 1); }

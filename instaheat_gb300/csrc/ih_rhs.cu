@@ -1278,6 +1278,7 @@ static int z_pass_generic(Ctx *c, C2<T> *spec, const T *yfl, const double *ysc, 
                           T *rho) {
   const Geom &g = c->g;
   const long long N = g.N, M = g.M;
+  if (z_rhs_g_ok(c)) return z_rhs_g(c, spec, yfl, ysc, lap, p, rho);
   T *gs = (T *)c->gscratch;
   const int gw = c->p.enable_gw;
   IH_TRY((fft_zc2r<T>(c, spec, M, gs, N, 3)));
