@@ -280,7 +280,9 @@ def f64_roofline(ms_per_step, peak, peak_src, fp64=FP64_NOMINAL_TFLOPS, fp64_src
     per-step formula at 8 bytes per value) against the HBM copy peak, and its
     flops -- 12 RHS x 11 transforms x 2.5 N log2 N plus about 160 Ntot in the
     stage combinations -- against the FP64 FMA rate (measured by
-    ih_fp64_fma_peak on this GPU)."""
+    ih_fp64_fma_peak on this GPU).  A fraction above 1 says that the FP64 pipe
+    does not do them: the transforms and sums run on the integer pipes
+    (csrc/ih_fix.cuh)."""
     n = N_GRID
     N = n ** 3
     Next = 2 * n * n * (n // 2 + 1)
@@ -291,7 +293,8 @@ def f64_roofline(ms_per_step, peak, peak_src, fp64=FP64_NOMINAL_TFLOPS, fp64_src
     alu = {"flops_per_step": flops, "achieved": tflops, "peak": fp64, "peak_source": fp64_src,
            "unit": "TFLOP/s", "frac": tflops / fp64,
            "floor_ms_per_step": flops / (fp64 * 1e12) * 1e3}
-    return {"bound": "fp64" if alu["frac"] >= hbm["frac"] else "hbm", "hbm": hbm, "fp64": alu}
+    fp64_bound = hbm["frac"] <= alu["frac"] <= 1.0
+    return {"bound": "fp64" if fp64_bound else "hbm", "hbm": hbm, "fp64": alu}
 
 
 def bench_e2e(gpu, ctx, steps):
