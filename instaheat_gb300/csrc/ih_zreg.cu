@@ -250,7 +250,7 @@ struct RzIn {
   const F2 *d4;
   long long dstride;
   float kzu, invnz;
-  int nz, zsrc;  // zsrc: d/dz from Z in slot 4
+  int zsrc;  // d/dz from Z in slot 4
 };
 template <int H>
 __device__ __forceinline__ void rz_deriv(const RzIn &in, int a, const RzLane &ln, const RzTw<H> &w,
@@ -496,7 +496,7 @@ struct RzRhs {
       c->err = "grid too large for the RHS partial-sum buffer";
       return IH_ERR_ARG;
     }
-    const RzIn in{(const F2 *)d4, g.M, (float)g.kzu, (float)(1.0 / (double)g.nz), g.nz, zsrc};
+    const RzIn in{(const F2 *)d4, g.M, (float)g.kzu, (float)(1.0 / (double)g.nz), zsrc};
     RzPoint pt{};
     pt.yfl = (const float *)yfl;
     pt.p = (float *)p;
