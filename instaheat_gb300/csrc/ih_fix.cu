@@ -271,7 +271,7 @@ static int fx_upload_twiddles(Ctx *c, void **dst, int L) {
     }
     const long long C = llrintl(ldexpl(re, 62)), S = llrintl(ldexpl(-im, 62));
     fx_split(C, a[4 * k], a[4 * k + 1]);
-    fx_split(S - C, a[4 * k + 2], a[4 * k + 3]);
+    fx_split(C - S, a[4 * k + 2], a[4 * k + 3]);
     fx_split(S + C, b[2 * k], b[2 * k + 1]);
   }
   IH_CUDA(c, cudaMalloc(dst, sizeof(int) * host.size()));

@@ -29,8 +29,8 @@ struct __align__(16) fx2 {
 };
 
 // a table twiddle c + i s as the three products of a complex multiplication
-// need it: c, s - c, s + c in Q62, each split as high * 2^32 + low with a
-// signed low word (a = {c high, c low, s-c high, s-c low}, b = {s+c})
+// need it: c, c - s, c + s in Q62, each split as high * 2^32 + low with a
+// signed low word (a = {c high, c low, c-s high, c-s low}, b = {c+s})
 struct FxTab {
   const int4 *a;
   const int2 *b;
@@ -59,10 +59,23 @@ __device__ __forceinline__ fx2 operator-(fx2 a, fx2 b) { return fx_mk(a.x - b.x,
 __device__ __forceinline__ int fx_hi(long long a) {
   return (int)(a >> 32) + (int)((unsigned)a >> 31);
 }
-// a w / 2^64 from the split halves of both: the low * low product is left out
-// (below half a unit, of either sign), the two cross products round down, on
-// average by one unit together, which the + 1 returns
+// a w / 2^64 from the split halves of both, the low * low product (a quarter of a
+// unit at most, of either sign) left out.  A product with zero is zero in the first two
+// forms, so that what cancels exactly in FP64 transforms cancels here.
+//   fx_mul_low: both cross products round down, by a unit on average together, half
+//   a unit for a small a; for differences of two products, where that goes away.
+__device__ __forceinline__ long long fx_mul_low(int ah, int al, int wh, int wl) {
+  return (long long)ah * wh + (__mulhi(ah, wl) + __mulhi(al, wh));
+}
+//   fx_mul: al w rounds to nearest, so a small a has no bias, a large one half a
+//   unit.  (Both to nearest: 5% more time in every pass that has it.)
 __device__ __forceinline__ long long fx_mul(int ah, int al, int wh, int wl) {
+  const int c = __mulhi(ah, wl) + (int)(((long long)al * wh + 0x80000000LL) >> 32);
+  return (long long)ah * wh + c;
+}
+//   fx_mul_sum: the + 1 returns the average unit; one unit for a zero.  For sums
+//   of a few products, where a unit is nothing.
+__device__ __forceinline__ long long fx_mul_sum(int ah, int al, int wh, int wl) {
   const int c = __mulhi(ah, wl) + __mulhi(al, wh) + 1;
   return (long long)ah * wh + c;
 }
@@ -73,15 +86,19 @@ __device__ __forceinline__ long long fx_mul(long long a, int wh, int wl) {
 __device__ __forceinline__ long long fx_mul(long long a, long long w) {
   return fx_mul(fx_hi(a), (int)a, fx_hi(w), (int)w);
 }
+__device__ __forceinline__ long long fx_mul_sum(long long a, long long w) {
+  return fx_mul_sum(fx_hi(a), (int)a, fx_hi(w), (int)w);
+}
 // v (c + i s) / 4 (S = -1) or v (c - i s) / 4 (S = +1), the table holding the
-// forward twiddle
+// forward twiddle; each component the difference of two products
 template <int S>
 __device__ __forceinline__ fx2 fx_cmul(fx2 v, const FxW &w) {
-  const long long k = fx_mul(v.x + v.y, w.a.x, w.a.y);
+  const long long m = v.x + v.y;
+  const long long k = fx_mul_low(fx_hi(m), (int)m, w.a.x, w.a.y);
   const int xh = fx_hi(v.x), xl = (int)v.x, yh = fx_hi(v.y), yl = (int)v.y;
   if (S < 0)
-    return fx_mk(k - fx_mul(yh, yl, w.b.x, w.b.y), k + fx_mul(xh, xl, w.a.z, w.a.w));
-  return fx_mk(k + fx_mul(yh, yl, w.a.z, w.a.w), k - fx_mul(xh, xl, w.b.x, w.b.y));
+    return fx_mk(k - fx_mul_low(yh, yl, w.b.x, w.b.y), k - fx_mul_low(xh, xl, w.a.z, w.a.w));
+  return fx_mk(k - fx_mul_low(yh, yl, w.a.z, w.a.w), k - fx_mul_low(xh, xl, w.b.x, w.b.y));
 }
 // v / 4, the trivial twiddle
 __device__ __forceinline__ fx2 fx_quarter(fx2 v) { return fx_mk((v.x + 2) >> 2, (v.y + 2) >> 2); }
@@ -125,14 +142,14 @@ __device__ __forceinline__ fx2 fx_rot32(fx2 v) {
       v.y += v.x - fx_mul(v.x, kFxOneMinusSin3Pi16);
     else
       v.y += fx_mul(v.x, ra == 1 ? kFxSinPi16 : kFxSinPi8);
-    v.x -= fx_mul(v.y, T);
+    v.x += fx_mul(v.y, -T);  // (of the sign that the first product's bias does not have)
   } else {
     v.x += fx_mul(v.y, T);
     if (ra == 3)
       v.y -= v.x - fx_mul(v.x, kFxOneMinusSin3Pi16);
     else
       v.y -= fx_mul(v.x, ra == 1 ? kFxSinPi16 : kFxSinPi8);
-    v.x += fx_mul(v.y, T);
+    v.x -= fx_mul(v.y, -T);
   }
   return v;
 }
@@ -241,7 +258,7 @@ __device__ __forceinline__ FxScale fx_scale(unsigned m, int p) {
       s.pre = 0.0;
       s.post = __longlong_as_double(0x7ff8000000000000LL);
     }
-    if (m == 0) s.post = 0.0;  // all zero: products of zeros carry a rounding unit
+    if (m == 0) s.post = 0.0;  // all zero
   }
   s.in = p + 1022 - E;
   s.out = -s.in;
@@ -363,8 +380,8 @@ __device__ __forceinline__ fx2 fx_shift(fx2 v, const FxShift &f) {
 // unit per term, 2^-57 of the largest product: below that of an FP64 sum, whose
 // terms each round to 2^-53 of a partial sum.
 constexpr int kFxSum = 3;  // terms from which FP64 sums of vectors are summed so
-__device__ __forceinline__ long long fx_mul(int ah, int al, FxCoef c) {
-  return fx_mul(ah, al, c.h, c.l);
+__device__ __forceinline__ long long fx_mul_sum(int ah, int al, FxCoef c) {
+  return fx_mul_sum(ah, al, c.h, c.l);
 }
 __device__ __forceinline__ int fx_exponent(double x, int k) {  // biased, of x 2^k
   return ((__double2hiint(x) >> 20) & 0x7ff) + k;

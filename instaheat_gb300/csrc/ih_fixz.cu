@@ -268,8 +268,8 @@ struct FxZPoint {
                    fz = fx_out<true>(gz, ex[2]) * post[2];
       return fx * fx + fy * fy + fz * fz;
     }
-    return fx_out<true>((fx_mul(gx, gx) >> r[0]) + (fx_mul(gy, gy) >> r[1]) +
-                            (fx_mul(gz, gz) >> r[2]), eg);
+    return fx_out<true>((fx_mul_sum(gx, gx) >> r[0]) + (fx_mul_sum(gy, gy) >> r[1]) +
+                            (fx_mul_sum(gz, gz) >> r[2]), eg);
   }
   __device__ __forceinline__ void operator()(double grad, double f, double d, double s, double &rho,
                                              double &p) const {
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(32 * kFxWarps, fx_z_ctas<H>()) k_fx_z_rhs(
 #pragma unroll
     for (int m = 0; m < A; ++m) {
       const fx2 a = ln.valid ? ga[B * m] : fx_mk(0, 0), b = ln.valid ? gb[B * m] : fx_mk(0, 0);
-      v[m] = fx_mk(fx_mul(a.x, b.x), fx_mul(a.y, b.y));
+      v[m] = fx_mk(fx_mul_sum(a.x, b.x), fx_mul_sum(a.y, b.y));
     }
     const int ea = ia == 0 ? pt.ex[0] : (ia == 1 ? pt.ex[1] : pt.ex[2]);
     const int eb = ib == 0 ? pt.ex[0] : (ib == 1 ? pt.ex[1] : pt.ex[2]);
@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(256, fx_zco_ctas<H>()) k_fx_z_rhs_co(
 #pragma unroll
     for (int m = 0; m < A; ++m) {
       const fx2 a = sm.grad[ia][m][lane], b = sm.grad[ib][m][lane];
-      v[m] = fx_mk(fx_mul(a.x, b.x), fx_mul(a.y, b.y));
+      v[m] = fx_mk(fx_mul_sum(a.x, b.x), fx_mul_sum(a.y, b.y));
     }
     const bool slow =
         sm.post[0][grp] != 1.0 || sm.post[1][grp] != 1.0 || sm.post[2][grp] != 1.0;

@@ -440,8 +440,8 @@ __device__ __forceinline__ void tensor_sums(const double (&x)[6], const long lon
     for (int a = 0; a < 6; ++a) {
       const long long xi = pt.get(x[a], e[a]);
       const int xh = fx_hi(xi), xl = (int)xi;
-      s0 += fx_mul(xh, xl, fx_hi(al[a]), (int)al[a]);
-      s1 += fx_mul(xh, xl, fx_hi(be[a]), (int)be[a]);
+      s0 += fx_mul_sum(xh, xl, fx_hi(al[a]), (int)al[a]);
+      s1 += fx_mul_sum(xh, xl, fx_hi(be[a]), (int)be[a]);
     }
     n0 = pt.put(s0, k0);
     n1 = pt.put(s1, k1);

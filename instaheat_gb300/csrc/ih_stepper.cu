@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(256) k_lincomb(const T *__restrict__ base, con
 #pragma unroll
           for (int j = 0; j < NT; ++j) {
             const long long xi = pt.get(x[j][w], e[j]);
-            s += fx_mul(fx_hi(xi), (int)xi, args.fx[j]);
+            s += fx_mul_sum(fx_hi(xi), (int)xi, args.fx[j]);
           }
           acc[w] = fma(sc, (T)pt.put(s), x[NT][w]);
           continue;
@@ -432,9 +432,9 @@ __global__ void __launch_bounds__(256) k_dopri_final(const T *__restrict__ y, co
           for (int j = 0; j < 8; ++j) {
             const long long xi = pt.get(x[j][w], e[j]);
             const int xh = fx_hi(xi), xl = (int)xi;
-            sb += fx_mul(xh, xl, a.fb[j]);
-            s3 += fx_mul(xh, xl, a.fe3[j]);
-            if (j == 0 || j == 4 || j == 7) sh += fx_mul(xh, xl, a.fbhh[j == 0 ? 0 : j == 4 ? 1 : 2]);
+            sb += fx_mul_sum(xh, xl, a.fb[j]);
+            s3 += fx_mul_sum(xh, xl, a.fe3[j]);
+            if (j == 0 || j == 4 || j == 7) sh += fx_mul_sum(xh, xl, a.fbhh[j == 0 ? 0 : j == 4 ? 1 : 2]);
           }
           ab[w] = pt.put(sb);
           a5[w] = pt.put(sb - sh);

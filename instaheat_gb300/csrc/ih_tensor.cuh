@@ -206,8 +206,8 @@ __device__ __forceinline__ double2 nl_sum2(const NextLin &nl, double dt, long lo
     auto add = [&](double2 v, FxCoef c) {
       const long long x = px.get(v.x, fx_exponent(v.x, c.k));
       const long long y = py.get(v.y, fx_exponent(v.y, c.k));
-      sx += fx_mul(fx_hi(x), (int)x, c);
-      sy += fx_mul(fx_hi(y), (int)y, c);
+      sx += fx_mul_sum(fx_hi(x), (int)x, c);
+      sy += fx_mul_sum(fx_hi(y), (int)y, c);
     };
 #pragma unroll 1
     for (int j = 0; j < nl.n; ++j) add(load(nl.k[j]), nl.fx[j]);
