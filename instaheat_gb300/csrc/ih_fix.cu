@@ -314,15 +314,18 @@ int fix_tables(Ctx *c) {
   IH_TRY(fx_upload_twiddles(c, &c->fx_tw[3], g.nz));
   const double qx = g.kx2 * (g.nx / 2) * (g.nx / 2), qy = g.ky2 * (g.ny / 2) * (g.ny / 2),
                qz = g.kz2 * (g.nz / 2) * (g.nz / 2);
-  c->fx_e[0] = fx_exp(g.kxmax);
-  c->fx_e[1] = fx_exp(qx);
-  c->fx_e[2] = fx_exp(g.kymax);
-  c->fx_e[3] = fx_exp(qy + qz);
-  c->fx_e[4] = fx_exp(g.kzmax);
+  const int oz = fx_odd(g.nz), ox = fx_odd(g.nx) * oz, oy = fx_odd(g.ny) * oz;
+  // of the coefficients as they are stored, with the odd parts taken out: the
+  // bits that a larger exponent leaves empty are lost to the products (144x96x96
+  // laplacian of white noise 8.4 -> 0.6 times the error of an FP64 round trip)
+  c->fx_e[0] = fx_exp(g.kxmax / ox);
+  c->fx_e[1] = fx_exp(qx / ox);
+  c->fx_e[2] = fx_exp(g.kymax / oy);
+  c->fx_e[3] = fx_exp((qy + qz) / oy);
+  c->fx_e[4] = fx_exp(g.kzmax / oz);
   for (int e : c->fx_e)  // a box whose k leave the exponent range of the passes
     if (e < -200 || e > 200) return IH_OK;
   std::vector<long long> t;
-  const int oz = fx_odd(g.nz), ox = fx_odd(g.nx) * oz, oy = fx_odd(g.ny) * oz;
   fx_coefs(t, g.nx, g.nx, g.kxu, g.kx2, c->fx_e[0], c->fx_e[1], ox, ox);
   fx_coefs(t, g.ny, g.ny, g.kyu, g.ky2, c->fx_e[2], c->fx_e[3], oy, oy);
   fx_coefs(t, g.nz, g.mz, g.kzu, g.kz2, c->fx_e[4], c->fx_e[3], oz, oy);

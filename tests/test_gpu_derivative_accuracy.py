@@ -49,8 +49,8 @@ def exact(f, length, lead):
 
 
 def errors(ctx, axis, f, wave):
-    """Relative errors of the laplacian and, of phi = f alone, of the energy
-    density (the squared gradient for the most part) of one right-hand side."""
+    """Relative errors of the laplacian and, of phi = f alone, of the pressure
+    (the squared gradient for the most part) of one right-hand side."""
     n, L = ctx.n, ctx.box
     shape = [1, 1, 1]
     shape[axis] = -1
@@ -67,8 +67,8 @@ def errors(ctx, axis, f, wave):
     lap = (d2 - kz * kz * LD(TWO_PI * TWO_PI / (L[2] * L[2])) * f.reshape(shape)) * p + np.zeros(n)
     out = [norm(ctx.field("lap").reshape(n) - lap) / norm(lap)]
     if not wave:
-        rho = d1 * d1 / 2 + phi.astype(LD) ** 2 / 2
-        out.append(norm(ctx.field("rho").reshape(n) - rho) / norm(rho))
+        p = -d1 * d1 / 6 - phi.astype(LD) ** 2 / 2
+        out.append(norm(ctx.field("pressure").reshape(n) - p) / norm(p))
     return out
 
 
@@ -83,14 +83,15 @@ def compare(gpu_mod, n, axis, kind, L=(1.0, 1.0, 1.0)):
         fixed = errors(ctx, axis, f, wave)
         ctx.set_engine(9, 0)
         fp64 = errors(ctx, axis, f, wave)
-        print(n, axis, kind, wave, fixed, fp64)
-        for a, b in zip(fixed, fp64):
-            assert a <= max(b, 2.0 ** -53)
+        # a rounding of the laplacian; of the pressure four: its squares' sum, the
+        # two products of m^2 phi^2 / 2 and the sum
+        for a, b, roundings in zip(fixed, fp64, (1, 4)):
+            assert a <= max(b, roundings * 2.0 ** -53)
     ctx.close()
 
 
 @pytest.mark.parametrize("n", [(72, 24, 24), (72, 72, 24), (144, 48, 48), (96, 96, 96)])
-@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("axis", [0, 1])
 def test_white_noise_on_radix_3_axes(gpu_mod, n, axis):
     """The odd parts of the transforms' 1 / N factors sit in the derivative
     coefficients, which have to fill their words all the same."""
