@@ -59,8 +59,21 @@ template <int L, int B> __device__ __forceinline__ int fx_row(int r) {
   const int f = (a == b) ? (r >> a) : ((r >> a) ^ (r >> b));
   return r ^ (f & 1);
 }
-// the largest word of each column of the CTA: lanes of a warp that share a
-// column, then the warps through red[warps][B]; every thread of the CTA calls
+// over each column of the CTA: lanes of a warp that share a column, then the warps
+// through red[warps][B]; every thread of the CTA calls
+template <int B, int NT>
+__device__ __forceinline__ FxSize fx_col_size(FxSize z, FxSize *red, int tid) {
+#pragma unroll
+  for (int o = B; o < 32; o <<= 1) z = fx_join_lanes(z, o);
+  if constexpr (NT == 32) return z;
+  const int lane = tid & 31;
+  if (lane < B) red[(tid >> 5) * B + lane] = z;
+  __syncthreads();
+  z = red[tid & (B - 1)];
+#pragma unroll
+  for (int w = 1; w < NT / 32; ++w) z = fx_join(z, red[w * B + (tid & (B - 1))]);
+  return z;
+}
 template <int B, int NT>
 __device__ __forceinline__ unsigned fx_col_max(unsigned m, unsigned *red, int tid) {
 #pragma unroll
@@ -80,7 +93,7 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 512 /
   constexpr int R1 = FxFac<L>::R1, R2 = FxFac<L>::R2, NT = fx_threads<L, B>();
   extern __shared__ __align__(16) unsigned char smraw[];
   fx2 *ex = reinterpret_cast<fx2 *>(smraw);  // [L][B]
-  __shared__ unsigned red[NT / 32 * B];
+  __shared__ FxSize red[NT / 32 * B];
   const int tid = threadIdx.x, b = tid & (B - 1), q = tid / B;
   const int z0 = blockIdx.x * B;
   const bool col = b < mz - z0;
@@ -89,8 +102,7 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 512 /
 #pragma unroll
   for (int n2 = 0; n2 < R2; ++n2)
     x[n2] = (col && q < R1) ? base[(long long)(q + R1 * n2) * sj] : make_double2(0.0, 0.0);
-  const unsigned m = fx_col_max<B, NT>(fx_max_in(x), red, tid);
-  const FxScale sc = fx_scale(m, fx_p<L>());
+  const FxScale sc = fx_scale(fx_col_size<B, NT>(fx_size(x), red, tid), 62, 64);
   if (q < R1) {
     fx2 v[R2];
     fx_load<true>(x, sc, v);
@@ -134,7 +146,8 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 384 /
   constexpr int R1 = FxFac<L>::R1, R2 = FxFac<L>::R2, NT = fx_threads<L, B>();
   extern __shared__ __align__(16) unsigned char smraw[];
   fx2 *ex0 = reinterpret_cast<fx2 *>(smraw), *ex1 = ex0 + L * B;  // [L][B] each
-  __shared__ unsigned red[2][NT / 32 * B];
+  __shared__ FxSize size[NT / 32 * B];
+  __shared__ unsigned red[NT / 32 * B];
   const int tid = threadIdx.x, b = tid & (B - 1), q = tid / B;
   const int z0 = blockIdx.x * B;
   const bool col = b < mz - z0;
@@ -156,8 +169,7 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 384 /
       }
     }
   }
-  const unsigned m = fx_col_max<B, NT>(fx_max_in(x), red[0], tid);
-  const FxScale sc = fx_scale(m, fx_p<L>());
+  const FxScale sc = fx_scale(fx_col_size<B, NT>(fx_size(x), size, tid), 62, 64);
   if (q < R1) {
     fx2 v[R2];
     fx_load<false>(x, sc, v);
@@ -178,7 +190,7 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 384 /
 #pragma unroll
     for (int n1 = 0; n1 < R1; ++n1) u[n1] = fx_mk(0, 0);
   }
-  const unsigned mu = fx_col_max<B, NT>(fx_max_int(u), red[1], tid);
+  const unsigned mu = fx_col_max<B, NT>(fx_max_int(u), red, tid);
   __syncthreads();  // ex0 is rewritten below (also where fx_col_max has no barrier)
   const int room = fx_room(mu, fx_p<L>() + 2);
   const FxShift sh = fx_shift_of(room);

@@ -6,18 +6,20 @@
 // addition at 60, and the product of two 64-bit fractions (the upper 64 bits,
 // one IMAD.WIDE and two IMAD.HI) at 7.5 against 1.8 DMUL.  A transform is
 // mostly additions, so the passes here hold a pencil as 64-bit integers that
-// share one exponent: the largest magnitude of the pencil is brought to 2^p,
-// the butterflies are integer additions (exact), and every multiplication by
-// a twiddle rounds to a unit of 2^-p (or 2^(2-p) after the middle twiddle) of
-// the largest value, where p is as large as the worst-case growth of the
-// transform leaves room for.  With p >= 53 the error of a pass is at or below
-// that of the same pass in FP64, whose additions each round to 2^-53 of
-// partial sums that grow with the transform.
+// share one exponent, the butterflies are integer additions (exact), and every
+// multiplication by a twiddle rounds to a unit.  The exponent follows from the
+// pencil's sum of magnitudes (FxSize), which bounds every value on the way,
+// whatever the pencil holds: white noise has its units where the largest
+// value's worst growth would put them, a pencil with one dominant value 2^-57 of
+// that value.  Errors of a pass (2-norm) are 0.3 to 0.6 of those in FP64 for
+// white noise, a spike, a falling or a single-wave spectrum of 8 to 512 points.
 //
-// Growth: |Re|, |Im| <= 2^p at the input of an L-point transform bound every
-// output by L sqrt(2) 2^p; the multiplication by a table twiddle keeps the
-// upper 64 bits of a product with a Q62 fraction, a factor 1/4, so the bound
-// is L sqrt(2) 2^(p - 2) < 2^63 for p = 64 - log2 L.
+// Growth: sqrt(2) S bounds the sum of the magnitudes.  The part of it that one
+// thread holds bounds its first DFT, whose outputs are rotated (x + y: a factor
+// sqrt(2)), so that part's S stays below 2^62; the multiplication by a table twiddle
+// keeps the upper 64 bits of a product with a Q62 fraction, a factor 1/4, so that
+// the second DFT is bounded by sqrt(2) S / 4, its inner rotations by S / 2, and S
+// may be 2^64.
 #pragma once
 #include "ih_internal.cuh"
 #include "ih_fftcore.cuh"
@@ -222,10 +224,59 @@ __device__ __forceinline__ void fx_dft(fx2 (&v)[R]) {
 }
 
 // ---------------------------------------------------------------------------
-// FP64 <-> fixed point of one pencil.  m: the largest |high word| of its
-// components (fx_max_in).
+// FP64 <-> fixed point of one pencil
 __device__ __forceinline__ unsigned fx_absbits(double a) {
   return (unsigned)__double2hiint(a) & 0x7fffffffu;
+}
+// Size of a pencil, an upper bound of its sum of magnitudes over sqrt(2): what one
+// thread holds is below 2^(e - 1022), the pencil at most s 2^(e - 1042); s = 0 if
+// every value is 0, e = kFxBad if one is an Inf or NaN.  Groups of up to four values
+// count with their largest component (each value by itself would cost a tenth of a
+// pass in time and hardly change the bound).
+constexpr int kFxBad = 4096;
+struct FxSize {
+  int e;
+  unsigned s;
+};
+template <int R>
+__device__ __forceinline__ FxSize fx_size(const double2 (&x)[R]) {
+  constexpr int G = R % 4 == 0 ? 4 : (R % 3 == 0 ? 3 : R), NG = R / G;
+  unsigned m[NG], all = 0, low = 0;
+#pragma unroll
+  for (int g = 0; g < NG; ++g) {
+    m[g] = 0;
+#pragma unroll
+    for (int i = g; i < R; i += NG) {
+      m[g] = max(m[g], max(fx_absbits(x[i].x), fx_absbits(x[i].y)));
+      low |= (unsigned)(__double2loint(x[i].x) | __double2loint(x[i].y));
+    }
+    all = max(all, m[g]);
+  }
+  // a component is below (upper bits of its mantissa + 1) 2^(exponent - 1043)
+  const unsigned E = all >> 20;
+  unsigned s = NG;
+#pragma unroll
+  for (int g = 0; g < NG; ++g)
+    s += __funnelshift_rc((m[g] & 0xfffffu) | 0x100000u, 0u, E - (m[g] >> 20));
+  s *= G;
+  const int n = 32 - __clz((int)s);  // 2^20 < s < 2^n
+  FxSize z;
+  z.e = E == 2047 ? kFxBad : (int)E + n - 21;
+  z.s = (all | low) ? (s >> (n - 20)) + 1 : 0;
+  return z;
+}
+__device__ __forceinline__ FxSize fx_join(FxSize a, FxSize b) {
+  auto up = [](unsigned s, int d) { return (s + ((1u << d) - 1)) >> d; };
+  FxSize z;
+  z.e = max(a.e, b.e);
+  z.s = up(a.s, min(z.e - a.e, 31)) + up(b.s, min(z.e - b.e, 31));
+  return z;
+}
+__device__ __forceinline__ FxSize fx_join_lanes(FxSize z, int o) {
+  FxSize b;
+  b.e = __shfl_xor_sync(0xffffffffu, z.e, o);
+  b.s = __shfl_xor_sync(0xffffffffu, z.s, o);
+  return fx_join(z, b);
 }
 struct FxScale {
   int in;       // exponent added to the inputs: integer = round(x 2^in)
@@ -233,19 +284,22 @@ struct FxScale {
   bool slow;    // the pencil needs the factors below
   double pre, post;
 };
-// The common case (largest value 2^-323 to 2^37) takes exponents for which
+// The integers of a pencil of size z: a thread's below 2^bp in all, the pencil's
+// below 2^bs.
+// The common case (e for values of 2^-323 to 2^37) takes exponents for which
 // adding `in` to the exponent field of any component (zeros and subnormals
 // included) stays a finite number, and for which the exponents of products of
 // two pencils stay in range; other pencils are brought there by an exact power
 // of two, and a pencil with an Inf or NaN comes out as NaN.
-__device__ __forceinline__ FxScale fx_scale(unsigned m, int p) {
+__device__ __forceinline__ FxScale fx_scale(FxSize z, int bp, int bs) {
   FxScale s;
-  int E = (int)(m >> 20);
+  int E = z.e;
+  const int bits = min(bp, bs - (12 - __clz((int)z.s)));  // z.s < 2^(32 - clz)
   s.slow = E < 700 || E > 1060;
   s.pre = s.post = 1.0;
   if (s.slow) {
     int d;  // exponent taken off: values of the order of one, or as near as a factor comes
-    if (E == 2047) {
+    if (E == kFxBad) {
       d = 0;
       E = 1023;
     } else {
@@ -254,13 +308,13 @@ __device__ __forceinline__ FxScale fx_scale(unsigned m, int p) {
     }
     s.pre = __hiloint2double((1023 - d) << 20, 0);
     s.post = __hiloint2double((1023 + d) << 20, 0);
-    if ((m >> 20) == 2047) {
+    if (z.e == kFxBad) {
       s.pre = 0.0;
       s.post = __longlong_as_double(0x7ff8000000000000LL);
     }
-    if (m == 0) s.post = 0.0;  // all zero
+    if (z.s == 0) s.post = 0.0;  // all zero
   }
-  s.in = p + 1022 - E;
+  s.in = bits + 1022 - E;
   s.out = -s.in;
   return s;
 }
@@ -306,16 +360,6 @@ template <bool BITS>
 __device__ __forceinline__ double fx_out(long long v, int e) {
   return BITS ? fx_out_bits(v, e) : fx_out_pipe(v, e);
 }
-template <int R>
-__device__ __forceinline__ unsigned fx_max_in(const double2 (&x)[R]) {
-  unsigned m = 0, low = 0;
-#pragma unroll
-  for (int i = 0; i < R; ++i) {
-    m = max(m, max(fx_absbits(x[i].x), fx_absbits(x[i].y)));
-    low |= (unsigned)(__double2loint(x[i].x) | __double2loint(x[i].y));
-  }
-  return low ? m | 1u : m;  // 0 only where every value is 0
-}
 template <bool BITS, int R>
 __device__ __forceinline__ void fx_load(double2 (&x)[R], const FxScale &s, fx2 (&v)[R]) {
   if (s.slow) {
@@ -353,6 +397,22 @@ __device__ __forceinline__ unsigned fx_max_int(const fx2 (&v)[R]) {
 }
 __device__ __forceinline__ int fx_room(unsigned maxhi, int bits) {
   return bits - (64 - __clz(maxhi));  // |v| < 2^(64 - clz(maxhi))
+}
+// The same for integers: the sum of |Re| + |Im| over what a thread holds, in
+// units of 2^38, rounded up; and the shift that makes room for a transform, from the
+// largest such sum p and all of them together s (units of 2^unit)
+template <int R>
+__device__ __forceinline__ float fx_sum_int(const fx2 (&v)[R]) {
+  unsigned s = R;
+#pragma unroll
+  for (int i = 0; i < R; ++i) s += (fx_abshi(v[i].x) + fx_abshi(v[i].y)) >> 6;
+  return __uint2float_ru(s);
+}
+__device__ __forceinline__ int fx_float_exp(float f) {  // f < 2^(this), f > 0
+  return (__float_as_int(f) >> 23) - 126;
+}
+__device__ __forceinline__ int fx_room_sum(float p, float s, int unit, int bp, int bs) {
+  return min(bp - fx_float_exp(p), bs - fx_float_exp(s)) - unit;
 }
 struct FxShift {
   int l, r;

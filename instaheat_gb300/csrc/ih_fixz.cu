@@ -33,13 +33,17 @@ struct NumFx {
     return fx_mk(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
   }
 };
-template <int H> struct FxZG : ZRow<NumFx, H> {
-  // c2r: the split's 1/4 and the transform's growth H sqrt 2; r2c: the split
-  // adds two values and the last bit of growth
-  static constexpr int lg = clog2(2 * H - 1);  // log2 H, rounded up
-  static constexpr int pc = 64 - lg < 58 ? 64 - lg : 58;
-  static constexpr int pr = 63 - lg < 58 ? 63 - lg : 58;
-};
+template <int H> struct FxZG : ZRow<NumFx, H> {};
+// bits for a row's integers (fx_scale).  r2c: the split adds two outputs, each below
+// sqrt(2) S / 4.  c2r: the split comes first and rotates the sum of two values, each
+// in one thread's part
+constexpr int kFxRealP = 62, kFxRealS = 63, kFxHalfP = 61, kFxHalfS = 64;
+template <int B>
+__device__ __forceinline__ FxSize fx_row_size(FxSize z) {
+#pragma unroll
+  for (int o = 1; o < B; o <<= 1) z = fx_join_lanes(z, o);
+  return z;
+}
 constexpr int kFxWarps = 4;
 
 // Real rows -> half spectra.  The row's first value is taken off before the
@@ -73,7 +77,7 @@ __global__ void __launch_bounds__(32 * kFxWarps) k_fx_zr2c(
     x[i].x -= x0;
     x[i].y -= x0;
   }
-  const FxScale sc = fx_scale(zrow_max<FxZG<H>::B>(fx_max_in(x)), G::pr);
+  const FxScale sc = fx_scale(fx_row_size<B>(fx_size(x)), kFxRealP, kFxRealS);
   fx2 v[A];
   fx_load<true>(x, sc, v);
   zrow_forward<NumFx, H>(v, t, &xs[warp][grp * G::X], twh);
@@ -105,8 +109,10 @@ __device__ __forceinline__ FxScale fx_z_load(double2 (&x)[FxZG<H>::A], double2 x
                                              fx2 (&v)[FxZG<H>::A], fx2 &vH) {
   double2 h[1] = {xH};
   fx2 u[1];
-  const FxScale sc =
-      fx_scale(zrow_max<FxZG<H>::B>(max(fx_max_in(x), fx_max_in(h))), FxZG<H>::pc);
+  FxSize z = fx_size(x), zH = fx_size(h);
+  zH.e -= zH.s == 0 ? kFxBad : 0;  // (zero on the other lanes: no part of the size)
+  z = fx_join(z, zH);
+  const FxScale sc = fx_scale(fx_row_size<FxZG<H>::B>(z), kFxHalfP, kFxHalfS);
   fx_load<BITS>(x, sc, v);
   fx_load<BITS>(h, sc, u);
   vH = u[0];
@@ -232,7 +238,18 @@ template <int H>
 __device__ __forceinline__ void fx_z_product(fx2 (&v)[FxZG<H>::A], int e, bool slow, double post,
                                              const FxZIn &in, const FxZLane &ln, double2 *spec) {
   constexpr int A = FxZG<H>::A, B = FxZG<H>::B;
-  e += 4 - fx_z_norm<H>(v, FxZG<H>::pr);
+  float p = fx_sum_int(v), s = p;
+#pragma unroll
+  for (int o = 1; o < B; o <<= 1) {
+    p = fmaxf(p, __shfl_xor_sync(0xffffffffu, p, o));
+    s = __fadd_ru(s, __shfl_xor_sync(0xffffffffu, s, o));
+  }
+  // (the sums themselves, without the sqrt(2): a bit more than kFxRealS)
+  const int room = fx_room_sum(p, s, 38, 62, 64);
+  const FxShift sh = fx_shift_of(room);
+#pragma unroll
+  for (int m = 0; m < A; ++m) v[m] = fx_shift(v[m], sh);
+  e += 4 - room;
   zrow_forward<NumFx, H>(v, ln.t, ln.xch, in.twh);
   fx2 xH;
   zrow_r2c_post<NumFx, H>(v, ln.t, ln.gbase, in.twz, xH);
