@@ -4,6 +4,7 @@
 // in memory stay FP64 in the layouts of the other engines (ih_fft.cu); each
 // pass converts a pencil on its way in and out of registers.
 #include <math.h>
+#include <string.h>
 #include <vector>
 #include "ih_internal.cuh"
 #include "ih_fftcore.cuh"
@@ -40,9 +41,6 @@ template <> struct FxFac<144> { static constexpr int R1 = 12, R2 = 12; };
 template <> struct FxFac<192> { static constexpr int R1 = 16, R2 = 12; };
 template <> struct FxFac<288> { static constexpr int R1 = 12, R2 = 24; };
 template <> struct FxFac<384> { static constexpr int R1 = 16, R2 = 24; };
-template <int L> __host__ __device__ constexpr int fx_p() {  // log2 rounded up
-  return 64 - clog2(2 * L - 1) < 59 ? 64 - clog2(2 * L - 1) : 59;
-}
 template <int L> __host__ __device__ constexpr int fx_maxr() {
   return FxFac<L>::R1 > FxFac<L>::R2 ? FxFac<L>::R1 : FxFac<L>::R2;
 }
@@ -74,17 +72,31 @@ __device__ __forceinline__ FxSize fx_col_size(FxSize z, FxSize *red, int tid) {
   for (int w = 1; w < NT / 32; ++w) z = fx_join(z, red[w * B + (tid & (B - 1))]);
   return z;
 }
+// the largest sum of a thread and the sum of all (fx_room_sum), of two pencils
 template <int B, int NT>
-__device__ __forceinline__ unsigned fx_col_max(unsigned m, unsigned *red, int tid) {
+__device__ __forceinline__ void fx_col_sums(float2 &p, float2 &s, float4 *red, int tid) {
+  auto join = [&](float4 o) {
+    p.x = fmaxf(p.x, o.x);
+    p.y = fmaxf(p.y, o.y);
+    s.x = __fadd_ru(s.x, o.z);
+    s.y = __fadd_ru(s.y, o.w);
+  };
 #pragma unroll
-  for (int o = B; o < 32; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if constexpr (NT == 32) return m;
+  for (int o = B; o < 32; o <<= 1) {
+    float4 b;
+    b.x = __shfl_xor_sync(0xffffffffu, p.x, o);
+    b.y = __shfl_xor_sync(0xffffffffu, p.y, o);
+    b.z = __shfl_xor_sync(0xffffffffu, s.x, o);
+    b.w = __shfl_xor_sync(0xffffffffu, s.y, o);
+    join(b);
+  }
+  if constexpr (NT == 32) return;
   const int lane = tid & 31;
-  if (lane < B) red[(tid >> 5) * B + lane] = m;
+  if (lane < B) red[(tid >> 5) * B + lane] = make_float4(p.x, p.y, s.x, s.y);
   __syncthreads();
+  p = s = make_float2(0.0f, 0.0f);
 #pragma unroll
-  for (int w = 0; w < NT / 32; ++w) m = max(m, red[w * B + (tid & (B - 1))]);
-  return m;
+  for (int w = 0; w < NT / 32; ++w) join(red[w * B + (tid & (B - 1))]);
 }
 
 template <int L, int B, int S>
@@ -130,24 +142,27 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 512 /
 // Derivative round trips along x or y (see k_fft_xy_rt): d1 = IFFT(i k FFT(Z))
 // / (L nz), d2 = IFFT(-k^2 FFT(Z)) / (L nz).  c1, c2: k / 2^e1 and -k^2 / 2^e2
 // in Q62 (first derivative 0 on the Nyquist index).  ACC (the y round trip):
-// the coefficient of d2 takes -kz^2 too (cz, at the scale of c2), so that d2
-// is the y and z part of the laplacian, and the x part in out1 is added.
+// the coefficient of d2 takes -kz^2 too (cz / 2^ez in Q62, brought to a common
+// exponent with c2 for each column), so that d2 is the y and z part of the
+// laplacian, and the x part in out1 is added.
 // At 256^3: 344 us a round trip against 1359 us on the FP64 pipe, 128^3 53 us
 // against 178.  Inputs convert on the FP64 pipe, outputs (two per input) on the
 // integer pipe: 375 us with both on the former, 388 on the latter.
-// Between the transforms the spectrum is brought to 2 bits above the inverse
-// transform's p (the coefficients take 2), so no precision is lost whatever
-// its size.
+// Between the transforms each product k X, k^2 X is brought to the size that the
+// inverse transform has room for: a pencil whose power lies at small k (a k^-2
+// spectrum, a single wave) fills little of the coefficients' range, and with the
+// spectrum's size alone (in use before) its derivatives were up to 35 times as
+// far off as an FP64 round trip's at 512 points; now nowhere further.
 template <int L, int B, bool ACC>
 __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 384 / fx_threads<L, B>() : 1) k_fx_rt(
     const double2 *__restrict__ in, double2 *__restrict__ out0, double2 *out1, long long sj,
     long long so, int mz, FxTab tw, const long long *__restrict__ c1,
-    const long long *__restrict__ c2, const long long *__restrict__ cz, int e1, int e2) {
+    const long long *__restrict__ c2, const long long *__restrict__ cz, int e1, int e2, int ez) {
   constexpr int R1 = FxFac<L>::R1, R2 = FxFac<L>::R2, NT = fx_threads<L, B>();
   extern __shared__ __align__(16) unsigned char smraw[];
   fx2 *ex0 = reinterpret_cast<fx2 *>(smraw), *ex1 = ex0 + L * B;  // [L][B] each
   __shared__ FxSize size[NT / 32 * B];
-  __shared__ unsigned red[NT / 32 * B];
+  __shared__ float4 red[NT / 32 * B];
   const int tid = threadIdx.x, b = tid & (B - 1), q = tid / B;
   const int z0 = blockIdx.x * B;
   const bool col = b < mz - z0;
@@ -180,20 +195,22 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 384 /
           k2 == 0 ? fx_quarter(v[k2]) : fx_cmul<-1>(v[k2], fx_tw(tw, q * k2));
   }
   __syncthreads();
-  fx2 u[R1];
-  if (q < R2) {
-#pragma unroll
-    for (int n1 = 0; n1 < R1; ++n1) u[n1] = ex0[fx_row<L, B>(n1 * R2 + q) * B + b];
-    fx_dft<R1, -1>(u);  // u[k1] = X[q + R2 k1]
-    if (z0 + b + q == 0) u[0] = fx_mk(0, 0);  // the constant: both coefficients are 0
-  } else {
-#pragma unroll
-    for (int n1 = 0; n1 < R1; ++n1) u[n1] = fx_mk(0, 0);
+  int zshift = 0;
+  long long z2 = 0;
+  if (ACC) {  // the column's -kz^2; c2 >> zshift and z2 at the exponent e2
+    const long long v = __ldg(cz + min(z0 + b, mz - 1));
+    if (v != 0) {
+      const int up = max(__clzll((unsigned long long)-v) - 2, 0);
+      const int e = max(e2, ez - up) + 1;
+      zshift = min(e - e2, 63);
+      z2 = (v << up) >> min(e - (ez - up), 63);
+      e2 = e;
+    }
   }
-  const unsigned mu = fx_col_max<B, NT>(fx_max_int(u), red, tid);
-  __syncthreads();  // ex0 is rewritten below (also where fx_col_max has no barrier)
-  const int room = fx_room(mu, fx_p<L>() + 2);
-  const FxShift sh = fx_shift_of(room);
+  auto coef = [&](int o, int k1) {
+    const long long c = __ldg((o ? c2 : c1) + q + R2 * k1);
+    return ACC && o ? (c >> zshift) + z2 : c;
+  };
   // the spectrum waits in the thread's own slots of ex1 between the two
   // inverse transforms (in registers it would halve the resident CTAs).  From 16
   // points a thread on the two share their code: unrolled, the kernel waited for
@@ -201,21 +218,38 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 384 /
   // 33.0 -> 31.6, 256^3 351 -> 344; 64^3 the other way, 13.5 -> 14.3).
   constexpr int kShare = R1 >= 16 || R2 >= 16 || R1 % 3 == 0 ? 1 : 2;
   auto slot = [&](int k1) { return (k1 * R2 + q) * B + b; };
+  fx2 u[R1];
+  float2 p = make_float2(0.0f, 0.0f);  // the sizes of the two products, units of 4
   if (q < R2) {
 #pragma unroll
-    for (int k1 = 0; k1 < R1; ++k1) ex1[slot(k1)] = fx_shift(u[k1], sh);
+    for (int n1 = 0; n1 < R1; ++n1) u[n1] = ex0[fx_row<L, B>(n1 * R2 + q) * B + b];
+    fx_dft<R1, -1>(u);  // u[k1] = X[q + R2 k1]
+    if (z0 + b + q == 0) u[0] = fx_mk(0, 0);  // the constant: both coefficients are 0
+    unsigned long long p1 = 0, p2 = 0;
+#pragma unroll
+    for (int k1 = 0; k1 < R1; ++k1) {
+      // (|Re| + |Im| <= 2^63, a coefficient 2^62: 16 products fit)
+      const unsigned long long t = ((fx_abshi(u[k1].x) + fx_abshi(u[k1].y)) >> 2) + 1;
+      p1 += t * (fx_abshi(coef(0, k1)) + 1);
+      p2 += t * (fx_abshi(coef(1, k1)) + 1);
+      ex1[slot(k1)] = u[k1];
+    }
+    p = make_float2(__ull2float_ru(p1), __ull2float_ru(p2));
   }
+  float2 s = p;
+  fx_col_sums<B, NT>(p, s, red, tid);
+  __syncthreads();  // ex0 is rewritten below (also where fx_col_sums has no barrier)
+  const int room[2] = {fx_room_sum(p.x, s.x, 2, 62, 64), fx_room_sum(p.y, s.y, 2, 62, 64)};
 #pragma unroll kShare
   for (int o = 0; o < 2; ++o) {
     if (q < R2) {
-      const long long *cc = o ? c2 : c1;
-      const long long z2 = ACC && o ? __ldg(cz + min(z0 + b, mz - 1)) : 0;
+      const int up = max(o ? room[1] : room[0], 0), down = up - (o ? room[1] : room[0]);
 #pragma unroll
       for (int k1 = 0; k1 < R1; ++k1) {
         const fx2 v = ex1[slot(k1)];
-        const long long c = __ldg(cc + q + R2 * k1) + z2;
+        const long long c = coef(o, k1) >> down;
         const int ch = fx_hi(c), cl = (int)c;
-        const long long cx = fx_mul(v.x, ch, cl), cy = fx_mul(v.y, ch, cl);
+        const long long cx = fx_mul(v.x, ch, cl) << up, cy = fx_mul(v.y, ch, cl) << up;
         u[k1] = o ? fx_mk(cx, cy) : fx_mk(-cy, cx);  // -k^2 X, i k X
       }
       fx_dft<R1, +1>(u);
@@ -232,7 +266,7 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 384 /
   __syncthreads();
   if (q < R1) {
     // forward twiddle, coefficient and inverse twiddle took 2 bits each
-    const int e = sc.out + 6 - room;
+    const int e = sc.out + 6;
 #pragma unroll kShare
     for (int o = 0; o < 2; ++o) {
       const fx2 *ex = o ? ex1 : ex0;
@@ -245,7 +279,7 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 384 /
 #pragma unroll
         for (int n2 = 0; n2 < R2; ++n2) {
           double2 *d = dst + (long long)(q + R1 * n2) * sj;
-          double2 r = fx_store<true>(v[n2], e + (o ? e2 : e1), sc);
+          double2 r = fx_store<true>(v[n2], e + (o ? e2 - room[1] : e1 - room[0]), sc);
           if (ACC && o == 1) {
             const double2 a = *d;
             r.x += a.x;
@@ -295,15 +329,16 @@ static int fx_upload_twiddles(Ctx *c, void **dst, int L) {
 // derivative coefficients of one axis: c1[k] = k_f / (odd 2^e1) (0 on Nyquist),
 // c2[k] = -k_f^2 / (odd 2^e2) in Q62, k folded to [-L/2, L/2); odd: the odd part
 // of the transforms' 1 / N factors, whose power of two goes into the exponents
-static void fx_coefs(std::vector<long long> &t, int L, int count, double unit, double unit2, int e1,
-                     int e2, int odd1, int odd2) {
-  for (int k = 0; k < count; ++k) {
+static void fx_coefs1(std::vector<long long> &t, int L, double unit, int e1, int odd) {
+  for (int k = 0; k < L; ++k) {
     const int f = k > L / 2 ? k - L : k;
-    t.push_back(2 * k == L ? 0 : llrintl(ldexpl((long double)unit * f / odd1, 62 - e1)));
+    t.push_back(2 * k == L ? 0 : llrintl(ldexpl((long double)unit * f / odd, 62 - e1)));
   }
+}
+static void fx_coefs2(std::vector<long long> &t, int L, int count, double unit2, int e2, int odd) {
   for (int k = 0; k < count; ++k) {
     const int f = k > L / 2 ? L - k : k;
-    t.push_back(-llrintl(ldexpl((long double)unit2 * f * f / odd2, 62 - e2)));
+    t.push_back(-llrintl(ldexpl((long double)unit2 * f * f / odd, 62 - e2)));
   }
 }
 static int fx_odd(int n) {
@@ -333,14 +368,22 @@ int fix_tables(Ctx *c) {
   c->fx_e[0] = fx_exp(g.kxmax / ox);
   c->fx_e[1] = fx_exp(qx / ox);
   c->fx_e[2] = fx_exp(g.kymax / oy);
-  c->fx_e[3] = fx_exp((qy + qz) / oy);
-  c->fx_e[4] = fx_exp(g.kzmax / oz);
+  c->fx_e[3] = fx_exp(qy / oy);
+  c->fx_e[4] = fx_exp(qz / oy);
   for (int e : c->fx_e)  // a box whose k leave the exponent range of the passes
     if (e < -200 || e > 200) return IH_OK;
   std::vector<long long> t;
-  fx_coefs(t, g.nx, g.nx, g.kxu, g.kx2, c->fx_e[0], c->fx_e[1], ox, ox);
-  fx_coefs(t, g.ny, g.ny, g.kyu, g.ky2, c->fx_e[2], c->fx_e[3], oy, oy);
-  fx_coefs(t, g.nz, g.mz, g.kzu, g.kz2, c->fx_e[4], c->fx_e[3], oz, oy);
+  fx_coefs1(t, g.nx, g.kxu, c->fx_e[0], ox);
+  fx_coefs2(t, g.nx, g.nx, g.kx2, c->fx_e[1], ox);
+  fx_coefs1(t, g.ny, g.kyu, c->fx_e[2], oy);
+  fx_coefs2(t, g.ny, g.ny, g.ky2, c->fx_e[3], oy);
+  for (int k = 0; k < g.mz; ++k) {  // d/dz's kz / nz: FP64
+    const double f = (double)((long double)g.kzu * k / g.nz);
+    long long bits;
+    memcpy(&bits, &f, sizeof f);
+    t.push_back(bits);
+  }
+  fx_coefs2(t, g.nz, g.mz, g.kz2, c->fx_e[4], oy);
   IH_CUDA(c, cudaMalloc(&c->fx_coef, sizeof(long long) * t.size()));
   c->dev_bytes += sizeof(long long) * t.size();
   IH_CUDA(c, cudaMemcpy(c->fx_coef, t.data(), sizeof(long long) * t.size(),
@@ -418,13 +461,14 @@ struct FxRT {
                     *cz = cy + 2 * g.ny;
     const long long *c1 = axis == 0 ? cx : cy;
     const int scale = fx_twos(L) + fx_twos(g.nz);  // 1 / (L nz), its powers of two
-    const int e1 = c->fx_e[2 * axis] - scale, e2 = c->fx_e[2 * axis + 1] - scale;
+    const int e1 = c->fx_e[2 * axis] - scale, e2 = c->fx_e[2 * axis + 1] - scale,
+              ez = c->fx_e[4] - scale;
     const size_t sm = sizeof(fx2) * L * B * 2;
     const dim3 grid((g.mz + B - 1) / B, outer);
     auto kf = axis == 1 ? k_fx_rt<L, B, true> : k_fx_rt<L, B, false>;
     want_smem(kf, sm);
     kf<<<grid, fx_threads<L, B>(), sm, c->stream>>>(z, d1, d2, sj, so, g.mz, tw, c1, c1 + L,
-                                                    cz + g.mz, e1, e2);
+                                                    cz + g.mz, e1, e2, ez);
     return IH_OK;
   }
 };

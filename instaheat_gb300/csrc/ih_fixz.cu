@@ -168,8 +168,7 @@ __global__ void __launch_bounds__(32 * kFxWarps) k_fx_zc2r(
 struct FxZIn {
   const double2 *d4;  // d/dx, d/dy, (d/dz), laplacian, (Z) in (x, y, kz)
   long long dstride;
-  const long long *ckz;
-  int ekz, lognz;
+  const double *ckz;  // kz / nz
   int zsrc;  // d/dz from Z in slot 4
   FxTab twh, twz;
 };
@@ -186,27 +185,20 @@ __device__ __forceinline__ int fx_z_deriv(const FxZIn &in, int a, const FxZLane 
   constexpr int A = FxZG<H>::A, B = FxZG<H>::B;
   double2 x[A], xH;
   fx2 vH;
-  int e;
   fx_z_fetch<H>(in.d4 + (in.zsrc && a == 2 ? 4 : a) * in.dstride + ln.row * (H + 1), ln.t, ln.valid,
                 x, xH);
-  if (in.zsrc && a == 2) {  // i kz Z / nz: the constant drops out
-    if (ln.t == 0) x[0] = make_double2(0.0, 0.0);
-    sc = fx_z_load<H, false>(x, xH, v, vH);
+  if (in.zsrc && a == 2) {  // i kz Z / nz, in FP64: the row's size is that of the product
 #pragma unroll
     for (int m = 0; m < A; ++m) {
-      const long long c = __ldg(in.ckz + ln.t + B * m);
-      const int ch = fx_hi(c), cl = (int)c;
-      v[m] = fx_mk(-fx_mul(v[m].y, ch, cl), fx_mul(v[m].x, ch, cl));
+      const double f = __ldg(in.ckz + ln.t + B * m);
+      x[m] = make_double2(-x[m].y * f, x[m].x * f);
     }
-    vH = fx_mk(0, 0);  // zero on the Nyquist index
-    e = sc.out + 2 + in.ekz - in.lognz;
-  } else {
-    sc = fx_z_load<H, false>(x, xH, v, vH);
-    e = sc.out;
+    xH = make_double2(0.0, 0.0);  // zero on the Nyquist index
   }
+  sc = fx_z_load<H, false>(x, xH, v, vH);
   zrow_c2r_prep<NumFx, H>(v, vH, ln.t, ln.gbase, in.twz);
   zrow_inverse<NumFx, H>(v, ln.t, ln.xch, in.twh);
-  return e + 4;
+  return sc.out + 4;
 }
 // bring a row to 2^bits; the exponent taken off
 template <int H>
@@ -558,9 +550,8 @@ struct FxZRhs {
       c->err = "grid too large for the RHS partial-sum buffer";
       return IH_ERR_ARG;
     }
-    const long long *cz = (const long long *)c->fx_coef + 2 * g.nx + 2 * g.ny;
-    const FxZIn in{d4, g.M, cz, c->fx_e[4], fx_twos(g.nz), zsrc, fx_tab(c->fx_tw[2], H),
-                   fx_tab(c->fx_tw[3], 2 * H)};
+    const double *kz = (const double *)c->fx_coef + 2 * g.nx + 2 * g.ny;
+    const FxZIn in{d4, g.M, kz, zsrc, fx_tab(c->fx_tw[2], H), fx_tab(c->fx_tw[3], 2 * H)};
     const FxZOut out{yfl, p, rho, g.N};
     c->z_blocks = (int)nblk;
     if constexpr (kFxZCo<H>) {

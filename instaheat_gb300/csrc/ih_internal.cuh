@@ -259,7 +259,7 @@ struct Ctx {
   // (ih_fix.cu).  fx_on: the passes that run so (bits as the passes of
   // ih_fft_set_engine: 0 x, 1 y, 3 / 4 the round trips, 6 the z passes);
   // fx_tw: twiddles of x, y, h, nz; fx_coef: derivative coefficients;
-  // fx_e: their exponents (x first, x second, y first, y and z second, z first)
+  // fx_e: their exponents (x first, x second, y first, y second, z second)
   int fx_on = 0, fx_can = 0;    // fx_can: the passes that have the form on this grid
   void *fx_tw[4] = {};
   void *fx_coef = nullptr;

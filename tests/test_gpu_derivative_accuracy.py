@@ -96,3 +96,28 @@ def test_white_noise_on_radix_3_axes(gpu_mod, n, axis):
     """The odd parts of the transforms' 1 / N factors sit in the derivative
     coefficients, which have to fill their words all the same."""
     compare(gpu_mod, n, axis, "white")
+
+
+@pytest.mark.parametrize("kind", ["low", "k^-2", "wave"])
+@pytest.mark.parametrize("n,axis", [((256, 8, 8), 0), ((256, 256, 8), 1), ((512, 8, 8), 0),
+                                    ((512, 512, 8), 1), ((144, 48, 48), 0), ((144, 144, 48), 1),
+                                    ((288, 24, 24), 0), ((288, 288, 24), 1), ((96, 96, 96), 2),
+                                    ((128, 128, 128), 2), ((192, 192, 192), 2)])
+def test_power_at_small_wave_numbers(gpu_mod, n, axis, kind):
+    """Pencils whose derivatives come from a few small k: the products k X are
+    small beside the spectrum's and the coefficients' largest values."""
+    compare(gpu_mod, n, axis, kind)
+
+
+@pytest.mark.parametrize("n", [(72, 24, 24), (72, 72, 24), (96, 96, 96), (256, 8, 8), (64, 64, 64)])
+def test_fields_of_z_alone(gpu_mod, n):
+    """k_x = k_y = 0: one product in a pencil, far below the largest coefficient."""
+    compare(gpu_mod, n, 2, "white")
+
+
+@pytest.mark.parametrize("axis", [0, 1])
+@pytest.mark.parametrize("L", [(1.0, 100.0, 0.01), (1.0, 1.0, 0.001)])
+def test_elongated_boxes(gpu_mod, L, axis):
+    """k_z beyond k_y by orders of magnitude: the columns of small k_z keep
+    their own exponent."""
+    compare(gpu_mod, (64, 64, 64), axis, "low", L)
