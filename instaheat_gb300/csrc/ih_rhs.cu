@@ -24,6 +24,7 @@
 #include "ih_tensor.cuh"
 #include "ih_fftcore.cuh"
 #include "ih_fix.cuh"
+#include "ih_fork.cuh"
 
 namespace ih {
 
@@ -1369,10 +1370,8 @@ static int rhs_t(Ctx *c, Vec &y, Vec &k, int filter, int output, const Vec *smry
   // in one stream.
   const bool fork = output != 1 && !c->prof_on && c->p.enable_gw;
   const cudaStream_t st = fork ? c->side : c->stream;
-  if (fork) {
-    IH_CUDA(c, cudaEventRecord(c->fork[0], c->stream));
-    IH_CUDA(c, cudaStreamWaitEvent(c->side, c->fork[0], 0));
-  }
+  Fork beside;
+  if (fork) IH_CUDA(c, beside.start(c->stream, c->side, c->fork[0], c->fork[2]));
   k_reduce_finish<<<1, 256, 0, st>>>(c->partials, c->z_blocks, g, y.sc, k.sc, c->rs, c->mixed);
   IH_TRY(check_launch(c, "k_reduce_finish"));
   if (fork) IH_CUDA(c, cudaEventRecord(c->fork[1], c->side));
@@ -1388,7 +1387,6 @@ static int rhs_t(Ctx *c, Vec &y, Vec &k, int filter, int output, const Vec *smry
   prof_end(c, KK_UPDATE_PHI_PSI,
            ((nl.skip_pos ? 8.0 : 10.0) + (next ? 4.0 * (next->n + 2) : 0.0)) * N * sizeof(T));
   IH_TRY(check_launch(c, "k_update_phi_psi"));
-  if (fork) IH_CUDA(c, cudaEventRecord(c->fork[2], c->side));
   // 5. tensor modes
   if (c->p.enable_gw) {
     auto join = [&]() {  // the equation of motion reads the scalars
@@ -1415,7 +1413,7 @@ static int rhs_t(Ctx *c, Vec &y, Vec &k, int filter, int output, const Vec *smry
       IH_TRY(tensor_last_pass(c, spec, yfl, kfl, k.sc, next));
     }
   }
-  if (fork) IH_CUDA(c, cudaStreamWaitEvent(c->stream, c->fork[2], 0));
+  IH_CUDA(c, beside.join());
   if (next) {
     k_next_sc<<<1, 32, 0, c->stream>>>(*next, k.sc, y.sc);
     IH_TRY(check_launch(c, "k_next_sc"));
