@@ -205,7 +205,7 @@ static int create(const ih_params *p, Ctx *c) {
   IH_TRY(alloc_vec(c, c->ytmp));
   IH_TRY(alloc_vec(c, c->k[1]));
   IH_TRY(mask_init(c, c->mask));
-  if (!c->mixed) IH_TRY(tensor_table(c));
+  if (!c->mixed && p->enable_gw) IH_TRY(tensor_table(c));
   IH_CUDA(c, cudaStreamSynchronize(c->stream));
   return IH_OK;
 }

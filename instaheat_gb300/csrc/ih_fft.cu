@@ -2669,8 +2669,10 @@ static int autotune_t(Ctx *c) {
     }
   }
   // the last x pass of the tensor sources: x passes + update_h, or fused
-  // (timed on the scratch spectra with the state vectors y -> ytmp)
-  for (int v = 0; v < 2 && st == IH_OK; ++v) {
+  // (timed on the scratch spectra with the state vectors y -> ytmp; an FP64
+  // context without tensor modes has no table for the former and needs neither)
+  const int forms = sizeof(T) == 4 || c->p.enable_gw ? 2 : 0;
+  for (int v = 0; v < forms && st == IH_OK; ++v) {
     c->tensor_fused = v;
     float ms = 0.f;
     for (int r = 0; r <= reps && st == IH_OK; ++r) {

@@ -265,7 +265,7 @@ struct Ctx {
   void *fx_coef = nullptr;
   int fx_e[5] = {};
   int *shell = nullptr;         // shell of every mode of an octant (k_shell_table)
-  void *tensor_coef = nullptr;  // FP64 form: projection coefficients (k_tensor_table)
+  void *tensor_coef = nullptr;  // FP64 form with GW: projection coefficients (k_tensor_table)
   std::string tune_report;
 };
 constexpr int kFxAll = 0x5b;

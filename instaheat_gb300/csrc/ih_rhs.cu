@@ -615,6 +615,10 @@ static int tensor_last_pass_t(Ctx *c, C2<T> *s, T *y, T *out, double *outsc,
     if (c->tensor_fused && g.pow2) return fft_x_tensor<T>(c, s, y, out, outsc, next);
     IH_TRY((fft_xy<T>(c, s, M, 6, 0, -1)));
   }
+  if (sizeof(T) == 8 && !c->tensor_coef) {
+    c->err = "the tensor equation of motion of a context without tensor modes";
+    return IH_ERR_STATE;
+  }
   prof_begin(c, KK_UPDATE_H);
   if constexpr (sizeof(T) == 4) {
     const unsigned gm = grid_for(M, 256, 4);
