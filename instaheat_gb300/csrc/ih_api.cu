@@ -971,8 +971,10 @@ int ih_ensemble_autotune(ih_ensemble *e) {
     const Ctx *twin = nullptr;
     for (size_t j = 0; j < i; ++j) {
       const Ctx *d = &e->m[j]->c;
+      // (the passes that have a fixed-point form depend on the box too: without them
+      // there are no tables to read)
       if (d->g.nx == c->g.nx && d->g.ny == c->g.ny && d->g.nz == c->g.nz && d->mixed == c->mixed &&
-          d->p.device == c->p.device)
+          d->fx_can == c->fx_can && d->p.device == c->p.device)
         twin = d;
     }
     if (twin) {
