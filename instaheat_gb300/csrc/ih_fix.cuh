@@ -446,6 +446,20 @@ __device__ __forceinline__ long long fx_mul_sum(int ah, int al, FxCoef c) {
 __device__ __forceinline__ int fx_exponent(double x, int k) {  // biased, of x 2^k
   return ((__double2hiint(x) >> 20) & 0x7ff) + k;
 }
+// the mantissa of x with its leading one and sign, 2^61 to 2^62 (a zero's or
+// subnormal's is of no use), split for products: x = m 2^(fx_exponent - 1084)
+struct FxMantissa {
+  int h, l;
+};
+__device__ __forceinline__ FxMantissa fx_mantissa(double x) {
+  const int hi = __double2hiint(x);
+  long long v = ((long long)((hi & 0xfffff) | 0x100000) << 32 | (unsigned)__double2loint(x)) << 9;
+  if (hi < 0) v = -v;
+  FxMantissa m;
+  m.h = fx_hi(v);
+  m.l = (int)v;
+  return m;
+}
 struct FxPoint {
   bool fast;  // every x_j finite, the sums' exponents in range (k_j within 64)
   int in;     // integer = x_j 2^(k_j + in)
