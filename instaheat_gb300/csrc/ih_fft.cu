@@ -2023,11 +2023,14 @@ struct XYLaunch {
           return run_2s<L, B / 2>(grid, sj, so, tw);
         }
       }
-      if constexpr (sizeof(T) == 4 && L >= 8) {
+      if constexpr (sizeof(T) == 8) {
+        return run_st<B>(L, grid, sj, so, tw);
+      } else if constexpr (L >= 8) {
         constexpr int Bh = B / 2;
         return run_stk<L, Bh>(dim3((mz + Bh - 1) / Bh, outer, count), sj, so, tw);
+      } else {  // (no axis is shorter)
+        return IH_ERR_ARG;
       }
-      return run_st<B>(L, grid, sj, so, tw);
     }
   }
 };
@@ -2107,22 +2110,26 @@ struct Z3Launch {
   bool forward;
   template <int H>
   int run_reg() {
-    const long long rows = (long long)c->g.nx * c->g.ny;
-    const size_t sm = zg_smem<T>(H);
-    const dim3 grid((unsigned)((rows + kZB - 1) / kZB), count);
-    constexpr int nt = stk_threads<H, kZB>();
-    if (forward) {
-      auto kf = k_fft_zr2c_g<T, H>;
-      want_smem(kf, sm);
-      kf<<<grid, nt, sm, c->stream>>>((const T *)in, istride, (C2<T> *)out, ostride, rows, H,
-                                      tab<T>(c->tw_h), tab<T>(c->tw_z));
+    if constexpr (H > 192) {  // (nz <= 512)
+      return IH_ERR_ARG;
     } else {
-      auto kf = k_fft_zc2r_g<T, H>;
-      want_smem(kf, sm);
-      kf<<<grid, nt, sm, c->stream>>>((const C2<T> *)in, istride, (T *)out, ostride, rows, H,
-                                      tab<T>(c->tw_h), tab<T>(c->tw_z));
+      const long long rows = (long long)c->g.nx * c->g.ny;
+      const size_t sm = zg_smem<T>(H);
+      const dim3 grid((unsigned)((rows + kZB - 1) / kZB), count);
+      constexpr int nt = stk_threads<H, kZB>();
+      if (forward) {
+        auto kf = k_fft_zr2c_g<T, H>;
+        want_smem(kf, sm);
+        kf<<<grid, nt, sm, c->stream>>>((const T *)in, istride, (C2<T> *)out, ostride, rows, H,
+                                        tab<T>(c->tw_h), tab<T>(c->tw_z));
+      } else {
+        auto kf = k_fft_zc2r_g<T, H>;
+        want_smem(kf, sm);
+        kf<<<grid, nt, sm, c->stream>>>((const C2<T> *)in, istride, (T *)out, ostride, rows, H,
+                                        tab<T>(c->tw_h), tab<T>(c->tw_z));
+      }
+      return IH_OK;
     }
-    return IH_OK;
   }
 };
 
@@ -2300,8 +2307,13 @@ struct D4Launch {
       if (var == FV_PIPELINED) return run_pipe<L, B>();
       if (var == FV_TWOSTEP) return run_2s<L, B>();
       if (var == FV_TWOSTEP_HALF) return run_2s<L, B / 2>();
-      if constexpr (sizeof(T) == 4 && L >= 8) return run_reg<L>();
-      return run_st(L);
+      if constexpr (sizeof(T) == 8) {
+        return run_st(L);
+      } else if constexpr (L >= 8) {
+        return run_reg<L>();
+      } else {  // (no axis is shorter)
+        return IH_ERR_ARG;
+      }
     }
   }
 };

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 512 /
     if (col) {
 #pragma unroll
       for (int k1 = 0; k1 < R1; ++k1)
-        base[(long long)(q + R2 * k1) * sj] = fx_store<true>(u[k1], sc.out + 2, sc);
+        base[(long long)(q + R2 * k1) * sj] = fx_store(u[k1], sc.out + 2, sc);
     }
   }
 }
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 384 /
 #pragma unroll
         for (int n2 = 0; n2 < R2; ++n2) {
           double2 *d = dst + (long long)(q + R1 * n2) * sj;
-          double2 r = fx_store<true>(v[n2], e + (o ? e2 - room[1] : e1 - room[0]), sc);
+          double2 r = fx_store(v[n2], e + (o ? e2 - room[1] : e1 - room[0]), sc);
           if (ACC && o == 1) {
             const double2 a = *d;
             r.x += a.x;

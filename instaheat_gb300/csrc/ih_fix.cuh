@@ -318,15 +318,10 @@ __device__ __forceinline__ FxScale fx_scale(FxSize z, int bp, int bs) {
   s.out = -s.in;
   return s;
 }
-// Conversions on the FP64 pipe (2.1 per clock and SM) ...
+// Conversion on the FP64 pipe (2.1 per clock and SM) ...
 __device__ __forceinline__ long long fx_in_pipe(double a, const FxScale &s) {
   return __double2ll_rn(
       __hiloint2double(__double2hiint(a) + s.in * (1 << 20), __double2loint(a)));
-}
-__device__ __forceinline__ double fx_out_pipe(long long v, int e) {
-  const double d = __ll2double_rn(v);
-  const int h = __double2hiint(d);
-  return __hiloint2double(h == 0 ? 0 : h + e * (1 << 20), __double2loint(d));
 }
 // ... and on the integer pipe (about 3.5 per clock and SM): the mantissa, its
 // leading one put in, shifted to the pencil's exponent, and back by a count of
@@ -356,10 +351,6 @@ template <bool BITS>
 __device__ __forceinline__ long long fx_in(double a, const FxScale &s) {
   return BITS ? fx_in_bits(a, s) : fx_in_pipe(a, s);
 }
-template <bool BITS>
-__device__ __forceinline__ double fx_out(long long v, int e) {
-  return BITS ? fx_out_bits(v, e) : fx_out_pipe(v, e);
-}
 template <bool BITS, int R>
 __device__ __forceinline__ void fx_load(double2 (&x)[R], const FxScale &s, fx2 (&v)[R]) {
   if (s.slow) {
@@ -373,9 +364,8 @@ __device__ __forceinline__ void fx_load(double2 (&x)[R], const FxScale &s, fx2 (
   for (int i = 0; i < R; ++i) v[i] = fx_mk(fx_in<BITS>(x[i].x, s), fx_in<BITS>(x[i].y, s));
 }
 // value of v at exponent e, through the slow factor where the pencil has one
-template <bool BITS>
 __device__ __forceinline__ double2 fx_store(fx2 v, int e, const FxScale &s) {
-  double2 r = make_double2(fx_out<BITS>(v.x, e), fx_out<BITS>(v.y, e));
+  double2 r = make_double2(fx_out_bits(v.x, e), fx_out_bits(v.y, e));
   if (s.slow) {
     r.x *= s.post;
     r.y *= s.post;

@@ -87,11 +87,11 @@ __global__ void __launch_bounds__(32 * kFxWarps) k_fx_zr2c(
     double2 *dst = out + blockIdx.y * ostride + row * (H + 1);
 #pragma unroll
     for (int m = 0; m < A; ++m) {
-      double2 r = fx_store<true>(v[m], sc.out + 4, sc);
+      double2 r = fx_store(v[m], sc.out + 4, sc);
       if (m == 0 && t == 0) r.x += 2 * H * x0;
       dst[t + B * m] = r;
     }
-    if (t == 0) dst[H] = fx_store<true>(xH, sc.out + 4, sc);
+    if (t == 0) dst[H] = fx_store(xH, sc.out + 4, sc);
   }
 }
 
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(32 * kFxWarps) k_fx_zc2r(
     for (int q = 0; q < B; ++q) {
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        double2 r = fx_store<true>(v[E * q + e], sc.out + 4, sc);
+        double2 r = fx_store(v[E * q + e], sc.out + 4, sc);
         r.x += x0;
         r.y += x0;
         dst[E * t + e + A * q] = r;
@@ -219,7 +219,7 @@ __device__ __forceinline__ void fx_z_lap(const fx2 (&v)[FxZG<H>::A], int e, cons
   for (int q = 0; q < B; ++q) {
 #pragma unroll
     for (int j = 0; j < E; ++j)
-      dst[E * ln.t + j + A * q] = fx_store<true>(v[E * q + j], e, sc);
+      dst[E * ln.t + j + A * q] = fx_store(v[E * q + j], e, sc);
   }
 }
 // the six products: xx, xy, xz, yy, yz, zz
@@ -251,8 +251,8 @@ __device__ __forceinline__ void fx_z_product(fx2 (&v)[FxZG<H>::A], int e, bool s
   so.slow = slow;
   so.post = post;
 #pragma unroll
-  for (int m = 0; m < A; ++m) dst[ln.t + B * m] = fx_store<true>(v[m], e, so);
-  if (ln.t == 0) dst[H] = fx_store<true>(xH, e, so);
+  for (int m = 0; m < A; ++m) dst[ln.t + B * m] = fx_store(v[m], e, so);
+  if (ln.t == 0) dst[H] = fx_store(xH, e, so);
 }
 // rho and p of a point; |grad phi|^2 from the integer squares at the largest
 // exponent of the three rows
@@ -273,11 +273,11 @@ struct FxZPoint {
   }
   __device__ __forceinline__ double grad2(long long gx, long long gy, long long gz) const {
     if (slow) {  // extreme rows: in FP64
-      const double fx = fx_out<true>(gx, ex[0]) * post[0], fy = fx_out<true>(gy, ex[1]) * post[1],
-                   fz = fx_out<true>(gz, ex[2]) * post[2];
+      const double fx = fx_out_bits(gx, ex[0]) * post[0], fy = fx_out_bits(gy, ex[1]) * post[1],
+                   fz = fx_out_bits(gz, ex[2]) * post[2];
       return fx * fx + fy * fy + fz * fz;
     }
-    return fx_out<true>((fx_mul_sum(gx, gx) >> r[0]) + (fx_mul_sum(gy, gy) >> r[1]) +
+    return fx_out_bits((fx_mul_sum(gx, gx) >> r[0]) + (fx_mul_sum(gy, gy) >> r[1]) +
                             (fx_mul_sum(gz, gz) >> r[2]), eg);
   }
   __device__ __forceinline__ void operator()(double grad, double f, double d, double s, double &rho,
