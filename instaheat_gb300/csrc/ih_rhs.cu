@@ -391,13 +391,13 @@ __global__ void __launch_bounds__(256, 3) k_update_h_next(
 // instructions per mode are 0.59 ms); 64^3: 21 us against 42.
 //
 // The twelve products of a mode's real and of its imaginary parts are summed in
-// integers (tensor_sum: 13 FP64 instructions a mode are left): 256^3 555 -> 464 us
-// (4.1 TB/s), 128^3 80 -> 71.  Registers (122) leave 4 CTAs an SM; 5, with spills,
-// take 436 and 67 us, but 18.4 instead of 16.8 at 64^3.  One exponent for all sources of
+// integers (tensor_sum: 13 FP64 instructions a mode are left): 256^3 555 -> 439 us
+// (4.3 TB/s), 128^3 80 -> 68, 64^3 15.1.  Registers (about 120) leave 4 CTAs an SM.  One exponent for all sources of
 // a mode, in use before, took 387 us and lost the components that the largest
-// source has no part in.  The coefficients are stored for these sums, as fractions
-// of 2^k, alpha and beta with a k each.
-constexpr int kTensorCoefs = 14;
+// source has no part in.  The coefficients are stored for these sums: the mantissa
+// of each, a fraction of 2^(k - shift), alpha and beta with a k each, and the shift in
+// its lowest bits.
+constexpr int kTensorCoefs = 14, kNoCoef = 511;
 __global__ void k_tensor_table(long long *coef, long long Mo, Geom g) {
   const int nyh = g.ny / 2 + 1;
   for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < Mo;
@@ -418,8 +418,13 @@ __global__ void k_tensor_table(long long *coef, long long Mo, Geom g) {
         m = fmax(m, fabs(c[n][a]));
       }
       frexp(m, &e[n]);
-      for (int a = 0; a < 6; ++a)
-        coef[(6 * n + a) * Mo + o] = __double2ll_rn(ldexp(c[n][a], 62 - e[n]));
+      for (int a = 0; a < 6; ++a) {
+        int ea;  // the mantissa, 2^61 to 2^62 with nine zero bits, and in these its shift
+        const double f = frexp(c[n][a], &ea);
+        const bool none = f == 0.0 || e[n] - ea >= kNoCoef;
+        coef[(6 * n + a) * Mo + o] =
+            none ? kNoCoef : __double2ll_rn(ldexp(f, 62)) | (long long)(e[n] - ea);
+      }
     }
     coef[12 * Mo + o] = __double_as_longlong(ksq);
     coef[13 * Mo + o] = (long long)e[1] << 32 | (unsigned)e[0];
@@ -427,23 +432,22 @@ __global__ void k_tensor_table(long long *coef, long long Mo, Geom g) {
 }
 // v, negated where f
 __device__ __forceinline__ long long flip(long long v, int f) { return (v ^ -(long long)f) + f; }
-// sum_a c_a x_a: c_a a fraction of 2^(k + ec_a) between 2^61 and 2^62, or 0 with
+// sum_a c_a x_a: c_a a fraction of 2^(k - up_a) between 2^61 and 2^62, or 0 with
 // kNoCoef; x_a as its mantissa m_a (FxMantissa) at the biased exponent e_a, all: the
 // largest of these.  The products are added at the exponent of the largest product,
 // so that a mode whose largest source has a small or no part in one of its
 // components (S_zz along kz in n1) keeps that component to 2^-57 of its own.
-constexpr int kNoCoef = -4096;
 __device__ __forceinline__ double tensor_sum(const double (&x)[6], const FxMantissa (&m)[6],
                                              const int (&e)[6], int all, const long long (&c)[6],
-                                             const int (&ec)[6], int k) {
+                                             const int (&up)[6], int k) {
   int em = 0;
 #pragma unroll
-  for (int a = 0; a < 6; ++a) em = max(em, e[a] + ec[a]);
+  for (int a = 0; a < 6; ++a) em = max(em, e[a] - up[a]);
   if (em >= 200 && all <= 1900) {
     long long s = 0;
 #pragma unroll
     for (int a = 0; a < 6; ++a)
-      s += fx_mul_low(m[a].h, m[a].l, fx_hi(c[a]), (int)c[a]) >> min(em - (e[a] + ec[a]), 63);
+      s += fx_mul_low(m[a].h, m[a].l, fx_hi(c[a]), (int)c[a]) >> min(em - (e[a] - up[a]), 63);
     return fx_out_bits(s, em + k - 1082);
   }
   double n = 0.0;
@@ -451,22 +455,22 @@ __device__ __forceinline__ double tensor_sum(const double (&x)[6], const FxManti
   for (int a = 0; a < 6; ++a) {
     double xa = x[0];
     long long ca = c[0];
-    int ea = ec[0];
+    int ua = up[0];
 #pragma unroll
     for (int b = 1; b < 6; ++b) {
       if (a == b) {
         xa = x[b];
         ca = c[b];
-        ea = ec[b];
+        ua = up[b];
       }
     }
-    n += ldexp(__ll2double_rn(ca), k + ea - 62) * xa;
+    n += ldexp(__ll2double_rn(ca), k - ua - 62) * xa;
   }
   return n;
 }
 __device__ __forceinline__ void tensor_sums(const double (&x)[6], const long long (&al)[6],
-                                            const long long (&be)[6], const int (&ea)[6],
-                                            const int (&eb)[6], int k0, int k1, double &n0,
+                                            const long long (&be)[6], const int (&ua)[6],
+                                            const int (&ub)[6], int k0, int k1, double &n0,
                                             double &n1) {
   FxMantissa m[6];
   int e[6], all = 0;
@@ -476,15 +480,8 @@ __device__ __forceinline__ void tensor_sums(const double (&x)[6], const long lon
     all = max(all, e[a]);
     m[a] = fx_mantissa(x[a]);
   }
-  n0 = tensor_sum(x, m, e, all, al, ea, k0);
-  n1 = tensor_sum(x, m, e, all, be, eb, k1);
-}
-// a coefficient of the table brought to 2^61 .. 2^62; the exponent that takes
-__device__ __forceinline__ int tensor_norm(long long &c) {
-  if (c == 0) return kNoCoef;
-  const int up = max(__clzll((unsigned long long)(c < 0 ? -c : c)) - 2, 0);
-  c <<= up;
-  return -up;
+  n0 = tensor_sum(x, m, e, all, al, ua, k0);
+  n1 = tensor_sum(x, m, e, all, be, ub, k1);
 }
 // per: modes of an octant entry per thread (4, or fewer with the rest on
 // gridDim.y where the grid would otherwise leave SMs idle)
@@ -500,13 +497,15 @@ __global__ void __launch_bounds__(128) k_update_h_tab(
   const TensorConsts<double> tc(rs);
   const double dt = NEXT ? *nl.dt : 0.0;
   long long al[6], be[6];
-  int ea[6], eb[6];
+  int ua[6], ub[6];
 #pragma unroll
   for (int a = 0; a < 6; ++a) {
     al[a] = coef[(long long)a * Mo + o];
     be[a] = coef[(long long)(6 + a) * Mo + o];
-    ea[a] = tensor_norm(al[a]);
-    eb[a] = tensor_norm(be[a]);
+    ua[a] = (int)al[a] & kNoCoef;
+    ub[a] = (int)be[a] & kNoCoef;
+    al[a] &= ~(long long)kNoCoef;
+    be[a] &= ~(long long)kNoCoef;
   }
   const double ksq = __longlong_as_double(coef[(long long)12 * Mo + o]);
   const long long ks = coef[(long long)13 * Mo + o];
@@ -538,8 +537,8 @@ __global__ void __launch_bounds__(128) k_update_h_tab(
       xi[a] = v[a].y;
     }
     double2 n0, n1;
-    tensor_sums(xr, al, be, ea, eb, k0, k1, n0.x, n1.x);
-    tensor_sums(xi, al, be, ea, eb, k0, k1, n0.y, n1.y);
+    tensor_sums(xr, al, be, ua, ub, k0, k1, n0.x, n1.x);
+    tensor_sums(xi, al, be, ua, ub, k0, k1, n0.y, n1.y);
     if (id == 0) n0 = n1 = make_double2(0.0, 0.0);
     tensor_eom<double, NEXT>(g, id, n0, n1, ksq, tc, y, out, nl, dt);
   }
