@@ -183,8 +183,11 @@ int ih_variance_host(ih_context *c, double mean, const double *f_host, size_t n,
  * the kz slab widths of the tensor sources' y/x passes and, where it
  * applies, the plane-major tail of the tensor sources (pass 8 below) of the
  * RHS on the context's scratch spectra and keeps the fastest per pass.  Until
- * it is called the passes use the shared-memory Stockham engine.  Results are identical across variants up to rounding.  The report
- * lists the timings and the choice (valid until the next ih_autotune). */
+ * it is called the FP64 passes run in fixed point where the grid has that form
+ * (pass 9 below), the others on the Stockham engine (its stages in registers for
+ * FP32 axes of 2^a, 3 2^a and 9 2^a points, in shared memory for the rest).
+ * Results are identical across variants up to rounding.  The report lists the
+ * timings and the choice (valid until the next ih_autotune). */
 int ih_autotune(ih_context *c);
 const char *ih_autotune_report(const ih_context *c);
 /* Pin or read the engine of one pass: pass 0 = x, 1 = y, 2 = the fused

@@ -263,11 +263,12 @@ __device__ __forceinline__ void load_table(V *dst, const V *src, int n, int tid,
 // by its exchanges: a barrier pair, a round trip through shared memory and index
 // divisions per stage, three or four stages a pass.  Here: value by value the
 // operations of smem_fft and smem_fft_g in their order, so that the results are
-// the same to the bit, but several stages per thread and one exchange in all.  With elements q + st p of a stage of remaining length Lc
-// (p < Lc, st = L / Lc), a radix-r stage takes p = pp + t Lc/r to q + st (r pp +
-// t') with the twiddle w_L^(t' pp st); radix 4 while 4 divides Lc, then 2, then
-// 3.  Step 1: the first stage or the first two, S1 = 4 or 16 values: thread pp
-// over p = pp + i L/S1.  Step 2: the rest, thread q over all p of its S2 = L/S1.
+// the same to the bit, but several stages per thread and one exchange in all.  With
+// elements q + st p of a stage of remaining length Lc (p < Lc, st = L / Lc), a
+// radix-r stage takes p = pp + t Lc/r to q + st (r pp + t') with the twiddle
+// w_L^(t' pp st); radix 4 while 4 divides Lc, then 2, then 3.  Step 1: the first
+// stage or the first two, S1 = 4 or 16 values: thread pp over p = pp + i L/S1.
+// Step 2: the rest, thread q over all p of its S2 = L/S1.
 template <int L> struct StkFac {
   static constexpr int S1 = L % 16 == 0 && L >= 48 ? 16 : 4, S2 = L / S1;
 };
@@ -1729,8 +1730,8 @@ __global__ void __launch_bounds__(32 * zwarps<T>(), (sizeof(T) == 4 && H <= 128 
 // passes of z_pass_generic (ih_rhs.cu) for kZB rows per CTA: 4 c2r, rho and p and
 // their FP64 sums, 6 products and their r2c, each value with the operations of
 // k_fft_zc2r_g, k_pointwise_g and k_fft_zr2c_g.  Unfused it moved 33 arrays of the
-// grid through memory instead of 15: 96^3 94 us (4 + 1 + 6 launches) -> 49.5, step 2.16
-// -> 1.92 ms; 192^3 step 11.6 -> 9.7 ms.  Spectra d4 (d/dx, d/dy, d/dz, laplacian) and
+// grid through memory instead of 15: 96^3 94 us (4 + 1 + 6 launches) -> 49.5, step
+// 2.16 -> 1.92 ms; 192^3 step 11.6 -> 9.7 ms.  Spectra d4 (d/dx, d/dy, d/dz, laplacian) and
 // s6 may share their rows: a CTA reads all of its own before it writes.
 template <int H>
 __global__ void __launch_bounds__(stk_threads<H, kZB>()) k_fft_z_rhs_g(

@@ -18,10 +18,12 @@ namespace ih {
 // thread (b, n1) holds x[n1 + R1 n2] of column b, an R2-point DFT, the table
 // twiddle, one exchange through shared memory, an R1-point DFT.  Tiles of 8
 // columns are 128-byte lines.  At 256^3 (55 launches of a DOPRI853 step, 3 to
-// 4 arrays each): 272 us a launch against 1298 us on the FP64 pipe, 3.0 TB/s;
-// 128^3: 47 against 163 us.  Both conversions are on the integer pipe: on the
-// FP64 pipe (1.9 clocks per complex value and SM) they bound the pass, 340 and
-// 57 us (inputs alone on the integer pipe 295 / 51, outputs alone 271 / 49).
+// 6 arrays each): 501 us a launch on average, 3.0 TB/s (six arrays 556 us; on the
+// FP64 pipe four took 1298 us); 128^3: 82 us.  Sizing a pencil by its sum of
+// magnitudes takes 6% of that (473 and 75 us by its largest value).  Both
+// conversions are on the integer pipe: on the FP64 pipe (1.9 clocks per complex
+// value and SM) they bounded the pass, 340 against 272 us of four arrays (inputs
+// alone on the integer pipe 295, outputs alone 271).
 template <int L> struct FxFac;
 template <> struct FxFac<8> { static constexpr int R1 = 4, R2 = 2; };
 template <> struct FxFac<16> { static constexpr int R1 = 4, R2 = 4; };
@@ -145,9 +147,10 @@ __global__ void __launch_bounds__(fx_threads<L, B>(), fx_maxr<L>() <= 16 ? 512 /
 // the coefficient of d2 takes -kz^2 too (cz / 2^ez in Q62, brought to a common
 // exponent with c2 for each column), so that d2 is the y and z part of the
 // laplacian, and the x part in out1 is added.
-// At 256^3: 344 us a round trip against 1359 us on the FP64 pipe, 128^3 53 us
-// against 178.  Inputs convert on the FP64 pipe, outputs (two per input) on the
-// integer pipe: 375 us with both on the former, 388 on the latter.
+// At 256^3: 362 us a round trip against 1359 us on the FP64 pipe, 128^3 56 us
+// against 178 (344 and 53 without the products' sizes, below).  Inputs convert on
+// the FP64 pipe, outputs (two per input) on the integer pipe: 375 us instead of 344
+// with both on the former, 388 on the latter.
 // Between the transforms each product k X, k^2 X is brought to the size that the
 // inverse transform has room for: a pencil whose power lies at small k (a k^-2
 // spectrum, a single wave) fills little of the coefficients' range, and with the

@@ -11,7 +11,7 @@
 // pencil's sum of magnitudes (FxSize), which bounds every value on the way,
 // whatever the pencil holds: white noise has its units where the largest
 // value's worst growth would put them, a pencil with one dominant value 2^-57 of
-// that value.  Errors of a pass (2-norm) are 0.3 to 0.6 of those in FP64 for
+// that value.  Errors of a pass (2-norm) are 0.2 to 0.7 of those in FP64 for
 // white noise, a spike, a falling or a single-wave spectrum of 8 to 512 points.
 //
 // Growth: sqrt(2) S bounds the sum of the magnitudes.  The part of it that one

@@ -392,11 +392,11 @@ __global__ void __launch_bounds__(256, 3) k_update_h_next(
 //
 // The twelve products of a mode's real and of its imaginary parts are summed in
 // integers (tensor_sum: 13 FP64 instructions a mode are left): 256^3 555 -> 439 us
-// (4.3 TB/s), 128^3 80 -> 68, 64^3 15.1.  Registers (about 120) leave 4 CTAs an SM.  One exponent for all sources of
-// a mode, in use before, took 387 us and lost the components that the largest
-// source has no part in.  The coefficients are stored for these sums: the mantissa
-// of each, a fraction of 2^(k - shift), alpha and beta with a k each, and the shift in
-// its lowest bits.
+// (4.3 TB/s), 128^3 80 -> 68, 64^3 15.1.  Registers (about 120) leave 4 CTAs an SM.
+// One exponent for all sources of a mode, in use before, took 387 us and lost the
+// components that the largest source has no part in.  The coefficients are stored
+// for these sums: the mantissa of each, a fraction of 2^(k - shift), alpha and beta
+// with a k each, and the shift in its lowest bits.
 constexpr int kTensorCoefs = 14, kNoCoef = 511;
 __global__ void k_tensor_table(long long *coef, long long Mo, Geom g) {
   const int nyh = g.ny / 2 + 1;

@@ -488,8 +488,9 @@ __global__ void __launch_bounds__(256) k_dopri_final(const T *__restrict__ y, co
       acc3d = (double)acc3;
     } else {
       // the homogeneous parts of the plain form are 0; one reciprocal for both
-      // ratios; |y| compared as bits, off the FP64 pipe, which has the rest: 9 operations an element with recip, 17 with a division
-      // (256^3: 8.24 and 7.78 ms with the sums on the FP64 pipe)
+      // ratios; |y| compared as bits, off the FP64 pipe, which has the rest: 9
+      // operations an element with recip, 17 with a division (256^3: 7.78 and 8.24
+      // ms with the sums on the FP64 pipe)
       acc5d = 0.0;
       acc3d = 0.0;
 #pragma unroll
